@@ -122,9 +122,8 @@ int fp64_diff_main_device(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam
                             lambda, fac, edges));
     PBT_TRY(upload(ctx->d_fac, fac.data(), fac.size(), st));
     PBT_TRY(upload(ctx->d_edge, edges.data(), edges.size(), st));
-    const K1Facet *df = ctx->d_fac.as<K1Facet>();
-    PBT_TRY(k1_launch(ctx, st, df, nbeam, ctx->d_edge.as<K1Edge>(), lambda, fast_diff, d_afb));
-    PBT_TRY(k1_launch(ctx, st, df + nbeam, next, ctx->d_edge.as<K1Edge>(), lambda, fast_diff, d_afe));
+    PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), nbeam, next, ctx->d_edge.as<K1Edge>(), lambda,
+                      fast_diff, d_afb, d_afe));
     // the host vectors are released at return: finish the copies first
     PBT_CUDA_TRY(cudaStreamSynchronize(st));
     return PBT_OK;
@@ -256,8 +255,8 @@ extern "C" int pbt_diffraction_c(pbt_ctx *ctx, const pbt_outbeam *outbeam, const
     PBT_TRY(upload(ctx->d_fac, fac.data(), fac.size(), st));
     PBT_TRY(upload(ctx->d_edge, edges.data(), edges.size(), st));
     PBT_TRY(ctx->d_out.ensure(8 * nb * sizeof(double)));
-    PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), 1, ctx->d_edge.as<K1Edge>(), lambda,
-                      is_fast_diff ? 1 : 0, ctx->d_out.as<double>()));
+    PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), 1, 0, ctx->d_edge.as<K1Edge>(), lambda,
+                      is_fast_diff ? 1 : 0, ctx->d_out.as<double>(), nullptr));
     PBT_CUDA_TRY(cudaMemcpyAsync(amplC, ctx->d_out.p, 8 * nb * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
     PBT_CUDA_TRY(cudaStreamSynchronize(st));

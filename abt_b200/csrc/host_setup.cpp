@@ -199,6 +199,86 @@ int grid_prepare(pbt_ctx *ctx, const double *theta, int64_t ntheta, const double
     return PBT_OK;
 }
 
+void k1_facet(const FacetFrame &fr, const pbt_outbeam &ob, double fov, int nv, const double *rx,
+              const double *ry, const double *rz, double *xs, double *ys, double *ms, double waveno,
+              double lambda, int64_t edge_off, K1Facet &F, K1Edge *E) {
+    for (int c = 0; c < 3; c++) {
+        F.com[c] = fr.com[c];
+        F.inc2[c] = fr.inc2[c];
+        F.prop0[c] = ob.prop_out[c];
+    }
+    for (int a = 0; a < 3; a++)
+        for (int b = 0; b < 3; b++) F.R[3 * a + b] = fr.R.m[a][b];
+    for (int b = 0; b < 2; b++) {
+        // column b: a(1,b) = ampl[4b], a(2,b) = ampl[4b + 2] (re), u+- = a(1,b) +- i a(2,b)
+        const double s = fr.sign < 0 ? -1.0 : 1.0;
+        const double *a = ob.ampl + 4 * b;
+        F.circ[2 * b] = s * (a[0] - a[3]);
+        F.circ[2 * b + 1] = s * (a[1] + a[2]);
+        F.circ[4 + 2 * b] = s * (a[0] + a[3]);
+        F.circ[4 + 2 * b + 1] = s * (a[1] - a[2]);
+    }
+    F.cos_fov = cos(fov);  // src/diff_mod.f90:523
+    F.kinc0 = fr.prop2[0] * waveno;
+    F.kinc1 = fr.prop2[1] * waveno;
+    F.Kx = fr.prop2[0];
+    F.Ky = fr.prop2[1];
+    F.Kz = fr.prop2[2];
+    F.edge_off = edge_off;
+    F.nv = nv;
+    // contour_integral set-up, src/diff_mod.f90:334-354
+    for (int i = 0; i < nv; i++) {
+        double c[3] = {rx[i], ry[i], rz[i]}, r[3];
+        mv33(fr.R, c, r);
+        xs[i] = r[0];
+        ys[i] = r[1];
+    }
+    for (int i = 0; i < nv; i++) {
+        int in = (i == nv - 1) ? 0 : i + 1;
+        ms[i] = (ys[in] - ys[i]) / (xs[in] - xs[i]);
+    }
+    bool clamped = false;
+    double area = 0.0, rmax = 0.0, lmax = 0.0;
+    for (int i = 0; i < nv; i++) {
+        double mj = ms[i], nj = 1 / ms[i];
+        // slope clamps, in the reference's order, src/diff_mod.f90:379-382
+        if (fabs(mj) > DBL_MAX) mj = 1e6;
+        if (fabs(nj) > DBL_MAX) nj = 1e6;
+        if (fabs(mj) < 1e-9) nj = 1e6;
+        if (fabs(nj) < 1e-9) mj = 1e6;
+        clamped = clamped || !(fabs(mj * nj - 1.0) < 1e-9);
+        int in = (i == nv - 1) ? 0 : i + 1;
+        E[i].xj = xs[i];
+        E[i].yj = ys[i];
+        E[i].mj = mj;
+        E[i].nj = nj;
+        E[i].dx = xs[in] - xs[i];
+        E[i].dy = ys[in] - ys[i];
+        area += 0.5 * (xs[i] * ys[in] - xs[in] * ys[i]);
+        rmax = std::max(rmax, fabs(xs[i]) + fabs(ys[i]));
+        lmax = std::max(lmax, fabs(E[i].dx) + fabs(E[i].dy));
+    }
+    F.area2 = 2.0 * area / lambda;
+    for (int i = 0; i < 3; i++) {
+        F.xy[2 * i] = xs[i];
+        F.xy[2 * i + 1] = ys[i];
+    }
+    for (int i = 0; i < 2; i++) {
+        F.dxy[2 * i] = E[i].dx;
+        F.dxy[2 * i + 1] = E[i].dy;
+    }
+    F.pad[0] = F.pad[1] = 0.0;
+    // The contour's rounding noise relative to the facet's area: nv edges of
+    // ulp(d) L / (min(|kxx|, |kyy|) |omega| A), |d| <= 2 k rmax; `cond` is where it
+    // reaches 5e-11.  A clamped slope has no closed form: the contour everywhere (and
+    // with phases beyond the kernel's argument reduction).
+    const double noise = nv * 2.0 * waveno * rmax * 2.2e-16 * lmax;
+    F.cond = clamped || !(fabs(area) > 0) || 2.0 * waveno * (rmax + kFarR) > 1e9
+                 ? HUGE_VAL
+                 : noise / (fabs(area) * 5e-11);
+    if (!(F.cond > 1e-200)) F.cond = HUGE_VAL;
+}
+
 int k1_build_facets(const pbt_outbeam *obs, int64_t n, double fov_override, const double *verts,
                     int64_t nverts, const int64_t *face_off, const int64_t *face_vi,
                     int64_t nfaces, double lambda, std::vector<K1Facet> &fac,
@@ -244,50 +324,10 @@ int k1_build_facets(const pbt_outbeam *obs, int64_t n, double fov_override, cons
         FacetFrame fr;
         fr.sign = 1.0;
         facet_frame(vx, vy, vz, nv, ob.prop_out, ob.vk7, fr, rx, ry, rz);
-        K1Facet &F = fac[f0 + j];
-        for (int c = 0; c < 3; c++) {
-            F.com[c] = fr.com[c];
-            F.prop2[c] = fr.prop2[c];
-            F.inc2[c] = fr.inc2[c];
-            F.prop0[c] = ob.prop_out[c];
-        }
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) F.R[3 * a + b] = fr.R.m[a][b];
-        for (int q = 0; q < 8; q++) F.ampl[q] = fr.sign < 0 ? -ob.ampl[q] : ob.ampl[q];
-        double fov = fov_override >= 0 ? fov_override : ob.fov;
-        F.cos_fov = cos(fov);  // src/diff_mod.f90:523
-        F.kinc[0] = fr.prop2[0] * waveno;
-        F.kinc[1] = fr.prop2[1] * waveno;
-        F.edge_off = (int64_t)e0 + eoff[j];
-        F.nv = nv;
-        // contour_integral set-up, src/diff_mod.f90:334-354
-        std::vector<double> xs(nv), ys(nv), ms(nv);
-        for (int i = 0; i < nv; i++) {
-            double c[3] = {rx[i], ry[i], rz[i]}, r[3];
-            mv33(fr.R, c, r);
-            xs[i] = r[0];
-            ys[i] = r[1];
-        }
-        for (int i = 0; i < nv; i++) {
-            int in = (i == nv - 1) ? 0 : i + 1;
-            ms[i] = (ys[in] - ys[i]) / (xs[in] - xs[i]);
-        }
-        for (int i = 0; i < nv; i++) {
-            double mj = ms[i], nj = 1 / ms[i];
-            // slope clamps, in the reference's order, src/diff_mod.f90:379-382
-            if (fabs(mj) > DBL_MAX) mj = 1e6;
-            if (fabs(nj) > DBL_MAX) nj = 1e6;
-            if (fabs(mj) < 1e-9) nj = 1e6;
-            if (fabs(nj) < 1e-9) mj = 1e6;
-            int in = (i == nv - 1) ? 0 : i + 1;
-            K1Edge &E = edges[F.edge_off + i];
-            E.xj = xs[i];
-            E.yj = ys[i];
-            E.mj = mj;
-            E.nj = nj;
-            E.dx = xs[in] - xs[i];
-            E.dy = ys[in] - ys[i];
-        }
+        std::vector<double> sb(3 * nv);
+        const double fov = fov_override >= 0 ? fov_override : ob.fov;
+        k1_facet(fr, ob, fov, nv, rx, ry, rz, sb.data(), sb.data() + nv, sb.data() + 2 * nv, waveno,
+                 lambda, (int64_t)e0 + eoff[j], fac[f0 + j], edges.data() + e0 + eoff[j]);
     }
     return PBT_OK;
 }

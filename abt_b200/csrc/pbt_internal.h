@@ -84,20 +84,29 @@ struct HostBuf {
 
 // ------------------------------------------- reference-exact FP64 records
 // One outgoing facet, prepared for the FP64 kernel (all values formed in the
-// reference's operation order).  272 bytes.
-struct K1Facet {
+// reference's operation order).  384 bytes, in the order the kernel reads it
+// from shared memory, 16 bytes at a time.
+struct alignas(16) K1Facet {
     double com[3];
+    double kinc0;     // prop2(1) * waveno  (src/diff_mod.f90:336)
     double R[9];      // matmul(rot2, rot), row-major
-    double prop2[3];
-    double inc2[3];
-    double kinc[2];   // prop2(1:2) * waveno  (src/diff_mod.f90:336)
-    double ampl[8];   // amplitude after the anti-parallel flip: (1,1),(2,1),(1,2),(2,2) re/im
+    double kinc1;     // prop2(2) * waveno
+    double Kz;        // prop2(3)
+    double area2;     // triangles: 2 A / lambda, A the signed aperture area
+    double circ[8];   // amplitude after the anti-parallel flip, columns in the circular basis
+                      // u+- = a(1,:) +- i a(2,:): u+_1, u+_2, u-_1, u-_2, re/im
+    double xy[6];     // the first three vertices, x and y
+    double dxy[4];    // their first two edges, dx and dy
+    double cond;      // bins with min |omega| min(|kxx|, |kyy|) below it take the contour (k1_fp64.cu)
+    int64_t nv;
     double prop0[3];  // lab-frame propagation (field-of-view test)
     double cos_fov;
     int64_t edge_off;
-    int64_t nv;
+    double Kx, Ky;    // prop2(1:2)
+    double inc2[3];
+    double pad[2];
 };
-static_assert(sizeof(K1Facet) == 272, "K1Facet layout");
+static_assert(sizeof(K1Facet) == 384, "K1Facet layout");
 
 // One aperture edge after the slope clamps of src/diff_mod.f90:379-393.
 struct K1Edge {
@@ -181,9 +190,17 @@ int k1_build_facets(const pbt_outbeam *obs, int64_t n, double fov_override, cons
                     int64_t nfaces, double lambda, std::vector<K1Facet> &fac,
                     std::vector<K1Edge> &edges);
 
-// FP64 far-field sum of nf facets into a complex (nphi,ntheta,2,2) grid (overwritten).
-int k1_launch(pbt_ctx *ctx, cudaStream_t st, const K1Facet *d_fac, int64_t nf,
-              const K1Edge *d_edges, double lambda, int fast_diff, double *d_grid);
+// One facet's kernel record and edges from its frame (rx/ry/rz: vertices relative
+// to the centre; xs/ys/ms: scratch of nv doubles each).
+struct FacetFrame;
+void k1_facet(const FacetFrame &fr, const pbt_outbeam &ob, double fov, int nv, const double *rx,
+              const double *ry, const double *rz, double *xs, double *ys, double *ms, double waveno,
+              double lambda, int64_t edge_off, K1Facet &F, K1Edge *E);
+
+// FP64 far-field sums of two lists, facets [0, n0) and [n0, n0 + n1), into complex
+// (nphi,ntheta,2,2) grids (overwritten; grid1 NULL: the first list only).
+int k1_launch(pbt_ctx *ctx, cudaStream_t st, const K1Facet *d_fac, int64_t n0, int64_t n1,
+              const K1Edge *d_edges, double lambda, int fast_diff, double *d_grid0, double *d_grid1);
 
 // Reference-exact finalise on device grids.  Writes mueller (nb*16),
 // mueller_1d (ntheta*16) and params (18 doubles) to device memory; adds to the
