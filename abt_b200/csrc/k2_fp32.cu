@@ -135,10 +135,12 @@ __global__ void k2_count_kernel(RefSrc S, int64_t nrefs, const int64_t *__restri
 }
 
 // Write record r into half r % 2 of pair r / 2 (K2Pair's half-phase and
-// scaled forms): kzc = -Kz / (1 - Ky^2) and the circular-basis amplitudes uc
-// times sqrt(1 - Ky^2) / 4, both formed in FP64 by the caller.
+// scaled forms): kzc = -Kz / (1 - Ky^2), the circular-basis amplitudes uc
+// times sqrt(1 - Ky^2) / 4 and the scaled vertex ordinates vys, all formed in
+// FP64 by the caller.
 __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const K2Rec &rec,
-                                                double kzc, const double (&uc)[8]) {
+                                                double kzc, const double (&uc)[8],
+                                                const double (&vys)[3]) {
     K2Pair &P = pairs[r >> 1];
     const int h = (int)(r & 1);
     auto put = [h](float2 &dst, float v) {
@@ -150,15 +152,12 @@ __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const 
     for (int c = 0; c < 3; c++) {
         P.kc[c][h] = 0.5 * rec.kc[c];
         put(P.eps[c], rec.eps[c]);
-        put(P.nea[c], -rec.ea[c]);
-        put(P.inc[c], rec.inc[c]);
         put(P.vx[c], rec.vx[c]);
-        put(P.vy[c], rec.vy[c]);
+        put(P.vy[c], (float)vys[c]);
     }
     put(P.b, rec.b);
     for (int q = 0; q < 9; q++) put(P.R[q], rec.R[q]);
-    put(P.kp[0], 0.5f * rec.kp[0]);
-    put(P.kp[1], 0.5f * rec.kp[1]);
+    put(P.kp, 0.5f * rec.kp[0]);
     put(P.kzc, (float)kzc);
     for (int q = 0; q < 8; q++) put(P.amp[q], (float)uc[q]);
 }
@@ -262,7 +261,8 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
             const double uc[8] = {sk * (am[0] - am[3]), sk * (am[1] + am[2]), sk * (am[0] + am[3]),
                                   sk * (am[1] - am[2]), sk * (am[4] - am[7]), sk * (am[5] + am[6]),
                                   sk * (am[4] + am[7]), sk * (am[5] - am[6])};
-            store_pair_half(pairs, r0 + t, rec, -fr.prop2[2] * cf * cf, uc);
+            const double vys[3] = {-0.5 * waveno * ya[0], -0.5 * waveno * ya[1], -0.5 * waveno * ya[2]};
+            store_pair_half(pairs, r0 + t, rec, -fr.prop2[2] * cf * cf, uc, vys);
         } else {
             recs[r0 + t] = rec;
         }
@@ -769,6 +769,13 @@ __global__ void __launch_bounds__(K2_THREADS, 2) k2_main_kernel(K2MainArgs P) {
 // even record of a K2Pair, the y lane the odd one.  The bin's data are
 // loop-invariant broadcast pairs.  Special-function calls, the sort of the
 // three phases and the FP64 phase stay per facet.
+//
+// Bound: issue.  Over the pair loop the FMA pipe's cycles (an FFMA2 holds it two)
+// and the other instructions add up to 88 % of the cycles, at 16 and 20 warps per SM
+// alike, so only fewer operations help.  With the plane's normal taken from the lab
+// frame (no R s + R e, no h in the aperture frame) and the sinc series formed by
+// every lane instead of behind a vote, 200,000 triangles x 259,560 bins take 224.1 ms
+// (244.8 ms before; the lab frame alone 227.8).
 
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 // the special-function unit's approximations with subnormal inputs flushed
@@ -796,27 +803,24 @@ __device__ __forceinline__ float2 sel2(bool px, bool py, float2 a, float2 b) {
     return make_float2(px ? a.x : b.x, py ? a.y : b.y);
 }
 
-// A bin of the packed kernel.  The direction is held as s = u + sg z, sg = +1 in
-// the hemisphere of the incidence direction (0,0,-1) and -1 in the other, so
-// that sz = uz + sg (formed in FP64, rounded once) is small and exact to FP32
-// precision near both poles; u = (fx, fy, sz - sg).  The forward-bodge bin
-// direction, used near the poles only, is kept in shared memory (slot hslot of
-// the kernel's bodge table) in the same form with the kernel's sgh.
+// A bin of the packed kernel: the unit direction in FP64 and as FP32 broadcast
+// pairs.  The forward-bodge bin direction, used near the poles only, is kept in
+// shared memory (slot hslot of the kernel's bodge table).
 struct BinPk {
     double ux, uy, uz;     // unit bin direction, FP64
-    float2 fx, fy, sz, sg; // broadcast FP32 pairs
+    float2 fx, fy, fz;     // broadcast FP32 pairs
     int hslot;
     bool pole;             // within reach of the forward bodge (|uz| near 1) for some record
     int64_t bin;           // bin index
 };
 constexpr int K2P_HB = K2_THREADS * 2;  // bodge table slots (bins per thread <= 2)
 
-// sin(h)/h below h = 0.5, where the MUFU sine's absolute error would be a large
-// relative one: 1 + c1 h^2 + c2 h^4 with c1, c2 the minimax fit to the relative
-// error on [0, 0.5] (Lawson's iteration: 1.2e-7, 1.6e-7 evaluated in FP32)
-__device__ __forceinline__ float2 sinc_series(float2 h) {
+// sin(h)/(2h) below h = 0.5, where the MUFU sine's absolute error would be a large
+// relative one: half of 1 + c1 h^2 + c2 h^4 with c1, c2 the minimax fit to the
+// relative error on [0, 0.5] (Lawson's iteration: 1.2e-7, 1.6e-7 evaluated in FP32)
+__device__ __forceinline__ float2 half_sinc_series(float2 h) {
     const float2 hh = mul2(h, h);
-    return fma2(hh, fma2(hh, bc2(8.264339e-3f), bc2(-1.6666131e-1f)), bc2(1.0f));
+    return fma2(hh, fma2(hh, bc2(0.5f * 8.264339e-3f), bc2(0.5f * -1.6666131e-1f)), bc2(0.5f));
 }
 
 // 2 sc g for each lane, g the second divided difference of e^{ix} at the full
@@ -828,7 +832,7 @@ __device__ __forceinline__ float2 sinc_series(float2 h) {
 // tri_back with the polarisation block's |h|^2 and tt (for the shared reciprocal
 // square root below).
 struct TriF {
-    float2 lo, mid, hi, Dh, h1, h2, s1, k1, s2, k2, p12, S1, S2;
+    float2 lo, mid, hi, Dh, s1, k1, s2, k2, p12, S1, S2;
 };
 __device__ __forceinline__ TriF tri_front(float2 t1, float2 t2, float2 t3) {
     TriF F;
@@ -847,75 +851,63 @@ __device__ __forceinline__ TriF tri_front(float2 t1, float2 t2, float2 t3) {
     const float2 h1 = add2(mid, neg2(lo));
     const float2 h2 = add2(hi, neg2(mid));
     const float2 c1 = add2(lo, mid), c2 = add2(mid, hi);
-    float2 s1, k1, s2, k2;
-    s1 = make_float2(sin_fz(c1.x), sin_fz(c1.y));
-    k1 = make_float2(cos_fz(c1.x), cos_fz(c1.y));
-    s2 = make_float2(sin_fz(c2.x), sin_fz(c2.y));
-    k2 = make_float2(cos_fz(c2.x), cos_fz(c2.y));
+    F.s1 = make_float2(sin_fz(c1.x), sin_fz(c1.y));
+    F.k1 = make_float2(cos_fz(c1.x), cos_fz(c1.y));
+    F.s2 = make_float2(sin_fz(c2.x), sin_fz(c2.y));
+    F.k2 = make_float2(cos_fz(c2.x), cos_fz(c2.y));
     // With a1 = max(h1, .5) and a2 = max(h2, .5), 2 sc g = scr (S1 e^{i c1} -
     // S2 e^{i c2}) (imaginary unit and sign aside), S1 = sinc(h1) a1 a2,
     // S2 = sinc(h2) a1 a2 and scr = sc / (a1 a2 Dh): one reciprocal square root,
     // rsqrt(hn2 (tt a1 a2 Dh)^2), gives the polarisation block's normalisation,
-    // 1/a1, 1/a2 and 2/D.  Where h >= 0.5, sinc(h1) a1 a2 = a2 sin(h1).
+    // 1/a1, 1/a2 and 2/D.  sinc(h1) a1 is sin(h1) where h1 >= 0.5 and half of the
+    // sinc series below.  Some lane of a warp nearly always needs the series (two of
+    // a triangle's phases within 1 rad), so every lane forms it, without a vote.
     const float2 a1 = make_float2(fmaxf(h1.x, 0.5f), fmaxf(h1.y, 0.5f));
     const float2 a2 = make_float2(fmaxf(h2.x, 0.5f), fmaxf(h2.y, 0.5f));
-    const float2 p12 = mul2(a1, a2);
-    F.lo = lo; F.mid = mid; F.hi = hi; F.Dh = Dh; F.h1 = h1; F.h2 = h2;
-    F.s1 = s1; F.k1 = k1; F.s2 = s2; F.k2 = k2; F.p12 = p12;
-    F.S1 = mul2(make_float2(sin_fz(h1.x), sin_fz(h1.y)), a2);
-    F.S2 = mul2(make_float2(sin_fz(h2.x), sin_fz(h2.y)), a1);
+    F.lo = lo; F.mid = mid; F.hi = hi; F.Dh = Dh;
+    F.p12 = mul2(a1, a2);
+    F.S1 = mul2(sel2(h1.x < 0.5f, h1.y < 0.5f, half_sinc_series(h1),
+                     make_float2(sin_fz(h1.x), sin_fz(h1.y))), a2);
+    F.S2 = mul2(sel2(h2.x < 0.5f, h2.y < 0.5f, half_sinc_series(h2),
+                     make_float2(sin_fz(h2.x), sin_fz(h2.y))), a1);
     return F;
 }
 
 __device__ __forceinline__ void tri_back(const TriF &F, float2 hn2, float2 tt, float2 &gx, float2 &gy) {
-    const float2 lo = F.lo, mid = F.mid, hi = F.hi, Dh = F.Dh, h1 = F.h1, h2 = F.h2;
-    const float2 s1 = F.s1, k1 = F.k1, s2 = F.s2, k2 = F.k2, p12 = F.p12;
-    const float2 q = mul2(mul2(p12, Dh), tt);
+    const float2 Dh = F.Dh;
+    const float2 q = mul2(mul2(F.p12, Dh), tt);
     const float2 hq = mul2(hn2, mul2(q, q));
     const float2 scr = make_float2(rsqrt_fz(hq.x), rsqrt_fz(hq.y));
-    float2 S1 = F.S1, S2 = F.S2;
-    // below h = 0.5 sinc(h) from its series, evaluated only when a lane of the
-    // warp needs it (small gaps occur near a facet's specular and forward
-    // directions), one vote for both
-    const bool ax = h1.x < 0.5f, ay = h1.y < 0.5f, bx = h2.x < 0.5f, by = h2.y < 0.5f;
-    if (__any_sync(0xffffffffu, ax || ay || bx || by)) {
-        S1 = sel2(ax, ay, mul2(sinc_series(h1), p12), S1);
-        S2 = sel2(bx, by, mul2(sinc_series(h2), p12), S2);
-        gx = mul2(fma2(S1, s1, neg2(mul2(S2, s2))), scr);
-        gy = mul2(fma2(S2, k2, neg2(mul2(S1, k1))), scr);
-        if (Dh.x < 0.125f || Dh.y < 0.125f) {
-            // all three full phases within 0.25 rad: Taylor series about the middle
-            // phase, g = e^{2i mid} sum_n i^(n+2)/(n+2)! q_n(ya, yc) with the complete
-            // homogeneous q_n of the full-phase offsets 2 ya, 2 yc (2^n folded into
-            // the coefficients)
-            const float2 ya = add2(lo, neg2(mid)), yc = add2(hi, neg2(mid));
-            const float2 q1 = add2(ya, yc);
-            const float2 ya2 = mul2(ya, ya);
-            const float2 q2 = fma2(yc, q1, ya2);
-            const float2 ya3 = mul2(ya2, ya);
-            const float2 q3 = fma2(yc, q2, ya3);
-            const float2 ya4 = mul2(ya3, ya);
-            const float2 q4 = fma2(yc, q3, ya4);
-            const float2 q5 = fma2(yc, q4, mul2(ya4, ya));
-            const float2 q6 = fma2(yc, q5, mul2(ya4, ya2));
-            const float2 ht = mul2(mul2(hn2, tt), tt);
-            const float2 tsc = make_float2(2.0f * rsqrt_fz(ht.x), 2.0f * rsqrt_fz(ht.y));
-            const float2 re = mul2(tsc, fma2(q6, bc2(1.0f / 630.0f),
-                                             fma2(q4, bc2(-1.0f / 45.0f), fma2(q2, bc2(1.0f / 6.0f), bc2(-0.5f)))));
-            const float2 im = mul2(tsc, fma2(q5, bc2(-2.0f / 315.0f),
-                                             fma2(q3, bc2(1.0f / 15.0f), mul2(q1, bc2(-1.0f / 3.0f)))));
-            const float2 m2 = add2(mid, mid);
-            float2 sm, cm;
-            sm = make_float2(sin_fz(m2.x), sin_fz(m2.y));
-            cm = make_float2(cos_fz(m2.x), cos_fz(m2.y));
-            const float2 sx = fma2(cm, re, neg2(mul2(sm, im)));
-            const float2 sy = fma2(cm, im, mul2(sm, re));
-            gx = sel2(Dh.x < 0.125f, Dh.y < 0.125f, sx, gx);
-            gy = sel2(Dh.x < 0.125f, Dh.y < 0.125f, sy, gy);
-        }
-    } else {
-        gx = mul2(fma2(S1, s1, neg2(mul2(S2, s2))), scr);
-        gy = mul2(fma2(S2, k2, neg2(mul2(S1, k1))), scr);
+    gx = mul2(fma2(F.S1, F.s1, neg2(mul2(F.S2, F.s2))), scr);
+    gy = mul2(fma2(F.S2, F.k2, neg2(mul2(F.S1, F.k1))), scr);
+    if (Dh.x < 0.125f || Dh.y < 0.125f) {
+        // all three full phases within 0.25 rad: Taylor series about the middle
+        // phase, g = e^{2i mid} sum_n i^(n+2)/(n+2)! q_n(ya, yc) with the complete
+        // homogeneous q_n of the full-phase offsets 2 ya, 2 yc (2^n folded into
+        // the coefficients)
+        const float2 ya = add2(F.lo, neg2(F.mid)), yc = add2(F.hi, neg2(F.mid));
+        const float2 q1 = add2(ya, yc);
+        const float2 ya2 = mul2(ya, ya);
+        const float2 q2 = fma2(yc, q1, ya2);
+        const float2 ya3 = mul2(ya2, ya);
+        const float2 q3 = fma2(yc, q2, ya3);
+        const float2 ya4 = mul2(ya3, ya);
+        const float2 q4 = fma2(yc, q3, ya4);
+        const float2 q5 = fma2(yc, q4, mul2(ya4, ya));
+        const float2 q6 = fma2(yc, q5, mul2(ya4, ya2));
+        const float2 ht = mul2(mul2(hn2, tt), tt);
+        const float2 tsc = make_float2(2.0f * rsqrt_fz(ht.x), 2.0f * rsqrt_fz(ht.y));
+        const float2 re = mul2(tsc, fma2(q6, bc2(1.0f / 630.0f),
+                                         fma2(q4, bc2(-1.0f / 45.0f), fma2(q2, bc2(1.0f / 6.0f), bc2(-0.5f)))));
+        const float2 im = mul2(tsc, fma2(q5, bc2(-2.0f / 315.0f),
+                                         fma2(q3, bc2(1.0f / 15.0f), mul2(q1, bc2(-1.0f / 3.0f)))));
+        const float2 m2 = add2(F.mid, F.mid);
+        const float2 sm = make_float2(sin_fz(m2.x), sin_fz(m2.y));
+        const float2 cm = make_float2(cos_fz(m2.x), cos_fz(m2.y));
+        const float2 sx = fma2(cm, re, neg2(mul2(sm, im)));
+        const float2 sy = fma2(cm, im, mul2(sm, re));
+        gx = sel2(Dh.x < 0.125f, Dh.y < 0.125f, sx, gx);
+        gy = sel2(Dh.x < 0.125f, Dh.y < 0.125f, sy, gy);
     }
 }
 
@@ -929,7 +921,7 @@ __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
 
 template <bool FAST>
 __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const BinPk &B,
-                                        float2 (&acc)[8], float2 nkh, float2 hkRh, float2 sgh,
+                                        float2 (&acc)[8], float2 nkh, float2 hkRh,
                                         const float (&hb)[3][K2P_HB], bool lo_ok, bool hi_ok,
                                         const double *__restrict__ xyz, int64_t nb,
                                         const float2 *__restrict__ rl) {
@@ -950,64 +942,50 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     float2 eps0, eps1, eps2, pb;
     ld22(&P.eps[0], eps0, eps1);
     ld22(&P.eps[2], eps2, pb);
-    // a = u . eps = s . eps - sg eps_z
-    const float2 a = fma2(neg2(B.sg), eps2, fma2(B.sz, eps2, fma2(B.fy, eps1, mul2(B.fx, eps0))));
-    // with y = b - a^2: half phase hkRh y (1 + a) - rf, and
-    // opa2 = 1 + a + 1.5 a^2 - 0.5 b = (1 + a) - 0.5 y + a^2
-    const float2 opa = add2(one, a);
-    const float2 y = fma2(neg2(a), a, pb);
+    const float2 al = fma2(B.fz, eps2, fma2(B.fy, eps1, mul2(B.fx, eps0)));  // u . eps
+    // with y = b - al^2: half phase hkRh y (1 + al) - rf, and
+    // opa2 = 1 + al + 1.5 al^2 - 0.5 b = (1 + al) - 0.5 y + al^2
+    const float2 opa = add2(one, al);
+    const float2 y = fma2(neg2(al), al, pb);
     const float2 ph = fma2(mul2(hkRh, y), opa, neg2(rf));
-    const float2 opa2 = fma2(a, a, fma2(bc2(-0.5f), y, opa));
-    // The bin direction enters through s = u + sg z (sg = +1 in the hemisphere of
-    // the incidence direction (0,0,-1), -1 in the other), which is small and known
-    // to full FP32 precision near both poles.  With inc = -R z (the incidence
-    // direction in the aperture frame), k = R u opa2 + nea opa = ks + sg opa2 inc
-    // with ks = R s opa2 + nea opa, and the normal of the scattering plane is
-    // h = inc x k = inc x ks: no cancellation of nearly parallel unit vectors near
-    // the forward and backward directions, where |h| is small.
-    float2 ks0, ks1, ks2;
+    const float2 opa2 = fma2(al, al, fma2(bc2(-0.5f), y, opa));
+    // The unit direction from the facet centre in the lab frame, (a, b, c) = u opa2 -
+    // eps opa, and k = R (a, b, c) in the aperture frame.  The normal of the
+    // scattering plane, h = inc x k with inc = (0, 0, -1), is (b, -a, 0): formed from
+    // the lab components it has no cancellation of nearly parallel unit vectors near
+    // the forward and backward directions, where a and b are small and known to full
+    // FP32 precision.
+    const float2 a = fma2(B.fx, opa2, neg2(mul2(eps0, opa)));
+    const float2 b = fma2(B.fy, opa2, neg2(mul2(eps1, opa)));
+    const float2 c = fma2(B.fz, opa2, neg2(mul2(eps2, opa)));
+    float2 r3, r4, r5, kp, kx, ky, kz, u;
     {
-        float2 r0, r1, r2, r3, r4, r5, r6, r7, r8, n0, n1, n2;
+        float2 r0, r1, r2, r6, r7, r8;
         ld22(&P.R[0], r0, r1);
         ld22(&P.R[2], r2, r3);
         ld22(&P.R[4], r4, r5);
         ld22(&P.R[6], r6, r7);
-        ld22(&P.R[8], r8, n0);
-        ld22(&P.nea[1], n1, n2);
-        const float2 w0 = fma2(r2, B.sz, fma2(r1, B.fy, mul2(r0, B.fx)));
-        const float2 w1 = fma2(r5, B.sz, fma2(r4, B.fy, mul2(r3, B.fx)));
-        const float2 w2 = fma2(r8, B.sz, fma2(r7, B.fy, mul2(r6, B.fx)));
-        ks0 = fma2(w0, opa2, mul2(n0, opa));
-        ks1 = fma2(w1, opa2, mul2(n1, opa));
-        ks2 = fma2(w2, opa2, mul2(n2, opa));
-    }
-    float2 kzc, inc0, inc1, inc2;
-    ld22(&P.kzc, kzc, inc0);
-    ld22(&P.inc[1], inc1, inc2);
-    const float2 so = mul2(B.sg, opa2);
-    float2 kx = fma2(so, inc0, ks0);
-    const float2 ky = fma2(so, inc1, ks1);
-    float2 kz = fma2(so, inc2, ks2);
-    // aperture wave vector (halved with the phases)
-    float2 kxx, kyy;
-    {
-        float2 kp0, kp1;
-        ld22(&P.kp[0], kp0, kp1);
-        kxx = fma2(nkh, kx, kp0);
-        kyy = fma2(nkh, ky, kp1);
+        ld22(&P.R[8], r8, kp);
+        kx = fma2(r2, c, fma2(r1, b, mul2(r0, a)));
+        u = fma2(r4, b, mul2(r3, a));
+        ky = fma2(r5, c, u);
+        kz = fma2(r8, c, fma2(r7, b, mul2(r6, a)));
     }
     // the divided difference's phases, sort, sines and cosines: independent of
     // the polarisation block and its rare branch, so formed ahead of the branch
-    // (one basic block with the direction arithmetic for the scheduler)
+    // (one basic block with the direction arithmetic for the scheduler).  The
+    // aperture wave vector's x part is halved with the phases; its y part is ky
+    // times the factor that vy carries.
     TriF tf;
     {
+        const float2 kxx = fma2(nkh, kx, kp);
         float2 vx0, vx1, vx2, vy0, vy1, vy2;
         ld22(&P.vx[0], vx0, vx1);
         ld22(&P.vx[2], vx2, vy0);
         ld22(&P.vy[1], vy1, vy2);
-        const float2 t1 = fma2(kyy, vy0, fma2(kxx, vx0, ph));
-        const float2 t2 = fma2(kyy, vy1, fma2(kxx, vx1, ph));
-        const float2 t3 = fma2(kyy, vy2, fma2(kxx, vx2, ph));
+        const float2 t1 = fma2(ky, vy0, fma2(kxx, vx0, ph));
+        const float2 t2 = fma2(ky, vy1, fma2(kxx, vx1, ph));
+        const float2 t3 = fma2(ky, vy2, fma2(kxx, vx2, ph));
         tf = tri_front(t1, t2, t3);
     }
     // Polarisation matrix [[d, e], [-e, d]] (see k2_record for the forms) and
@@ -1020,39 +998,42 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     // rounding and d1 = (sqrt(1 - Ky^2)/2) (kzc tt - kz), e1 = (sqrt(1 - Ky^2)/2)(-kx kyc)
     // (the Kx Ky term is below 1e-16 and left out); the common factor is in the
     // record's amplitudes and sc in the divided difference.
-    // Main path: |ky| < 0.999999 (no clamp) and no forward bodge, so kyc = ky
-    // and tt = kx^2 + kz^2; h = inc x (kx, ky, kz) = inc x ks.
+    // Main path: |ky| < 0.999999 (no clamp) and no forward bodge, so kyc = ky,
+    // tt = kx^2 + kz^2 and h is normal to k.  Then P1 = p |h| s = hy tt - kyc (hx kx +
+    // hz kz) is hy |k|^2 = hy (|k| = 1 up to rounding) and R1 = rr |h| s =
+    // hz kx - hx kz = -y . (k x h), with k x h = (c a, c b, -|h|^2) in the lab frame
+    // and y = (r3, r4, r5) the frame's second axis: neither needs h in the aperture
+    // frame.
     const float2 tr = fma2(kx, kx, mul2(kz, kz));
     float2 tt = tr;
-    float2 d1 = fma2(kzc, tr, neg2(kz));
-    float2 e1 = mul2(neg2(kx), ky);
-    float2 hx = fma2(inc1, ks2, neg2(mul2(inc2, ks1)));
-    float2 hy = fma2(inc2, ks0, neg2(mul2(inc0, ks2)));
-    float2 hz = fma2(inc0, ks1, neg2(mul2(inc1, ks0)));
-    // P1 = p |h| s = hy tt - kyc (hx kx + hz kz), from m = (-kx ky / s, s, -kz ky / s).
-    // Where h is normal to q = (kx, kyc, kz), hx kx + hz kz = -hy kyc and
-    // P1 = hy (tt + kyc^2) = hy |q|^2 = hy (|q| = 1 up to rounding; on the clamp
-    // tt + kyc^2 = 1 - c^2 + c^2); the forward bodge takes the general form.
-    // Inside the clamp evo2 = (-kz, 0, kx) / s, so R1 = rr |h| s = hz kx - hx kz.
-    float2 P1 = hy, R1;
+    float2 d1, e1;
+    float2 hn2 = fma2(a, a, mul2(b, b));
+    float2 P1 = fma2(r3, b, neg2(mul2(r4, a)));
+    float2 R1 = fma2(r5, hn2, neg2(mul2(c, u)));
+    float2 kzc = P.kzc;
     const bool cx = tr.x <= kOneMinusClampSq, cy = tr.y <= kOneMinusClampSq;
     if (B.pole || cx || cy) {
+        float2 r0, r1, r2, r6, r7, r8, q3, q4, q5, q9;
+        ld22(&P.R[0], r0, r1);
+        ld22(&P.R[2], r2, q3);
+        ld22(&P.R[4], q4, q5);
+        ld22(&P.R[6], r6, r7);
+        ld22(&P.R[8], r8, q9);
+        // h in the aperture frame, R (b, -a, 0)
+        float2 hx = fma2(r0, b, neg2(mul2(r1, a)));
+        float2 hz = fma2(r6, b, neg2(mul2(r7, a)));
+        float2 hy = P1;
         if (cx || cy) {
             // on the clamp: kx and kz from v = u - sigma R_1 (see clamp_v)
-            float2 a0, a1, a2, a3, a4, a5, c6, c7, c8, n0, n1, n2;
-            ld22(&P.R[0], a0, a1);
-            ld22(&P.R[2], a2, a3);
-            ld22(&P.R[4], a4, a5);
-            ld22(&P.R[6], c6, c7);
-            ld22(&P.R[8], c8, n0);
-            ld22(&P.nea[1], n1, n2);
             const float2 l0 = rl[0], l1 = rl[1], l2 = rl[2];
             const float sx = ky.x < 0.0f ? -1.0f : 1.0f, sy = ky.y < 0.0f ? -1.0f : 1.0f;
-            const float2 v0 = make_float2(clamp_v(a3.x, l0.x, B.ux, sx), clamp_v(a3.y, l0.y, B.ux, sy));
-            const float2 v1 = make_float2(clamp_v(a4.x, l1.x, B.uy, sx), clamp_v(a4.y, l1.y, B.uy, sy));
-            const float2 v2 = make_float2(clamp_v(a5.x, l2.x, B.uz, sx), clamp_v(a5.y, l2.y, B.uz, sy));
-            const float2 kxa = fma2(fma2(a2, v2, fma2(a1, v1, mul2(a0, v0))), opa2, mul2(n0, opa));
-            const float2 kza = fma2(fma2(c8, v2, fma2(c7, v1, mul2(c6, v0))), opa2, mul2(n2, opa));
+            const float2 v0 = make_float2(clamp_v(r3.x, l0.x, B.ux, sx), clamp_v(r3.y, l0.y, B.ux, sy));
+            const float2 v1 = make_float2(clamp_v(r4.x, l1.x, B.uy, sx), clamp_v(r4.y, l1.y, B.uy, sy));
+            const float2 v2 = make_float2(clamp_v(r5.x, l2.x, B.uz, sx), clamp_v(r5.y, l2.y, B.uz, sy));
+            const float2 e0 = fma2(r2, eps2, fma2(r1, eps1, mul2(r0, eps0)));
+            const float2 e2 = fma2(r8, eps2, fma2(r7, eps1, mul2(r6, eps0)));
+            const float2 kxa = fma2(fma2(r2, v2, fma2(r1, v1, mul2(r0, v0))), opa2, neg2(mul2(e0, opa)));
+            const float2 kza = fma2(fma2(r8, v2, fma2(r7, v1, mul2(r6, v0))), opa2, neg2(mul2(e2, opa)));
             kx = sel2(cx, cy, kxa, kx);
             kz = sel2(cx, cy, kza, kz);
         }
@@ -1066,28 +1047,21 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
         bool bx = false, by = false;
         if (B.pole) {
             // the forward bodge (src/diff_mod.f90:630-633) can apply only in bins near
-            // the poles; dinc = inc . (kx, kyc, kz)
-            const float2 dinc = fma2(inc2, kz, fma2(inc1, kyc, mul2(inc0, kx)));
+            // the poles; dinc = z . (kx, kyc, kz) = -inc . (kx, kyc, kz)
+            const float2 dinc = fma2(r8, kz, fma2(r5, kyc, mul2(r2, kx)));
             bx = !(fabsf(dinc.x) < 0.999f);
             by = !(fabsf(dinc.y) < 0.999f);
             if (bx || by) {
-                // the bodge direction in the s form: hs = uh + sgh z, uh . eps = hs . eps - sgh eps_z,
-                // h = inc x (R hs oh2 + nea oh)
-                const float2 hx_ = bc2(hb[0][B.hslot]), hy_ = bc2(hb[1][B.hslot]),
-                             hsz = bc2(hb[2][B.hslot]);
-                float2 ah = fma2(hsz, eps2, fma2(hy_, eps1, mul2(hx_, eps0)));
-                ah = fma2(neg2(sgh), eps2, ah);
+                // h from the direction (ba, bb, .) from the facet to the bodge's bin
+                const float2 ux = bc2(hb[0][B.hslot]), uy = bc2(hb[1][B.hslot]), uz = bc2(hb[2][B.hslot]);
+                const float2 ah = fma2(uz, eps2, fma2(uy, eps1, mul2(ux, eps0)));
                 const float2 oh = add2(one, ah);
                 const float2 oh2 = fma2(ah, fma2(bc2(1.5f), ah, one), fma2(bc2(-0.5f), pb, one));
-                const float2 vx = fma2(fma2(P.R[2], hsz, fma2(P.R[1], hy_, mul2(P.R[0], hx_))), oh2,
-                                       mul2(P.nea[0], oh));
-                const float2 vy = fma2(fma2(P.R[5], hsz, fma2(P.R[4], hy_, mul2(P.R[3], hx_))), oh2,
-                                       mul2(P.nea[1], oh));
-                const float2 vz = fma2(fma2(P.R[8], hsz, fma2(P.R[7], hy_, mul2(P.R[6], hx_))), oh2,
-                                       mul2(P.nea[2], oh));
-                const float2 gx = fma2(inc1, vz, neg2(mul2(inc2, vy)));
-                const float2 gy = fma2(inc2, vx, neg2(mul2(inc0, vz)));
-                const float2 gz = fma2(inc0, vy, neg2(mul2(inc1, vx)));
+                const float2 ba = fma2(ux, oh2, neg2(mul2(eps0, oh)));
+                const float2 bb = fma2(uy, oh2, neg2(mul2(eps1, oh)));
+                const float2 gx = fma2(r0, bb, neg2(mul2(r1, ba)));
+                const float2 gy = fma2(r3, bb, neg2(mul2(r4, ba)));
+                const float2 gz = fma2(r6, bb, neg2(mul2(r7, ba)));
                 const float2 gP = fma2(gy, tt, neg2(mul2(kyc, fma2(gx, kx, mul2(gz, kz)))));
                 hx = sel2(bx, by, gx, hx);
                 hy = sel2(bx, by, gy, hy);
@@ -1095,16 +1069,14 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
                 P1 = sel2(bx, by, gP, P1);
             }
         }
+        float2 Rq = fma2(hz, kx, neg2(mul2(hx, kz)));
         if (cx || cy) {
             // a lane on the clamp: outside the bodge, h = inc x (kx, kyc, kz) takes the
-            // clamped ky (q_y = ks1 + kyc - ky); evo2 = normalise(k x m) with the clamped
-            // ky, R1 = s (h . evo2)
-            const float2 qy = add2(ks1, add2(kyc, neg2(ky)));
-            const float2 fx = fma2(inc1, ks2, neg2(mul2(inc2, qy)));
-            const float2 fz = fma2(inc0, qy, neg2(mul2(inc1, ks0)));
+            // clamped ky; evo2 = normalise(k x m) with the clamped ky, R1 = s (h . evo2)
+            const float2 dk = add2(kyc, neg2(ky));
             const bool ux = cx && !bx, uy = cy && !by;
-            hx = sel2(ux, uy, fx, hx);
-            hz = sel2(ux, uy, fz, hz);
+            hx = sel2(ux, uy, fma2(r8, dk, hx), hx);
+            hz = sel2(ux, uy, fma2(neg2(r2), dk, hz), hz);
             const float2 rs = make_float2(rsqrtf(tt.x), rsqrtf(tt.y));
             const float2 s = mul2(tt, rs), kyrs = mul2(kyc, rs);
             const float2 m0 = neg2(mul2(kx, kyrs)), m1 = s, m2 = neg2(mul2(kz, kyrs));
@@ -1114,14 +1086,16 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
             const float2 en2 = fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
             const float2 ne = make_float2(cx ? rsqrtf(en2.x) : 1.0f, cy ? rsqrtf(en2.y) : 1.0f);
             const float2 rc = mul2(mul2(s, ne), fma2(hz, ez, fma2(hy, ey, mul2(hx, ex))));
-            R1 = sel2(cx, cy, rc, fma2(hz, kx, neg2(mul2(hx, kz))));
-        } else {
-            R1 = fma2(hz, kx, neg2(mul2(hx, kz)));
+            Rq = sel2(cx, cy, rc, fma2(hz, kx, neg2(mul2(hx, kz))));
         }
+        // lanes of the main form (an ordinary bin beside a clamped one) keep it
+        const bool gx_ = bx || cx, gy_ = by || cy;
+        R1 = sel2(gx_, gy_, Rq, R1);
+        hn2 = sel2(gx_, gy_, fma2(hz, hz, fma2(hy, hy, mul2(hx, hx))), hn2);
     } else {
-        R1 = fma2(hz, kx, neg2(mul2(hx, kz)));
+        d1 = fma2(kzc, tr, neg2(kz));
+        e1 = mul2(neg2(kx), ky);
     }
-    const float2 hn2 = fma2(hz, hz, fma2(hy, hy, mul2(hx, hx)));
     const float2 A = fma2(P1, d1, mul2(R1, e1));
     const float2 Bc = fma2(P1, e1, neg2(mul2(R1, d1)));
     // aperture integral on the half phases, its second half (the normalisation
@@ -1136,12 +1110,9 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     bool ok_x = lo_ok, ok_y = hi_ok;
     if (FAST) {
         // the field-of-view test (direction from the facet centre, lab frame)
-        const float2 dx = fma2(B.fx, opa, neg2(eps0));
-        const float2 dy = fma2(B.fy, opa, neg2(eps1));
-        const float2 dz = fma2(add2(B.sz, neg2(B.sg)), opa, neg2(eps2));
         const K2Fov &fa = fv[0], &fb = fv[1];
-        const float dpx = fmaf(dz.x, fa.p0[2], fmaf(dy.x, fa.p0[1], dx.x * fa.p0[0]));
-        const float dpy = fmaf(dz.y, fb.p0[2], fmaf(dy.y, fb.p0[1], dx.y * fb.p0[0]));
+        const float dpx = fmaf(c.x, fa.p0[2], fmaf(b.x, fa.p0[1], a.x * fa.p0[0]));
+        const float dpy = fmaf(c.y, fb.p0[2], fmaf(b.y, fb.p0[1], a.y * fb.p0[0]));
         bool in_x = !(dpx < fa.cos_fov), in_y = !(dpy < fb.cos_fov);
         if (ok_x && fabsf(dpx - fa.cos_fov) < fa.tol) in_x = fov_exact(fa, xyz, nb, B.bin);
         if (ok_y && fabsf(dpy - fb.cos_fov) < fb.tol) in_y = fov_exact(fb, xyz, nb, B.bin);
@@ -1157,12 +1128,12 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     }
     // acc: (U+ col 1, U- col 1, U+ col 2, U- col 2), re/im
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const float2 qr = (c & 1) ? qmr : qpr, qi = (c & 1) ? qmi : qpi;
+    for (int q = 0; q < 4; q++) {
+        const float2 qr = (q & 1) ? qmr : qpr, qi = (q & 1) ? qmi : qpi;
         float2 ur, ui;
-        ld22(&P.amp[2 * c], ur, ui);
-        acc[2 * c] = fma2(qr, ur, fma2(neg2(qi), ui, acc[2 * c]));
-        acc[2 * c + 1] = fma2(qr, ui, fma2(qi, ur, acc[2 * c + 1]));
+        ld22(&P.amp[2 * q], ur, ui);
+        acc[2 * q] = fma2(qr, ur, fma2(neg2(qi), ui, acc[2 * q]));
+        acc[2 * q + 1] = fma2(qr, ui, fma2(qi, ur, acc[2 * q + 1]));
     }
 }
 
@@ -1196,7 +1167,6 @@ struct K2PkArgs {
     int64_t theta_i;
     float k;
     float hkR;
-    float sgh;   // +1 when the bodge row theta_i lies in the hemisphere of (0,0,-1), else -1
     const unsigned *epsmax;  // float bits of a bound of |com| / R over the records
     double *ws;         // [seg][8][nb]
     unsigned *tickets;  // [seg][tile], splits added so far
@@ -1211,7 +1181,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
     __shared__ __align__(8) uint64_t bars[K2_NST];
     __shared__ long long s_item;
     __shared__ unsigned s_keep[2];  // is_fast_diff: records of the stage not culled for the tile
-    __shared__ float s_hb[3][K2P_HB];  // forward-bodge bin directions of this CTA's bins (s form)
+    __shared__ float s_hb[3][K2P_HB];  // forward-bodge bin directions of this CTA's bins
     __shared__ int s_ok;
     const int tid = threadIdx.x;
     if (tid == 0) {
@@ -1223,7 +1193,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
     const int64_t total = P.item_pre[P.nseg];
     constexpr int64_t TILE = (int64_t)K2_THREADS * BPT;
     // half phases: -k/2 and k R / 4
-    const float2 nkh = bc2(-0.5f * P.k), hkRh = bc2(0.5f * P.hkR), sgh = bc2(P.sgh);
+    const float2 nkh = bc2(-0.5f * P.k), hkRh = bc2(0.5f * P.hkR);
     // bins with |uz| below pole_cos are out of reach of the forward bodge for every
     // record: |inc . k - (-uz)| <= 2 |com| / R for the direction k from a facet centre
     const float pole_cos = 0.999f - 2.0f * __uint_as_float(*P.epsmax) - 1e-5f;
@@ -1262,9 +1232,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             bd[q].uz = Zc * ir;
             bd[q].fx = bc2((float)bd[q].ux);
             bd[q].fy = bc2((float)bd[q].uy);
-            const double sg = bd[q].uz <= 0.0 ? 1.0 : -1.0;
-            bd[q].sz = bc2((float)(bd[q].uz + sg));
-            bd[q].sg = bc2((float)sg);
+            bd[q].fz = bc2((float)bd[q].uz);
             bd[q].pole = !(fabs(bd[q].uz) < (double)pole_cos);
             const int64_t oh = (o % P.nphi) + P.nphi * P.theta_i;
             const double Xh = P.xyz[oh], Yh = P.xyz[P.nb + oh], Zh = P.xyz[2 * P.nb + oh];
@@ -1272,7 +1240,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             bd[q].hslot = q * K2_THREADS + tid;
             s_hb[0][bd[q].hslot] = (float)(Xh * irh);
             s_hb[1][bd[q].hslot] = (float)(Yh * irh);
-            s_hb[2][bd[q].hslot] = (float)(Zh * irh + (double)P.sgh);
+            s_hb[2][bd[q].hslot] = (float)(Zh * irh);
         }
         double acc64[BPT][8];
 #pragma unroll
@@ -1300,12 +1268,12 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             const bool ok = mbar_wait(smem_u32(&bars[st]), (parity >> st) & 1u);
             parity ^= 1u << st;
             const int n = (int)min((int64_t)CH, npair - c * CH);
-            if (!FAST && ok && tid < 39) {
+            if (!FAST && ok && tid < 33) {
                 // The item's first pair (odd rbeg) and last pair (odd rend) hold a
                 // record of another item or the array's padding: that half takes a
                 // copy of the pair's other record with zero amplitude, so the pair
                 // loop needs no per-pair range test.  Threads 0-2 copy the FP64
-                // phase, threads 3-38 the 36 float2 fields from eps on (the last 8
+                // phase, threads 3-32 the 30 float2 fields from eps on (the last 8
                 // are the amplitudes); the barrier below publishes the copy.
                 auto patch = [&](int j, int src, int dst) {
                     K2Pair &Q = sbuf[st][j];
@@ -1314,7 +1282,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     } else {
                         float2 *f = &Q.eps[0];
                         const int i = tid - 3;
-                        const float v = i >= 28 ? 0.0f : (src ? f[i].y : f[i].x);
+                        const float v = i >= 22 ? 0.0f : (src ? f[i].y : f[i].x);
                         if (dst)
                             f[i].y = v;
                         else
@@ -1362,7 +1330,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                 // patched above; a bin beyond nb is never written out)
 #pragma unroll
                 for (int q = 0; q < BPT; q++)
-                    k2_pair<FAST>(sbuf[st][j], fv, bd[q], acc[q], nkh, hkRh, sgh, s_hb,
+                    k2_pair<FAST>(sbuf[st][j], fv, bd[q], acc[q], nkh, hkRh, s_hb,
                                   FAST ? (lo_ok && valid[q]) : true,
                                   FAST ? (hi_ok && valid[q]) : true, P.xyz, P.nb,
                                   P.rlo + (p0 + c * CH + j) * 3);
@@ -1994,7 +1962,6 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
         B.theta_i = A.theta_i;
         B.k = A.k;
         B.hkR = A.hkR;
-        B.sgh = A.sgh;
         B.epsmax = S.epsmax;
         B.ws = ws;
         B.tickets = A.tickets;
