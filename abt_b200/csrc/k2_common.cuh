@@ -56,18 +56,18 @@ namespace pbt {
 // Two triangle records interleaved field by field (x = even record, y = odd
 // record), so that a shared-memory load of a float2 yields the operand pair of
 // a packed FP32x2 instruction evaluating two facets at once.  The packed kernel
-// works with half phases (kc and kp are halved, vy carries the factor -k/2 of
-// ky) and with the Karczewski-Wolf block divided by its factor sqrt(1 - Ky^2) / 2,
+// works with half phases (kc is halved and in units of pi, the vertices carry the factor -k/2 of the
+// aperture wave vector (kx - Kx, ky)) and with the Karczewski-Wolf block divided by its factor sqrt(1 - Ky^2) / 2,
 // which goes into the amplitudes together with the 1/2 of the half-phase divided
 // difference.  Every pair of adjacent float2 fields from eps on starts on a
 // 16-byte boundary, so the kernel reads them two at a time.  288 bytes.
 struct __align__(16) K2Pair {
-    double kc[3][2];  // k * com / 2, [component][half]
+    double kc[3][2];  // k * com / (2 pi), [component][half]
     float2 eps[3];
     float2 b;
     float2 R[9];
-    float2 kp;        // k * prop2(x) / 2; prop2(y) = 0 up to rounding (the set-up's in-plane rotation)
-    float2 vx[3], vy[3];  // vertices; y times -k/2
+    float2 nKx;       // -prop2(x); prop2(y) = 0 up to rounding (the set-up's in-plane rotation)
+    float2 vx[3], vy[3];  // vertices times -k/2
     float2 kzc;       // -Kz / (1 - Ky^2)
     float2 pad;
     float2 amp[8];    // the amplitude columns in the circular basis, u+_1, u-_1, u+_2, u-_2

@@ -35,6 +35,7 @@
 #include <stdlib.h>
 
 #include <cub/device/device_scan.cuh>
+#include <type_traits>
 
 #include "frame.h"
 #include "k2_common.cuh"
@@ -50,6 +51,7 @@ constexpr int K2_NST = 3;   // stages
 constexpr double kTwoPi = 6.283185307179586;
 constexpr double kInv2Pi = 0.15915494309189535;
 constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52, round-to-integer constant
+constexpr double kFracMagic = 1572864.0;  // 1.5 * 2^20: an FP64 unit of 2^-32
 constexpr double kPi = 3.141592653589793;
 constexpr double kInvPi = 0.3183098861837907;
 // 1 - c^2 for the reference's clamp c = 0.999999 (a float literal)
@@ -136,11 +138,12 @@ __global__ void k2_count_kernel(RefSrc S, int64_t nrefs, const int64_t *__restri
 
 // Write record r into half r % 2 of pair r / 2 (K2Pair's half-phase and
 // scaled forms): kzc = -Kz / (1 - Ky^2), the circular-basis amplitudes uc
-// times sqrt(1 - Ky^2) / 4 and the scaled vertex ordinates vys, all formed in
-// FP64 by the caller.
+// times sqrt(1 - Ky^2) / 4 and the vertices times -k/2, all formed in FP64 by the
+// caller.
 __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const K2Rec &rec,
                                                 double kzc, const double (&uc)[8],
-                                                const double (&vys)[3]) {
+                                                double Kx, const double (&xa)[3],
+                                                const double (&ya)[3], double nkh) {
     K2Pair &P = pairs[r >> 1];
     const int h = (int)(r & 1);
     auto put = [h](float2 &dst, float v) {
@@ -150,14 +153,14 @@ __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const 
             dst.x = v;
     };
     for (int c = 0; c < 3; c++) {
-        P.kc[c][h] = 0.5 * rec.kc[c];
+        P.kc[c][h] = 0.5 * kInvPi * rec.kc[c];
         put(P.eps[c], rec.eps[c]);
-        put(P.vx[c], rec.vx[c]);
-        put(P.vy[c], (float)vys[c]);
+        put(P.vx[c], (float)(nkh * xa[c]));
+        put(P.vy[c], (float)(nkh * ya[c]));
     }
     put(P.b, rec.b);
     for (int q = 0; q < 9; q++) put(P.R[q], rec.R[q]);
-    put(P.kp, 0.5f * rec.kp[0]);
+    put(P.nKx, (float)-Kx);
     put(P.kzc, (float)kzc);
     for (int q = 0; q < 8; q++) put(P.amp[q], (float)uc[q]);
 }
@@ -261,8 +264,8 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
             const double uc[8] = {sk * (am[0] - am[3]), sk * (am[1] + am[2]), sk * (am[0] + am[3]),
                                   sk * (am[1] - am[2]), sk * (am[4] - am[7]), sk * (am[5] + am[6]),
                                   sk * (am[4] + am[7]), sk * (am[5] - am[6])};
-            const double vys[3] = {-0.5 * waveno * ya[0], -0.5 * waveno * ya[1], -0.5 * waveno * ya[2]};
-            store_pair_half(pairs, r0 + t, rec, -fr.prop2[2] * cf * cf, uc, vys);
+            store_pair_half(pairs, r0 + t, rec, -fr.prop2[2] * cf * cf, uc, fr.prop2[0], xa, ya,
+                            -0.5 * waveno);
         } else {
             recs[r0 + t] = rec;
         }
@@ -394,6 +397,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
         "l"(src), "r"(bytes), "r"(bar)
         : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Bounded wait on an mbarrier phase: false after limit_ns of global time or
 // 2^26 polls, whichever comes first.
@@ -772,10 +778,13 @@ __global__ void __launch_bounds__(K2_THREADS, 2) k2_main_kernel(K2MainArgs P) {
 //
 // Bound: issue.  Over the pair loop the FMA pipe's cycles (an FFMA2 holds it two)
 // and the other instructions add up to 88 % of the cycles, at 16 and 20 warps per SM
-// alike, so only fewer operations help.  With the plane's normal taken from the lab
-// frame (no R s + R e, no h in the aperture frame) and the sinc series formed by
-// every lane instead of behind a vote, 200,000 triangles x 259,560 bins take 224.1 ms
-// (244.8 ms before; the lab frame alone 227.8).
+// alike, so only fewer operations help.  200,000 triangles x 259,560 bins take
+// 217.9 ms: 244.8 before the lab-frame normal (no R s + R e, no h in the aperture
+// frame; 227.8), the sinc series formed by every lane instead of behind a vote
+// (224.1), and the fixed-point phase with the item's state and sums in shared memory
+// (217.9; with CTA barriers between the stages or the sums in registers 224-226, five
+// CTAs per SM with 96 registers 228).  One operation less in the second-order terms
+// ((u - eps) opa2, no 1 + al) came out of the compiler slower, 221.7 ms.
 
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 // the special-function unit's approximations with subnormal inputs flushed
@@ -805,15 +814,13 @@ __device__ __forceinline__ float2 sel2(bool px, bool py, float2 a, float2 b) {
 
 // A bin of the packed kernel: the unit direction in FP64 and as FP32 broadcast
 // pairs.  The forward-bodge bin direction, used near the poles only, is kept in
-// shared memory (slot hslot of the kernel's bodge table).
+// shared memory.
 struct BinPk {
     double ux, uy, uz;     // unit bin direction, FP64
     float2 fx, fy, fz;     // broadcast FP32 pairs
-    int hslot;
     bool pole;             // within reach of the forward bodge (|uz| near 1) for some record
-    int64_t bin;           // bin index
+    int bin;               // bin index, -1: none
 };
-constexpr int K2P_HB = K2_THREADS * 2;  // bodge table slots (bins per thread <= 2)
 
 // sin(h)/(2h) below h = 0.5, where the MUFU sine's absolute error would be a large
 // relative one: half of 1 + c1 h^2 + c2 h^4 with c1, c2 the minimax fit to the
@@ -880,7 +887,8 @@ __device__ __forceinline__ void tri_back(const TriF &F, float2 hn2, float2 tt, f
     const float2 scr = make_float2(rsqrt_fz(hq.x), rsqrt_fz(hq.y));
     gx = mul2(fma2(F.S1, F.s1, neg2(mul2(F.S2, F.s2))), scr);
     gy = mul2(fma2(F.S2, F.k2, neg2(mul2(F.S1, F.k1))), scr);
-    if (Dh.x < 0.125f || Dh.y < 0.125f) {
+    // (uniform over the warp: the lanes that need it select)
+    if (__any_sync(0xffffffffu, Dh.x < 0.125f || Dh.y < 0.125f)) {
         // all three full phases within 0.25 rad: Taylor series about the middle
         // phase, g = e^{2i mid} sum_n i^(n+2)/(n+2)! q_n(ya, yc) with the complete
         // homogeneous q_n of the full-phase offsets 2 ya, 2 yc (2^n folded into
@@ -919,35 +927,42 @@ __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
     b = make_float2(v.z, v.w);
 }
 
-template <bool FAST>
+template <bool FAST, bool WIDE>
 __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const BinPk &B,
-                                        float2 (&acc)[8], float2 nkh, float2 hkRh,
-                                        const float (&hb)[3][K2P_HB], bool lo_ok, bool hi_ok,
+                                        float2 (&acc)[8], float2 hkRh,
+                                        const float4 &hb, bool lo_ok, bool hi_ok,
                                         const double *__restrict__ xyz, int64_t nb,
                                         const float2 *__restrict__ rl) {
-    // far-field half phase per facet: FP64 k u.c / 2, reduced mod pi
-    float2 rf;
+    // far-field half phase per facet, k u.c / 2 modulo pi, as a fixed-point fraction of
+    // pi (2^-32 units): added to 1.5 * 2^20 the FP64 sum's low word is that fraction, so
+    // the reduction costs no operation of its own (each of the three steps rounds to
+    // 2^-32 pi = 7e-10 rad).  That holds up to 2^19 half turns; records beyond (kWide, a
+    // launch with k |com| above 1.6e6) subtract the nearest integer.
+    float2 fr;
     {
         const double2 k0 = *reinterpret_cast<const double2 *>(&P.kc[0][0]);
         const double2 k1 = *reinterpret_cast<const double2 *>(&P.kc[1][0]);
         const double2 k2 = *reinterpret_cast<const double2 *>(&P.kc[2][0]);
-        const double ka = fma(B.uz, k2.x, fma(B.uy, k1.x, B.ux * k0.x));
-        const double nq = fma(ka, kInvPi, kMagic) - kMagic;
-        rf.x = (float)fma(-nq, kPi, ka);
-        const double kb = fma(B.uz, k2.y, fma(B.uy, k1.y, B.ux * k0.y));
-        const double nb = fma(kb, kInvPi, kMagic) - kMagic;
-        rf.y = (float)fma(-nb, kPi, kb);
+        if (!WIDE) {
+            fr.x = (float)__double2loint(fma(B.uz, k2.x, fma(B.uy, k1.x, fma(B.ux, k0.x, kFracMagic))));
+            fr.y = (float)__double2loint(fma(B.uz, k2.y, fma(B.uy, k1.y, fma(B.ux, k0.y, kFracMagic))));
+        } else {
+            const double ka = fma(B.uz, k2.x, fma(B.uy, k1.x, B.ux * k0.x));
+            const double kb = fma(B.uz, k2.y, fma(B.uy, k1.y, B.ux * k0.y));
+            fr.x = (float)((ka - ((ka + kMagic) - kMagic)) * 4294967296.0);
+            fr.y = (float)((kb - ((kb + kMagic) - kMagic)) * 4294967296.0);
+        }
     }
     const float2 one = bc2(1.0f);
     float2 eps0, eps1, eps2, pb;
     ld22(&P.eps[0], eps0, eps1);
     ld22(&P.eps[2], eps2, pb);
     const float2 al = fma2(B.fz, eps2, fma2(B.fy, eps1, mul2(B.fx, eps0)));  // u . eps
-    // with y = b - al^2: half phase hkRh y (1 + al) - rf, and
+    // with y = b - al^2: half phase hkRh y (1 + al) - pi 2^-32 fr, and
     // opa2 = 1 + al + 1.5 al^2 - 0.5 b = (1 + al) - 0.5 y + al^2
     const float2 opa = add2(one, al);
     const float2 y = fma2(neg2(al), al, pb);
-    const float2 ph = fma2(mul2(hkRh, y), opa, neg2(rf));
+    const float2 ph = fma2(fr, bc2((float)(-kPi / 4294967296.0)), mul2(mul2(hkRh, y), opa));
     const float2 opa2 = fma2(al, al, fma2(bc2(-0.5f), y, opa));
     // The unit direction from the facet centre in the lab frame, (a, b, c) = u opa2 -
     // eps opa, and k = R (a, b, c) in the aperture frame.  The normal of the
@@ -958,14 +973,14 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     const float2 a = fma2(B.fx, opa2, neg2(mul2(eps0, opa)));
     const float2 b = fma2(B.fy, opa2, neg2(mul2(eps1, opa)));
     const float2 c = fma2(B.fz, opa2, neg2(mul2(eps2, opa)));
-    float2 r3, r4, r5, kp, kx, ky, kz, u;
+    float2 r3, r4, r5, nKx, kx, ky, kz, u;
     {
         float2 r0, r1, r2, r6, r7, r8;
         ld22(&P.R[0], r0, r1);
         ld22(&P.R[2], r2, r3);
         ld22(&P.R[4], r4, r5);
         ld22(&P.R[6], r6, r7);
-        ld22(&P.R[8], r8, kp);
+        ld22(&P.R[8], r8, nKx);
         kx = fma2(r2, c, fma2(r1, b, mul2(r0, a)));
         u = fma2(r4, b, mul2(r3, a));
         ky = fma2(r5, c, u);
@@ -973,19 +988,17 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     }
     // the divided difference's phases, sort, sines and cosines: independent of
     // the polarisation block and its rare branch, so formed ahead of the branch
-    // (one basic block with the direction arithmetic for the scheduler).  The
-    // aperture wave vector's x part is halved with the phases; its y part is ky
-    // times the factor that vy carries.
+    // (one basic block with the direction arithmetic for the scheduler)
     TriF tf;
     {
-        const float2 kxx = fma2(nkh, kx, kp);
+        const float2 dx = add2(kx, nKx);
         float2 vx0, vx1, vx2, vy0, vy1, vy2;
         ld22(&P.vx[0], vx0, vx1);
         ld22(&P.vx[2], vx2, vy0);
         ld22(&P.vy[1], vy1, vy2);
-        const float2 t1 = fma2(ky, vy0, fma2(kxx, vx0, ph));
-        const float2 t2 = fma2(ky, vy1, fma2(kxx, vx1, ph));
-        const float2 t3 = fma2(ky, vy2, fma2(kxx, vx2, ph));
+        const float2 t1 = fma2(ky, vy0, fma2(dx, vx0, ph));
+        const float2 t2 = fma2(ky, vy1, fma2(dx, vx1, ph));
+        const float2 t3 = fma2(ky, vy2, fma2(dx, vx2, ph));
         tf = tri_front(t1, t2, t3);
     }
     // Polarisation matrix [[d, e], [-e, d]] (see k2_record for the forms) and
@@ -1053,7 +1066,7 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
             by = !(fabsf(dinc.y) < 0.999f);
             if (bx || by) {
                 // h from the direction (ba, bb, .) from the facet to the bodge's bin
-                const float2 ux = bc2(hb[0][B.hslot]), uy = bc2(hb[1][B.hslot]), uz = bc2(hb[2][B.hslot]);
+                const float2 ux = bc2(hb.x), uy = bc2(hb.y), uz = bc2(hb.z);
                 const float2 ah = fma2(uz, eps2, fma2(uy, eps1, mul2(ux, eps0)));
                 const float2 oh = add2(one, ah);
                 const float2 oh2 = fma2(ah, fma2(bc2(1.5f), ah, one), fma2(bc2(-0.5f), pb, one));
@@ -1156,7 +1169,7 @@ struct K2PkArgs {
     const K2Pair *pairs;
     const K2Fov *fovs;
     const int *perm;        // is_fast_diff: tile-major bin order (-1: padding)
-    const K2Cone *cones;    // is_fast_diff: cone of each tile
+    const K2Cone *cones;    // is_fast_diff: cone of each warp's 32 bins
     const int64_t *seg_rec;
     const int64_t *item_pre;
     int64_t nseg;
@@ -1165,8 +1178,8 @@ struct K2PkArgs {
     const double *xyz;
     int64_t nb, nphi;
     int64_t theta_i;
-    float k;
     float hkR;
+    float turns;  // k R / (2 pi): half turns of the far-field phase per unit of |com| / R
     const unsigned *epsmax;  // float bits of a bound of |com| / R over the records
     double *ws;         // [seg][8][nb]
     unsigned *tickets;  // [seg][tile], splits added so far
@@ -1174,59 +1187,107 @@ struct K2PkArgs {
     int *err;
 };
 
+// The record pairs go through K2_NST shared-memory stages.  `full` of a stage
+// completes when its bulk copy has landed, `empty` when all four warps are done with
+// it; thread 0 refills the stage of chunk c - 1 after its own chunk c, so a warp runs
+// up to a chunk ahead of or behind the others and no CTA barrier stands between the
+// chunks.
+// With the field-of-view test each warp culls the stage's records against the cone of
+// its own 4 x 8 bins (13.3 ms; 14.9 with one 8 x 16 cone for the CTA, on 16 lists of
+// 3,500 polygons x 64,979 bins).
 template <int BPT, bool FAST>
 __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kernel(K2PkArgs P) {
     constexpr int CH = FAST ? K2P_CH_FOV : K2P_CH_FULL;
+    constexpr int NW = K2_THREADS / 32;
     __shared__ __align__(128) K2Pair sbuf[K2_NST][CH];
-    __shared__ __align__(8) uint64_t bars[K2_NST];
-    __shared__ long long s_item;
-    __shared__ unsigned s_keep[2];  // is_fast_diff: records of the stage not culled for the tile
-    __shared__ float s_hb[3][K2P_HB];  // forward-bodge bin directions of this CTA's bins
+    __shared__ __align__(8) uint64_t full[K2_NST], empty[K2_NST];
+    __shared__ float4 s_hb[BPT][K2_THREADS];  // forward-bodge bin directions of this CTA's bins
+    // the item's FP64 sums, a column per thread: in registers (two bins a thread) they
+    // made the compiler spill inside the pair loop
+    constexpr bool ACCS = BPT == 1;
+    __shared__ double s_acc[ACCS ? 8 : 1][ACCS ? K2_THREADS : 1];
+    // the current item, decoded by thread 0: in shared memory, so that its state takes
+    // no registers across the pair loop
+    __shared__ struct {
+        int64_t seg, p0;          // segment; first record pair
+        int npair, nchunk, tile, split;
+        int edge;                 // bit 0 / 1: the first / last pair is half the item's
+        int st0, ph0, issued;     // first stage and its parity, chunks asked for
+    } I;
     __shared__ int s_ok;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0) {
-        for (int s = 0; s < K2_NST; s++) mbar_init(smem_u32(&bars[s]), 1);
+        for (int s = 0; s < K2_NST; s++) {
+            mbar_init(smem_u32(&full[s]), 1);
+            mbar_init(smem_u32(&empty[s]), NW);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    uint32_t parity = 0;  // bit s: phase of stage s
+    int st = 0;             // stage of the next chunk
+    uint32_t phase = 0;     // its parity: the number of rounds over the stages, modulo 2
     const int64_t total = P.item_pre[P.nseg];
     constexpr int64_t TILE = (int64_t)K2_THREADS * BPT;
-    // half phases: -k/2 and k R / 4
-    const float2 nkh = bc2(-0.5f * P.k), hkRh = bc2(0.5f * P.hkR);
+    // half phases: k R / 4
+    const float2 hkRh = bc2(0.5f * P.hkR);
     // bins with |uz| below pole_cos are out of reach of the forward bodge for every
     // record: |inc . k - (-uz)| <= 2 |com| / R for the direction k from a facet centre
     const float pole_cos = 0.999f - 2.0f * __uint_as_float(*P.epsmax) - 1e-5f;
+    const bool wide = !(P.turns * __uint_as_float(*P.epsmax) < 262144.0f);  // see k2_pair
     for (;;) {
-        if (tid == 0) s_item = (long long)atomicAdd(P.counter, 1ull);
-        __syncthreads();
-        const int64_t item = s_item;
-        if (item >= total) break;
-        int64_t lo = 0, hi = P.nseg;
-        while (hi - lo > 1) {
-            const int64_t m = (lo + hi) >> 1;
-            if (P.item_pre[m] <= item)
-                lo = m;
-            else
-                hi = m;
+        auto after = [](int s, int n) { return s + n >= K2_NST ? s + n - K2_NST : s + n; };
+        // chunk c of the item into its stage (s its index); thread 0 only
+        auto load = [&](int c, int s) {
+            const int n = min(CH, I.npair - c * CH);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            bulk_load(smem_u32(&sbuf[s][0]), P.pairs + I.p0 + c * CH, (uint32_t)(n * sizeof(K2Pair)),
+                      smem_u32(&full[s]));
+        };
+        if (tid == 0) {
+            const int64_t item = (int64_t)atomicAdd(P.counter, 1ull);
+            I.seg = -1;
+            if (item < total) {
+                int64_t lo = 0, hi = P.nseg;
+                while (hi - lo > 1) {
+                    const int64_t m = (lo + hi) >> 1;
+                    if (P.item_pre[m] <= item)
+                        lo = m;
+                    else
+                        hi = m;
+                }
+                const int64_t local = item - P.item_pre[lo];
+                const int64_t split = local / P.ntiles;
+                const int64_t rbeg = P.seg_rec[lo] + split * P.rpi;
+                const int64_t rend = min(rbeg + P.rpi, P.seg_rec[lo + 1]);
+                // record pairs [p0, p0 + npair) cover records [rbeg, rend)
+                I.seg = lo;
+                I.p0 = rbeg >> 1;
+                I.npair = (int)(((rend + 1) >> 1) - (rbeg >> 1));
+                I.nchunk = (I.npair + CH - 1) / CH;
+                I.tile = (int)(local - split * P.ntiles);
+                I.split = (int)split;
+                I.edge = (int)(rbeg & 1) | (int)(rend & 1) << 1;
+                I.st0 = st;
+                I.ph0 = (int)phase;
+                I.issued = min(I.nchunk, K2_NST);
+                // every stage is free: the previous item's chunks were consumed by all warps
+                for (int c = 0; c < I.issued; c++) load(c, after(st, c));
+            }
         }
-        const int64_t seg = lo;
-        const int64_t local = item - P.item_pre[seg];
-        const int64_t split = local / P.ntiles, tile = local % P.ntiles;
-        const int64_t rbeg = P.seg_rec[seg] + split * P.rpi;
-        const int64_t rend = min(rbeg + P.rpi, P.seg_rec[seg + 1]);
+        __syncthreads();
+        if (I.seg < 0) break;
+        // the bin of this thread's slot q in the item's tile, -1: none
+        auto bin_of = [&](int q) {
+            const int64_t li = I.tile * TILE + q * K2_THREADS + tid;
+            return FAST ? P.perm[li] : li < P.nb ? (int)li : -1;
+        };
         BinPk bd[BPT];
-        bool valid[BPT];
-        int64_t bin[BPT];
 #pragma unroll
         for (int q = 0; q < BPT; q++) {
-            const int64_t li = tile * TILE + q * K2_THREADS + tid;
-            bin[q] = FAST ? (int64_t)P.perm[li] : li;
-            valid[q] = FAST ? bin[q] >= 0 : bin[q] < P.nb;
-            const int64_t o = valid[q] ? bin[q] : 0;
+            bd[q].bin = bin_of(q);
+            const int64_t o = bd[q].bin >= 0 ? bd[q].bin : 0;
             const double X = P.xyz[o], Y = P.xyz[P.nb + o], Zc = P.xyz[2 * P.nb + o];
             const double ir = 1.0 / sqrt(X * X + Y * Y + Zc * Zc);
-            bd[q].bin = o;
             bd[q].ux = X * ir;
             bd[q].uy = Y * ir;
             bd[q].uz = Zc * ir;
@@ -1237,107 +1298,79 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             const int64_t oh = (o % P.nphi) + P.nphi * P.theta_i;
             const double Xh = P.xyz[oh], Yh = P.xyz[P.nb + oh], Zh = P.xyz[2 * P.nb + oh];
             const double irh = 1.0 / sqrt(Xh * Xh + Yh * Yh + Zh * Zh);
-            bd[q].hslot = q * K2_THREADS + tid;
-            s_hb[0][bd[q].hslot] = (float)(Xh * irh);
-            s_hb[1][bd[q].hslot] = (float)(Yh * irh);
-            s_hb[2][bd[q].hslot] = (float)(Zh * irh);
+            s_hb[q][tid] = make_float4((float)(Xh * irh), (float)(Yh * irh), (float)(Zh * irh), 0.0f);
         }
         double acc64[BPT][8];
+        auto sum = [&](int q, int c) -> double & {
+            if constexpr (ACCS)
+                return s_acc[c][tid];
+            else
+                return acc64[q][c];
+        };
 #pragma unroll
         for (int q = 0; q < BPT; q++)
 #pragma unroll
-            for (int c = 0; c < 8; c++) acc64[q][c] = 0.0;
-        K2Cone cone;
-        if (FAST) cone = P.cones[tile];
-        // record pairs [p0, p1) cover records [rbeg, rend)
-        const int64_t p0 = rbeg >> 1, p1 = (rend + 1) >> 1;
-        const int64_t npair = p1 - p0;
-        const int64_t nchunk = (npair + CH - 1) / CH;
-        if (tid == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            for (int64_t c = 0; c < nchunk && c < K2_NST; c++) {
-                const int64_t n = min((int64_t)CH, npair - c * CH);
-                bulk_load(smem_u32(&sbuf[c][0]), P.pairs + p0 + c * CH,
-                          (uint32_t)(n * sizeof(K2Pair)), smem_u32(&bars[c]));
+            for (int c = 0; c < 8; c++) sum(q, c) = 0.0;
+        bool failed = false;
+        for (int c = 0; c < I.nchunk; c++) {
+            if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&full[st]), phase))) {
+                failed = true;
+                break;
             }
-        }
-        bool timed_out = false;
-        int64_t c_out = 0;
-        for (int64_t c = 0; c < nchunk; c++) {
-            const int st = (int)(c % K2_NST);
-            const bool ok = mbar_wait(smem_u32(&bars[st]), (parity >> st) & 1u);
-            parity ^= 1u << st;
-            const int n = (int)min((int64_t)CH, npair - c * CH);
-            if (!FAST && ok && tid < 33) {
+            const int n = min(CH, I.npair - c * CH);
+            if (!FAST) {
                 // The item's first pair (odd rbeg) and last pair (odd rend) hold a
                 // record of another item or the array's padding: that half takes a
                 // copy of the pair's other record with zero amplitude, so the pair
-                // loop needs no per-pair range test.  Threads 0-2 copy the FP64
-                // phase, threads 3-32 the 30 float2 fields from eps on (the last 8
-                // are the amplitudes); the barrier below publishes the copy.
+                // loop needs no per-pair range test.  Every warp writes the same
+                // values for itself: 3 FP64 phases, then the 30 float2 fields from
+                // eps on (the last 8 are the amplitudes).
                 auto patch = [&](int j, int src, int dst) {
                     K2Pair &Q = sbuf[st][j];
-                    if (tid < 3) {
-                        Q.kc[tid][dst] = Q.kc[tid][src];
-                    } else {
-                        float2 *f = &Q.eps[0];
-                        const int i = tid - 3;
-                        const float v = i >= 22 ? 0.0f : (src ? f[i].y : f[i].x);
-                        if (dst)
-                            f[i].y = v;
-                        else
-                            f[i].x = v;
+                    for (int t = lane; t < 33; t += 32) {
+                        if (t < 3) {
+                            Q.kc[t][dst] = Q.kc[t][src];
+                        } else {
+                            float2 *f = &Q.eps[0];
+                            const int i = t - 3;
+                            const float v = i >= 22 ? 0.0f : (src ? f[i].y : f[i].x);
+                            if (dst)
+                                f[i].y = v;
+                            else
+                                f[i].x = v;
+                        }
                     }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
                 };
-                if (c == 0 && (rbeg & 1)) patch(0, 1, 0);
-                if (c == nchunk - 1 && (rend & 1)) patch(n - 1, 0, 1);
-            }
-            if (__syncthreads_or(!ok)) {
-                timed_out = true;
-                c_out = c;
-                break;
+                if (c == 0 && (I.edge & 1)) patch(0, 1, 0);
+                if (c == I.nchunk - 1 && (I.edge & 2)) patch(n - 1, 0, 1);
             }
             float2 acc[BPT][8];
 #pragma unroll
             for (int q = 0; q < BPT; q++)
 #pragma unroll
                 for (int cc = 0; cc < 8; cc++) acc[q][cc] = bc2(0.0f);
-            // only the item's first pair (odd rbeg) and last pair (odd rend) are partial
-            const int j_lo = (c == 0 && (rbeg & 1)) ? 0 : -1;
-            const int j_hi = (c == nchunk - 1 && (rend & 1)) ? n - 1 : -1;
             if (FAST) {
-                // the tile cull of the stage's 2n records, one per thread of
-                // warps 0 and 1: a record whose field of view misses the whole
-                // tile adds nothing
-                if (tid < 64) {
-                    const bool keep =
-                        tid < 2 * n && !cone_culled(P.fovs[2 * (p0 + c * CH) + tid], cone);
-                    const unsigned m = __ballot_sync(0xffffffffu, keep);
-                    if ((tid & 31) == 0) s_keep[tid >> 5] = m;
-                }
-                __syncthreads();
-            }
-            auto pair_step = [&](int j) {
-                bool lo_ok = j != j_lo, hi_ok = j != j_hi;
-                const K2Fov *fv = FAST ? P.fovs + 2 * (p0 + c * CH + j) : nullptr;
-                if (FAST) {
-                    const unsigned m = s_keep[j >> 4] >> (2 * (j & 15));
-                    lo_ok = lo_ok && (m & 1u);
-                    hi_ok = hi_ok && (m & 2u);
-                    if (!lo_ok && !hi_ok) return;  // uniform over the CTA
-                }
-                // without the field-of-view test every lane adds (the edge pairs are
-                // patched above; a bin beyond nb is never written out)
+                // the tile cull of the stage's 2n records, two per lane: a record
+                // whose field of view misses the warp's bins adds nothing
+                unsigned keep[2];
 #pragma unroll
-                for (int q = 0; q < BPT; q++)
-                    k2_pair<FAST>(sbuf[st][j], fv, bd[q], acc[q], nkh, hkRh, s_hb,
-                                  FAST ? (lo_ok && valid[q]) : true,
-                                  FAST ? (hi_ok && valid[q]) : true, P.xyz, P.nb,
-                                  P.rlo + (p0 + c * CH + j) * 3);
-            };
-            if (FAST) {
-                // visit only the pairs with a record the tile cull kept: bit j of pm
-                // is set when record 2j or 2j+1 is (the two ballot words compacted)
+                for (int h = 0; h < 2; h++) {
+                    const int r = h * 32 + lane;
+                    bool k = false;
+                    if (r < 2 * n) {
+                        const K2Fov &f = P.fovs[2 * (I.p0 + c * CH) + r];
+#pragma unroll
+                        for (int q = 0; q < BPT; q++)
+                            k = k || !cone_culled(f, P.cones[((int64_t)I.tile * BPT + q) * NW + (tid >> 5)]);
+                    }
+                    keep[h] = __ballot_sync(0xffffffffu, k);
+                }
+                if (c == 0 && (I.edge & 1)) keep[0] &= ~1u;
+                if (c == I.nchunk - 1 && (I.edge & 2)) keep[(2 * n - 1) >> 5] &= ~(1u << ((2 * n - 1) & 31));
+                // visit only the pairs with a record the cull kept: bit j of pm is
+                // set when record 2j or 2j+1 is (the two ballot words compacted)
                 auto pairs_of = [](unsigned x) {
                     x = (x | (x >> 1)) & 0x55555555u;
                     x = (x | (x >> 1)) & 0x33333333u;
@@ -1346,40 +1379,72 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     x = (x | (x >> 8)) & 0x0000FFFFu;
                     return x;
                 };
-                unsigned pm = pairs_of(s_keep[0]) | (pairs_of(s_keep[1]) << 16);
-                while (pm) {
-                    const int j = __ffs(pm) - 1;
-                    pm &= pm - 1u;
-                    pair_step(j);
-                }
+                const unsigned pm0 = pairs_of(keep[0]) | (pairs_of(keep[1]) << 16);
+                auto pairs = [&](auto w) {
+                    for (unsigned pm = pm0; pm; pm &= pm - 1u) {
+                        const int j = __ffs(pm) - 1;
+                        const unsigned m = (j & 16 ? keep[1] : keep[0]) >> (2 * (j & 15));
+                        const K2Fov *fv = P.fovs + 2 * (I.p0 + c * CH + j);
+#pragma unroll
+                        for (int q = 0; q < BPT; q++)
+                            k2_pair<true, decltype(w)::value>(
+                                sbuf[st][j], fv, bd[q], acc[q], hkRh, s_hb[q][tid],
+                                (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0, P.xyz, P.nb,
+                                P.rlo + (I.p0 + c * CH + j) * 3);
+                    }
+                };
+                if (wide)
+                    pairs(std::true_type());
+                else
+                    pairs(std::false_type());
             } else {
-                for (int j = 0; j < n; j++) pair_step(j);
+                // without the field-of-view test every lane adds (the edge pairs are
+                // patched above; a bin beyond nb is never written out)
+                auto pairs = [&](auto w) {
+                    for (int j = 0; j < n; j++)
+#pragma unroll
+                        for (int q = 0; q < BPT; q++)
+                            k2_pair<false, decltype(w)::value>(
+                                sbuf[st][j], nullptr, bd[q], acc[q], hkRh, s_hb[q][tid], true, true,
+                                P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
+                };
+                if (wide)
+                    pairs(std::true_type());
+                else
+                    pairs(std::false_type());
             }
 #pragma unroll
             for (int q = 0; q < BPT; q++)
 #pragma unroll
                 for (int cc = 0; cc < 8; cc++)
-                    acc64[q][cc] += (double)acc[q][cc].x + (double)acc[q][cc].y;
-            __syncthreads();
-            if (tid == 0 && c + K2_NST < nchunk) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                const int64_t c2 = c + K2_NST;
-                const int64_t n2 = min((int64_t)CH, npair - c2 * CH);
-                bulk_load(smem_u32(&sbuf[st][0]), P.pairs + p0 + c2 * CH,
-                          (uint32_t)(n2 * sizeof(K2Pair)), smem_u32(&bars[st]));
+                    sum(q, cc) += (double)acc[q][cc].x + (double)acc[q][cc].y;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&empty[st]));
+            // the stage before this one (chunk c - 1) takes chunk c - 1 + K2_NST once
+            // every warp has left it; its parity is this stage's, or the round before
+            if (tid == 0 && c > 0 && c - 1 + K2_NST < I.nchunk) {
+                const int sp = st == 0 ? K2_NST - 1 : st - 1;
+                if (mbar_wait(smem_u32(&empty[sp]), st == 0 ? phase ^ 1u : phase)) {
+                    load(c - 1 + K2_NST, sp);
+                    I.issued = c + K2_NST;
+                } else {
+                    failed = true;  // the other warps' waits for its chunk run out too
+                }
             }
+            st = after(st, 1);
+            if (st == 0) phase ^= 1u;
+            if (__any_sync(0xffffffffu, failed)) break;
         }
-        unsigned *tk = P.tickets + seg * P.ntiles + tile;
-        if (timed_out) {
+        unsigned *tk = P.tickets + I.seg * P.ntiles + I.tile;
+        if (__syncthreads_or(failed)) {
             if (tid == 0) {
                 atomicOr(P.err, 4);
                 atomicMax(tk, kTicketPoison);
-                // bounded wait for this CTA's bulk copies still in flight
-                for (int64_t c2 = c_out; c2 < min(nchunk, c_out + K2_NST); c2++) {
-                    const int s2 = (int)(c2 % K2_NST);
-                    const uint32_t ph = (parity >> s2) & 1u;
-                    mbar_wait(smem_u32(&bars[s2]), c2 == c_out ? ph ^ 1u : ph);
-                }
+                // bounded wait for this CTA's bulk copies still in flight: the latest
+                // copy of every stage
+                for (int c = max(0, I.issued - K2_NST); c < I.issued; c++)
+                    mbar_wait(smem_u32(&full[(I.st0 + c) % K2_NST]),
+                              (uint32_t)(I.ph0 ^ (((I.st0 + c) / K2_NST) & 1)));
             }
             return;
         }
@@ -1387,7 +1452,9 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
         double lin[BPT][8];
 #pragma unroll
         for (int q = 0; q < BPT; q++) {
-            const double *u = acc64[q];
+            double u[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) u[c] = sum(q, c);
             lin[q][0] = 0.5 * (u[0] + u[2]);
             lin[q][1] = 0.5 * (u[1] + u[3]);
             lin[q][2] = 0.5 * (u[1] - u[3]);
@@ -1397,7 +1464,14 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             lin[q][6] = 0.5 * (u[5] - u[7]);
             lin[q][7] = 0.5 * (u[6] - u[4]);
         }
-        ordered_add<BPT>(P.ws + seg * 8 * P.nb, P.nb, tk, (unsigned)split, valid, bin, lin, &s_ok,
+        bool valid[BPT];
+        int64_t bin[BPT];
+#pragma unroll
+        for (int q = 0; q < BPT; q++) {
+            bin[q] = bin_of(q);
+            valid[q] = bin[q] >= 0;
+        }
+        ordered_add<BPT>(P.ws + I.seg * 8 * P.nb, P.nb, tk, (unsigned)I.split, valid, bin, lin, &s_ok,
                          P.err);
     }
 }
@@ -1808,7 +1882,7 @@ int k2_launch_pk(pbt_ctx *ctx, cudaStream_t st, const K2PkArgs &A) {
     return PBT_OK;
 }
 
-// One warp per tile: unit centre of the tile's bin directions and the
+// One warp per group of `tile` bins: unit centre of their directions and the
 // largest angle of a bin from it (FP64).
 __global__ void k2_cone_kernel(const int *__restrict__ perm, int64_t ntiles, int64_t tile,
                                const double *__restrict__ xyz, int64_t nb, K2Cone *__restrict__ cones) {
@@ -1816,9 +1890,11 @@ __global__ void k2_cone_kernel(const int *__restrict__ perm, int64_t ntiles, int
     const int lane = threadIdx.x & 31;
     if (t >= ntiles) return;
     double sx = 0.0, sy = 0.0, sz = 0.0;
+    int n = 0;
     for (int64_t i = lane; i < tile; i += 32) {
         const int o = perm[t * tile + i];
         if (o < 0) continue;
+        n++;
         const double X = xyz[o], Y = xyz[nb + o], Z = xyz[2 * nb + o];
         const double ir = 1.0 / sqrt(X * X + Y * Y + Z * Z);
         sx += X * ir;
@@ -1843,22 +1919,25 @@ __global__ void k2_cone_kernel(const int *__restrict__ perm, int64_t ntiles, int
         dmin = fmin(dmin, (X * cx + Y * cy + Z * cz) * ir);
     }
     for (int off = 16; off > 0; off >>= 1) dmin = fmin(dmin, __shfl_xor_sync(0xffffffffu, dmin, off));
+    const bool some = __any_sync(0xffffffffu, n > 0);
     if (lane == 0) {
         const double psi = ok ? acos(fmax(-1.0, fmin(1.0, dmin))) + 1e-6 : 4.0;
         K2Cone c;
         c.c[0] = (float)cx;
         c.c[1] = (float)cy;
         c.c[2] = (float)cz;
-        c.psi = (float)psi;
-        c.cos_psi = (float)cos(psi);
-        c.sin_psi = (float)sin(psi);
+        // a group of padding only: culled for every record (cone_culled's bound is +inf)
+        c.psi = some ? (float)psi : 0.0f;
+        c.cos_psi = some ? (float)cos(psi) : 0.0f;
+        c.sin_psi = some ? (float)sin(psi) : -INFINITY;
         c.pad[0] = c.pad[1] = 0.0f;
         cones[t] = c;
     }
 }
 
-// is_fast_diff tiles of `tile` bins: blocks of (tile/16) theta x 16 phi bins,
-// so that a tile spans a small solid angle; cached with the bin grid.
+// is_fast_diff tiles of `tile` bins: blocks of (tile/16) theta x 16 phi bins, each
+// warp's 32 bins a block of 4 theta x 8 phi within it, so that a warp spans a small
+// solid angle; cached with the bin grid, a cone per warp.
 int k2_fast_tiles(pbt_ctx *ctx, cudaStream_t st, int64_t tile) {
     GridCache &g = ctx->grid;
     if (g.fast_tile == tile) return PBT_OK;
@@ -1868,19 +1947,20 @@ int k2_fast_tiles(pbt_ctx *ctx, cudaStream_t st, int64_t tile) {
     const int64_t ntiles = ntb * npb;
     std::vector<int> perm((size_t)(ntiles * tile), -1);
     for (int64_t a = 0; a < ntb; a++)
-        for (int64_t b = 0; b < npb; b++) {
-            const int64_t t = a * npb + b;
-            int64_t i = 0;
-            for (int64_t j = a * bt; j < std::min(ntheta, (a + 1) * bt); j++)
-                for (int64_t q = b * bp; q < std::min(nphi, (b + 1) * bp); q++)
-                    perm[(size_t)(t * tile + i++)] = (int)(q + nphi * j);
-        }
+        for (int64_t b = 0; b < npb; b++)
+            for (int64_t i = 0; i < tile; i++) {
+                const int64_t w = (i % 128) / 32, l = i % 32;
+                const int64_t j = a * bt + (i / 128) * 8 + (w >> 1) * 4 + (l >> 3);
+                const int64_t q = b * bp + (w & 1) * 8 + (l & 7);
+                if (j < ntheta && q < nphi) perm[(size_t)((a * npb + b) * tile + i)] = (int)(q + nphi * j);
+            }
+    const int64_t ncones = ntiles * tile / 32;
     PBT_TRY(g.fast_perm.ensure(perm.size() * sizeof(int)));
-    PBT_TRY(g.fast_cone.ensure((size_t)ntiles * sizeof(K2Cone)));
+    PBT_TRY(g.fast_cone.ensure((size_t)ncones * sizeof(K2Cone)));
     PBT_CUDA_TRY(cudaMemcpyAsync(g.fast_perm.p, perm.data(), perm.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, st));
-    k2_cone_kernel<<<(unsigned)((ntiles + 3) / 4), 128, 0, st>>>(
-        g.fast_perm.as<int>(), ntiles, tile, g.xyz.as<double>(), g.nb, g.fast_cone.as<K2Cone>());
+    k2_cone_kernel<<<(unsigned)((ncones + 3) / 4), 128, 0, st>>>(
+        g.fast_perm.as<int>(), ncones, 32, g.xyz.as<double>(), g.nb, g.fast_cone.as<K2Cone>());
     ctx->launches++;
     PBT_CUDA_TRY(cudaGetLastError());
     PBT_CUDA_TRY(cudaStreamSynchronize(st));  // perm (pageable) and cones ready before caching
@@ -1960,8 +2040,8 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
         B.nb = A.nb;
         B.nphi = A.nphi;
         B.theta_i = A.theta_i;
-        B.k = A.k;
         B.hkR = A.hkR;
+        B.turns = (float)(0.5 * waveno * kFarR * kInvPi);
         B.epsmax = S.epsmax;
         B.ws = ws;
         B.tickets = A.tickets;
