@@ -35,6 +35,7 @@
 #include <stdlib.h>
 
 #include <cub/device/device_scan.cuh>
+#include <algorithm>
 #include <type_traits>
 
 #include "frame.h"
@@ -89,6 +90,11 @@ struct RefSrc {
     const int64_t *ext_off;
     const int64_t *refbase;   // beam_off[o] + ext_off[o]
     int64_t norient;
+    // records before outbeam g: start[g] (k2_count and its scan), or g * per where every
+    // face has per + 2 vertices (start NULL): nothing to count then
+    const int64_t *start;
+    int64_t per;
+    __device__ __forceinline__ int64_t first(int64_t g) const { return start ? start[g] : g * per; }
 };
 
 __device__ __forceinline__ int64_t find_orient(const int64_t *base, int64_t n, int64_t g) {
@@ -167,8 +173,7 @@ __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const 
 
 __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restrict__ verts,
                                 int64_t nverts, const int64_t *__restrict__ face_off,
-                                const int64_t *__restrict__ face_vi, const int64_t *__restrict__ start,
-                                double waveno, double lambda, int fast_diff,
+                                int64_t nfaces, const int64_t *__restrict__ face_vi, double waveno, double lambda, int fast_diff,
                                 K2Rec *__restrict__ recs, K2Pair *__restrict__ pairs,
                                 K2Fov *__restrict__ fovs, float2 *__restrict__ rlo,
                                 int *__restrict__ err, unsigned *__restrict__ epsmax) {
@@ -178,7 +183,27 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
     int kind;
     const pbt_outbeam *ob = ref_lookup(S, g, o, kind);
     const int64_t fi = ob->fi;
-    if (fi < 1) return;  // reported by the count kernel
+    if (fi < 1 || fi > nfaces) {
+        atomicOr(err, 1);
+        if (!S.start) {
+            // the outbeam's records exist all the same: empty ones
+            K2Rec rec{};
+            rec.R[0] = rec.R[4] = rec.R[8] = 1.0f;
+            const double uc[8] = {}, z[3] = {};
+            for (int64_t r = g * S.per; r < (g + 1) * S.per; r++) {
+                if (pairs)
+                    store_pair_half(pairs, r, rec, 0.0, uc, 0.0, z, z, 0.0);
+                else
+                    recs[r] = rec;
+                for (int i = 0; i < 3; i++) {
+                    float2 &l = rlo[(r >> 1) * 3 + i];
+                    (r & 1 ? l.y : l.x) = 0.0f;
+                }
+                if (fast_diff) fovs[r] = K2Fov{};
+            }
+        }
+        return;
+    }
     const int64_t fb = face_off[fi - 1];
     const int nv = (int)(face_off[fi] - fb);
     const double *V = verts + o * 3 * nverts;
@@ -211,7 +236,10 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
     const double cf = 1.0 / sqrt(1.0 - Ky * Ky);
     double ea[3];
     mv33(fr.R, com, ea);
-    const int64_t r0 = start[g];
+    const int64_t r0 = S.first(g);
+    // an odd record count: the low parts of the last pair's unused half
+    if (g == nrefs - 1 && ((r0 + nv - 2) & 1))
+        for (int i = 0; i < 3; i++) rlo[((r0 + nv - 2) >> 1) * 3 + i].y = 0.0f;
     for (int t = 0; t < nv - 2; t++) {
         const int iv[3] = {0, t + 1, t + 2};
         double xa[3], ya[3];
@@ -299,27 +327,49 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
     }
 }
 
-// Per orientation chunk [o0, o0+no): segment records and work-item prefix.
-__global__ void k2_plan_kernel(const int64_t *__restrict__ start, const int64_t *__restrict__ refbase,
-                               const int64_t *__restrict__ beam_off, int64_t o0, int64_t no,
-                               int64_t rpi, int64_t ntiles, int64_t *__restrict__ seg_rec,
-                               int64_t *__restrict__ item_pre, unsigned long long *__restrict__ counter) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int64_t q = 0; q < no; q++) {
-        const int64_t o = o0 + q;
-        const int64_t nbo = beam_off[o + 1] - beam_off[o];
-        seg_rec[2 * q] = start[refbase[o]];
-        seg_rec[2 * q + 1] = start[refbase[o] + nbo];
+// Per orientation chunk [o0, o0+no): segment records and work-item prefix (block 0, a
+// scan over the segments), and the split tickets set to zero (the other blocks).
+constexpr int K2_PLAN_THREADS = 256;
+__global__ void k2_plan_kernel(RefSrc S, int64_t o0, int64_t no, int64_t rpi, int64_t ntiles,
+                               int64_t *__restrict__ seg_rec, int64_t *__restrict__ item_pre,
+                               unsigned long long *__restrict__ counter, unsigned *__restrict__ tickets) {
+    const int t = threadIdx.x;
+    if (blockIdx.x > 0) {
+        const int64_t n = 2 * no * ntiles, step = (int64_t)(gridDim.x - 1) * K2_PLAN_THREADS;
+        for (int64_t i = (int64_t)(blockIdx.x - 1) * K2_PLAN_THREADS + t; i < n; i += step) tickets[i] = 0u;
+        return;
     }
-    seg_rec[2 * no] = start[refbase[o0 + no]];
-    int64_t p = 0;
-    for (int64_t s = 0; s < 2 * no; s++) {
-        item_pre[s] = p;
-        const int64_t n = seg_rec[s + 1] - seg_rec[s];
-        p += ((n + rpi - 1) / rpi) * ntiles;
+    __shared__ int64_t sum[K2_PLAN_THREADS];
+    // thread t takes segments [s0, s1)
+    const int64_t nseg = 2 * no, each = (nseg + K2_PLAN_THREADS - 1) / K2_PLAN_THREADS;
+    const int64_t s0 = min(t * each, nseg), s1 = min(s0 + each, nseg);
+    auto rec_of = [&](int64_t s) {
+        const int64_t o = o0 + (s >> 1);
+        return S.first(S.refbase[o] + (s & 1 ? S.beam_off[o + 1] - S.beam_off[o] : 0));
+    };
+    int64_t items = 0, r = s0 < s1 ? rec_of(s0) : 0;
+    for (int64_t s = s0; s < s1; s++) {
+        const int64_t r1 = rec_of(s + 1);
+        seg_rec[s] = r;
+        if (s + 1 == nseg) seg_rec[nseg] = r1;
+        item_pre[s] = items;  // from the thread's first segment; its base is added below
+        items += ((r1 - r + rpi - 1) / rpi) * ntiles;
+        r = r1;
     }
-    item_pre[2 * no] = p;
-    *counter = 0ull;
+    sum[t] = items;
+    __syncthreads();
+    for (int d = 1; d < K2_PLAN_THREADS; d <<= 1) {
+        const int64_t v = t >= d ? sum[t - d] : 0;
+        __syncthreads();
+        sum[t] += v;
+        __syncthreads();
+    }
+    const int64_t base = sum[t] - items;
+    for (int64_t s = s0; s < s1; s++) item_pre[s] += base;
+    if (t == K2_PLAN_THREADS - 1) {
+        item_pre[nseg] = sum[t];
+        *counter = 0ull;
+    }
 }
 
 // ------------------------------------------------------------ main kernel
@@ -460,8 +510,9 @@ __device__ __forceinline__ void ordered_add(double *__restrict__ out, int64_t nb
             if (valid[q])
 #pragma unroll
                 for (int cc = 0; cc < 8; cc++) {
+                    // the first split of a tile stores: the workspace needs no clearing
                     double *o = out + cc * nb + bin[q];
-                    *o = __ldcg(o) + lin[q][cc];
+                    *o = split ? __ldcg(o) + lin[q][cc] : lin[q][cc];
                 }
         __threadfence();
     }
@@ -1507,15 +1558,17 @@ __device__ __forceinline__ void mueller16d(const Zd *S, double mu[16]) {
 }
 
 // Amplitude of segment seg at bin o as reference-layout complex 2x2 (with
-// T(phi) applied and scaled by sc), common phase e^{ik|X|} omitted.
-__device__ __forceinline__ void ws_ampl(const double *ws, int64_t seg, int64_t nb, int64_t o, double cp,
-                                        double sp, double sc, Zd S[4]) {
+// T(phi) applied and scaled by sc), common phase e^{ik|X|} omitted.  A segment
+// without records has no work items and nothing in the workspace: zero.
+__device__ __forceinline__ void ws_ampl(const double *ws, const int64_t *seg_rec, int64_t seg, int64_t nb,
+                                        int64_t o, double cp, double sp, double sc, Zd S[4]) {
     const double *w = ws + seg * 8 * nb + o;
     Zd a[4];
+    const bool some = seg_rec[seg + 1] > seg_rec[seg];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        a[c].re = w[(2 * c) * nb];
-        a[c].im = w[(2 * c + 1) * nb];
+        a[c].re = some ? w[(2 * c) * nb] : 0.0;
+        a[c].im = some ? w[(2 * c + 1) * nb] : 0.0;
     }
     // (S T)(a,b) = S(a,1) T(1,b) + S(a,2) T(2,b); T = [[-s, -c], [c, -s]]
     // order (1,1),(2,1),(1,2),(2,2): a[0]=S11 a[1]=S21 a[2]=S12 a[3]=S22
@@ -1526,60 +1579,56 @@ __device__ __forceinline__ void ws_ampl(const double *ws, int64_t seg, int64_t n
     S[3] = {(a[1].re * T12 + a[3].re * T22) * sc, (a[1].im * T12 + a[3].im * T22) * sc};
 }
 
-__device__ __forceinline__ double block_sum(double v, double *red) {
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) s += red[i];
-    __syncthreads();
-    return s;
+    return v;
 }
 
-// Pre-pass of -scaling: per-orientation scatt_beam / scatt_ext sums.
-// Per-orientation sums over the bins are reduced in two fixed-order steps (a
-// block sum into part[(q K + k) nblk + block], then k2_part_sum_kernel over the
-// blocks in order), so they are the same from run to run.
-__global__ void k2_scatt_be_kernel(const double *__restrict__ ws, int64_t no, int64_t o0, int64_t nb,
-                                   int64_t nphi, const double *__restrict__ phitab, double waveno,
+constexpr int K2_EPI_THREADS = 256;
+
+// Per-orientation sums over the bins are reduced in two fixed-order steps (a warp's
+// sum into part[(q K + k) nwarp + warp], then k2_part_sum_kernel over the warps in
+// order), so they are the same from run to run and no block waits for its warps.
+// Pre-pass of -scaling: per-orientation scatt_beam / scatt_ext sums; blockIdx.y takes
+// every gridDim.y-th orientation.
+__global__ void k2_scatt_be_kernel(const double *__restrict__ ws, const int64_t *__restrict__ seg_rec,
+                                   int64_t no, int64_t nb, int64_t nphi,
+                                   const double *__restrict__ phitab, double waveno,
                                    const double *__restrict__ wbin, double *__restrict__ part) {
-    __shared__ double red[32];
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = o < nb;
     const int64_t oo = in ? o : 0;
     const double cp = phitab[oo % nphi], sp = phitab[nphi + oo % nphi];
     const double W = in ? wbin[oo] / (waveno * waveno) : 0.0;
-    for (int64_t q = 0; q < no; q++) {
-        Zd Sb[4], Se[4];
-        ws_ampl(ws, 2 * q, nb, oo, cp, sp, waveno, Sb);
-        ws_ampl(ws, 2 * q + 1, nb, oo, cp, sp, waveno, Se);
-        double mb[16], me[16];
-        mueller16d(Sb, mb);
-        mueller16d(Se, me);
-        const double vb = block_sum(W * mb[0], red);
-        const double ve = block_sum(W * me[0], red);
-        if (threadIdx.x == 0) {
-            part[(2 * q) * gridDim.x + blockIdx.x] = vb;
-            part[(2 * q + 1) * gridDim.x + blockIdx.x] = ve;
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5), w = o >> 5;
+    for (int64_t q = blockIdx.y; q < no; q += gridDim.y) {
+        Zd S[4];
+        double m[16];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            ws_ampl(ws, seg_rec, 2 * q + k, nb, oo, cp, sp, waveno, S);
+            mueller16d(S, m);
+            const double v = warp_sum(W * m[0]);
+            if ((threadIdx.x & 31) == 0) part[(2 * q + k) * nw + w] = v;
         }
     }
-    (void)o0;
 }
-// out[k0 + r] = sum over b of part[r nblk + b] in block order, r < nrow (one warp
-// per row: lanes take blocks b = lane + 32 i in order, then a fixed shuffle tree).
-__global__ void k2_part_sum_kernel(const double *__restrict__ part, int64_t nrow, int64_t nblk,
-                                   double *__restrict__ out) {
-    const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (r >= nrow) return;
+// out[r] = sum over b of part[r n + b] (a block per row: each thread its stride in
+// order, then a fixed tree).
+__global__ void k2_part_sum_kernel(const double *__restrict__ part, int64_t n, double *__restrict__ out) {
+    __shared__ double red[8];
+    const double *p = part + blockIdx.x * n;
     double v = 0.0;
-    for (int64_t b = lane; b < nblk; b += 32) v += part[r * nblk + b];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == 0) out[r] = v;
+    for (int64_t b = threadIdx.x; b < n; b += blockDim.x) v += p[b];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = red[0];
+        for (int i = 1; i < (int)(blockDim.x >> 5); i++) t += red[i];
+        out[blockIdx.x] = t;
+    }
 }
 
 // sqrt(scatt_part / energy_part) per orientation (src/outputs_mod.f90:151,154)
@@ -1594,13 +1643,19 @@ __global__ void k2_scale_kernel(double *__restrict__ scale, const pbt_output_par
 
 // Main epilogue: Mueller sum over the chunk's orientations and per-orientation
 // weighted sums  red[o] = {scatt, scatt_beam, scatt_ext, g_num, g_num_beam, g_num_ext}.
-__global__ void k2_epi_kernel(const double *__restrict__ ws, int64_t no, int64_t o0, int64_t nb,
-                              int64_t nphi, const double *__restrict__ phitab,
-                              const double *__restrict__ cth, double waveno,
-                              const double *__restrict__ wbin, int64_t back_bin,
-                              const double *__restrict__ scale, double *__restrict__ mu_sum,
-                              double *__restrict__ part, double *__restrict__ bs) {
-    __shared__ double red[32];
+// blockIdx.y takes every gridDim.y-th orientation; with more than one, each leaves its
+// own Mueller sum in dst + blockIdx.y * 16 nb (k2_fold_kernel adds them), otherwise dst
+// is the running sum, stored (first) or added to.
+// Bound: HBM (128 B a bin and orientation).  A small grid has too few bins to fill the
+// SMs and walked its orientations one after another, twelve block barriers each: 256
+// orientations x 6,552 bins took 745 us, 86 us with the orientations over
+// blockIdx.y and warp sums.
+__global__ void __launch_bounds__(K2_EPI_THREADS)
+    k2_epi_kernel(const double *__restrict__ ws, const int64_t *__restrict__ seg_rec, int64_t no, int64_t o0,
+                  int64_t nb, int64_t nphi, const double *__restrict__ phitab, const double *__restrict__ cth,
+                  double waveno, const double *__restrict__ wbin, int64_t back_bin,
+                  const double *__restrict__ scale, double *__restrict__ dst, int first,
+                  double *__restrict__ part, double *__restrict__ bs) {
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = o < nb;
     const int64_t oo = in ? o : 0;
@@ -1608,16 +1663,17 @@ __global__ void k2_epi_kernel(const double *__restrict__ ws, int64_t no, int64_t
     const double cp = phitab[i], sp = phitab[nphi + i];
     const double W = in ? wbin[oo] / (waveno * waveno) : 0.0;
     const double ct = cth[j];
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5), w = o >> 5;
     double acc[16];
 #pragma unroll
     for (int e = 0; e < 16; e++) acc[e] = 0.0;
-    for (int64_t q = 0; q < no; q++) {
+    for (int64_t q = blockIdx.y; q < no; q += gridDim.y) {
         const int64_t og = o0 + q;
         const double sb = scale ? 1.0 / scale[2 * og] : 1.0;
         const double se = scale ? 1.0 / scale[2 * og + 1] : 1.0;
         Zd Sb[4], Se[4], St[4];
-        ws_ampl(ws, 2 * q, nb, oo, cp, sp, waveno * sb, Sb);
-        ws_ampl(ws, 2 * q + 1, nb, oo, cp, sp, waveno * se, Se);
+        ws_ampl(ws, seg_rec, 2 * q, nb, oo, cp, sp, waveno * sb, Sb);
+        ws_ampl(ws, seg_rec, 2 * q + 1, nb, oo, cp, sp, waveno * se, Se);
 #pragma unroll
         for (int c = 0; c < 4; c++) St[c] = {Sb[c].re + Se[c].re, Sb[c].im + Se[c].im};
         double m[16];
@@ -1628,76 +1684,94 @@ __global__ void k2_epi_kernel(const double *__restrict__ ws, int64_t no, int64_t
                                  re_mc(Sb[3], Sb[3]));
         const double me = 0.5 * (re_mc(Se[0], Se[0]) + re_mc(Se[2], Se[2]) + re_mc(Se[1], Se[1]) +
                                  re_mc(Se[3], Se[3]));
-        double v[6] = {W * m[0], W * mb, W * me, W * ct * m[0], W * ct * mb, W * ct * me};
+        const double v[6] = {W * m[0], W * mb, W * me, W * ct * m[0], W * ct * mb, W * ct * me};
 #pragma unroll
         for (int k = 0; k < 6; k++) {
-            const double s = block_sum(v[k], red);
-            if (threadIdx.x == 0) part[(6 * q + k) * gridDim.x + blockIdx.x] = s;
+            const double t = warp_sum(v[k]);
+            if ((threadIdx.x & 31) == 0) part[(6 * q + k) * nw + w] = t;
         }
         if (in && o == back_bin) bs[og] = m[0] * 4.0 * kPiRef / (waveno * waveno);
     }
-    if (in)
+    if (!in) return;
+    if (gridDim.y > 1) dst += (int64_t)blockIdx.y * 16 * nb;
 #pragma unroll
-        for (int e = 0; e < 16; e++) mu_sum[e * nb + o] += acc[e];
+    for (int e = 0; e < 16; e++) {
+        double *d = dst + e * nb + o;
+        *d = gridDim.y > 1 || first ? acc[e] : *d + acc[e];
+    }
 }
 
-__global__ void k2_final_kernel(const double *__restrict__ redo, const double *__restrict__ bs,
-                                const pbt_output_params *__restrict__ pin, int64_t norient,
-                                pbt_output_params *__restrict__ pout) {
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= norient) return;
-    const double *r = redo + 6 * o;
-    pbt_output_params p = pin[o];
-    const double scatt = r[0], scatt_b = r[1], scatt_e = r[2];
-    p.scatt = scatt;
-    p.ext = p.abs + scatt;
-    p.albedo = 1 - (p.ext - scatt) / p.ext;
-    p.asymmetry = r[3] / scatt;
-    p.abs_eff = p.abs / p.geo_cross_sec;
-    p.scatt_eff = scatt / p.geo_cross_sec;
-    p.ext_eff = p.ext / p.geo_cross_sec;
-    p.back_scatt = bs[o];
-    p.scatt_beam = scatt_b;
-    p.scatt_ext_diff = scatt_e;
-    p.asymmetry_beam = r[4] / scatt_b;
-    p.asymmetry_ext_diff = r[5] / scatt_e;
-    p.scatt_eff_beam = scatt_b / p.geo_cross_sec;
-    p.scatt_eff_ext_diff = scatt_e / p.geo_cross_sec;
-    pout[o] = p;
-}
-
-// Orientation average of the parameters (summation then divide), one thread per field.
-__global__ void k2_param_avg_kernel(const pbt_output_params *__restrict__ per, int64_t norient,
-                                    pbt_output_params *__restrict__ avg) {
-    const int f = threadIdx.x;
-    if (f >= 18) return;
-    const double *src = reinterpret_cast<const double *>(per);
-    double s = 0.0;
-    for (int64_t o = 0; o < norient; o++) s = s + src[18 * o + f];
-    // beam_energy_out / ext_energy_out are not summed by the reference
-    reinterpret_cast<double *>(avg)[f] = (f == 10 || f == 11) ? 0.0 : s / (double)norient;
-}
-
-__global__ void k2_mu_avg_kernel(const double *__restrict__ mu_sum, int64_t n, double inv_n,
-                                 double norient, double *__restrict__ mu_avg) {
+// mu_sum (stored when first, else added to) = the ny partial Mueller sums in order
+__global__ void k2_fold_kernel(const double *__restrict__ part, int ny, int64_t n, int first,
+                               double *__restrict__ mu_sum) {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) mu_avg[q] = mu_sum[q] / norient;
-    (void)inv_n;
+    if (q >= n) return;
+    double s = first ? 0.0 : mu_sum[q];
+    for (int y = 0; y < ny; y++) s += part[y * n + q];
+    mu_sum[q] = s;
 }
 
-__global__ void k2_phi_int_kernel(const double *__restrict__ mu, const double *__restrict__ wphi,
-                                  int64_t nphi, int64_t ntheta, double *__restrict__ m1d) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 16 * ntheta) return;
-    const int64_t j = t % ntheta, e = t / ntheta;
-    const double *src = mu + e * nphi * ntheta + nphi * j;
+// Per-orientation parameters (finalise, src/outputs_mod.f90:133-245), then their
+// orientation average (summation and divide): one block, a warp per field for the
+// average.
+__global__ void __launch_bounds__(608)
+    k2_final_kernel(const double *__restrict__ redo, const double *__restrict__ bs,
+                    const pbt_output_params *__restrict__ pin, int64_t norient,
+                    pbt_output_params *__restrict__ pout, pbt_output_params *__restrict__ avg) {
+    for (int64_t o = threadIdx.x; o < norient; o += blockDim.x) {
+        const double *r = redo + 6 * o;
+        pbt_output_params p = pin[o];
+        const double scatt = r[0], scatt_b = r[1], scatt_e = r[2];
+        p.scatt = scatt;
+        p.ext = p.abs + scatt;
+        p.albedo = 1 - (p.ext - scatt) / p.ext;
+        p.asymmetry = r[3] / scatt;
+        p.abs_eff = p.abs / p.geo_cross_sec;
+        p.scatt_eff = scatt / p.geo_cross_sec;
+        p.ext_eff = p.ext / p.geo_cross_sec;
+        p.back_scatt = bs[o];
+        p.scatt_beam = scatt_b;
+        p.scatt_ext_diff = scatt_e;
+        p.asymmetry_beam = r[4] / scatt_b;
+        p.asymmetry_ext_diff = r[5] / scatt_e;
+        p.scatt_eff_beam = scatt_b / p.geo_cross_sec;
+        p.scatt_eff_ext_diff = scatt_e / p.geo_cross_sec;
+        pout[o] = p;
+    }
+    __threadfence_block();
+    __syncthreads();
+    const int f = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (f >= 18) return;
+    const double *src = reinterpret_cast<const double *>(pout);
     double s = 0.0;
-    for (int64_t i = 0; i < nphi; i++) s += wphi[i] * src[i];
-    m1d[j + ntheta * e] = s;
+    for (int64_t o = lane; o < norient; o += 32) s += src[18 * o + f];
+    s = warp_sum(s);
+    // beam_energy_out / ext_energy_out are not summed by the reference
+    if (lane == 0) reinterpret_cast<double *>(avg)[f] = (f == 10 || f == 11) ? 0.0 : s / (double)norient;
+}
+
+// The orientation average of the Mueller sums and its phi integral: a warp per theta
+// row and element.
+__global__ void k2_avg_kernel(const double *__restrict__ mu_sum, const double *__restrict__ wphi,
+                              int64_t nphi, int64_t ntheta, double norient, double *__restrict__ mu_avg,
+                              double *__restrict__ m1d) {
+    const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (t >= 16 * ntheta) return;
+    const int64_t j = t % ntheta, e = t / ntheta, row = (e * ntheta + j) * nphi;
+    double s = 0.0;
+    for (int64_t i = lane; i < nphi; i += 32) {
+        const double v = mu_sum[row + i] / norient;
+        mu_avg[row + i] = v;
+        s += wphi[i] * v;
+    }
+    s = warp_sum(s);
+    if (lane == 0) m1d[j + ntheta * e] = s;
 }
 
 // FP32 diff_main output: reference-layout complex(8) grids, e^{ik|X|} S' T(phi).
-__global__ void k2_ampl_out_kernel(const double *__restrict__ ws, int64_t nb, int64_t nphi,
+__global__ void k2_ampl_out_kernel(const double *__restrict__ ws, const int64_t *__restrict__ seg_rec,
+                                   int64_t nb, int64_t nphi,
                                    const double *__restrict__ phitab, const double *__restrict__ xyz,
                                    double waveno, double *__restrict__ afb, double *__restrict__ afe) {
     const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1708,7 +1782,7 @@ __global__ void k2_ampl_out_kernel(const double *__restrict__ ws, int64_t nb, in
     sincos(waveno * sqrt(X * X + Y * Y + Zc * Zc), &sK, &cK);
     for (int kind = 0; kind < 2; kind++) {
         Zd S[4];
-        ws_ampl(ws, kind, nb, o, cp, sp, 1.0, S);
+        ws_ampl(ws, seg_rec, kind, nb, o, cp, sp, 1.0, S);
         double *dst = kind ? afe : afb;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -1757,44 +1831,64 @@ struct K2Setup {
     K2Pair *pairs = nullptr;
     K2Fov *fovs = nullptr;
     float2 *rlo = nullptr;  // R_1 - (float)R_1 per record (the y row), pair layout (3 per pair)
-    int64_t *start = nullptr;
-    int64_t *refbase = nullptr;
-    int64_t *beam_off = nullptr;
-    int64_t *ext_off = nullptr;
-    int *err = nullptr;
-    unsigned *epsmax = nullptr;  // float bits of a bound of |com| / R over the records
+    RefSrc src{};
+};
+
+// Error flags of a call (or of all its runs) and a bound of |com| / R over the
+// records, set to zero before the first set-up.
+struct K2Flags {
+    int err, pad;
+    unsigned epsmax, pad2;  // float bits
 };
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Smallest and largest vertex count of the faces.
+struct FaceRange {
+    int64_t lo, hi;
+};
+FaceRange face_range(const int64_t *h_face_off, int64_t nfaces) {
+    FaceRange r{h_face_off[1] - h_face_off[0], 3};
+    for (int64_t f = 0; f < nfaces; f++) {
+        const int64_t nv = h_face_off[f + 1] - h_face_off[f];
+        r.lo = std::min(r.lo, nv);
+        r.hi = std::max(r.hi, nv);
+    }
+    return r;
+}
+
 int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam *d_beam,
                const int64_t *h_beam_off, const pbt_outbeam *d_ext, const int64_t *h_ext_off,
-               const double *d_verts, int64_t nverts, const int64_t *d_face_off,
-               const int64_t *d_face_vi, int64_t nfaces, int64_t max_nv, double lambda,
-               int fast_diff, int variant, K2Setup &S) {
+               const double *d_verts, int64_t nverts, const int64_t *h_face_off,
+               const int64_t *d_face_off, const int64_t *d_face_vi, int64_t nfaces, double lambda,
+               int fast_diff, int variant, K2Flags *flags, K2Setup &S) {
     pbt::NvtxRange nvtx_("pbt: set-up (records)");
     const int64_t nrefs = h_beam_off[norient] + h_ext_off[norient];
-    const int64_t max_recs = std::max<int64_t>(1, nrefs * std::max<int64_t>(1, max_nv - 2));
-    // scan temp size
+    const FaceRange nv = face_range(h_face_off, nfaces);
+    const int64_t max_recs = std::max<int64_t>(1, nrefs * std::max<int64_t>(1, nv.hi - 2));
+    // Faces of one vertex count (triangles nearly always): outbeam g's records start at
+    // g (nv - 2), so the count and its scan (three launches) are for mixed faces only.
+    const bool uniform = nv.lo == nv.hi;
     size_t scan_tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr,
-                                  (int)(nrefs + 1), st);
-    // d_in: cnt | start | refbase | beam_off | ext_off | err | scan tmp
-    const size_t o_cnt = 0, o_start = align_up(o_cnt + (nrefs + 1) * 8),
-                 o_rb = align_up(o_start + (nrefs + 1) * 8),
-                 o_bo = align_up(o_rb + (norient + 1) * 8), o_eo = align_up(o_bo + (norient + 1) * 8),
-                 o_err = align_up(o_eo + (norient + 1) * 8), o_tmp = align_up(o_err + 64),
-                 o_end = align_up(o_tmp + scan_tmp);
+    if (!uniform)
+        cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr,
+                                      (int)(nrefs + 1), st);
+    // d_scan: refbase, beam_off, ext_off | cnt | start | scan tmp
+    const size_t nc = uniform ? 0 : (size_t)(nrefs + 1) * 8;
+    const size_t o_rb = 0, o_cnt = align_up(o_rb + 3 * (norient + 1) * 8), o_start = align_up(o_cnt + nc),
+                 o_tmp = align_up(o_start + nc), o_end = align_up(o_tmp + scan_tmp);
     PBT_TRY(ctx->d_scan.ensure(o_end));
     char *base = ctx->d_scan.as<char>();
-    int64_t *cnt = (int64_t *)(base + o_cnt);
-    S.start = (int64_t *)(base + o_start);
-    S.refbase = (int64_t *)(base + o_rb);
-    S.beam_off = (int64_t *)(base + o_bo);
-    S.ext_off = (int64_t *)(base + o_eo);
-    S.err = (int *)(base + o_err);
-    S.epsmax = (unsigned *)(base + o_err + 8);
-    void *tmp = base + o_tmp;
+    int64_t *rb = (int64_t *)(base + o_rb), *cnt = (int64_t *)(base + o_cnt);
+    RefSrc &src = S.src;
+    src.beam = d_beam;
+    src.ext = d_ext;
+    src.refbase = rb;
+    src.beam_off = rb + (norient + 1);
+    src.ext_off = rb + 2 * (norient + 1);
+    src.norient = norient;
+    src.start = uniform ? nullptr : (int64_t *)(base + o_start);
+    src.per = nv.lo - 2;
     // records (or record pairs; an even count so the last pair is whole)
     const int64_t nrec2 = (max_recs + 1) & ~(int64_t)1;
     const size_t rec_bytes = variant ? (size_t)(nrec2 / 2) * sizeof(K2Pair) : (size_t)max_recs * sizeof(K2Rec);
@@ -1818,29 +1912,28 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
         hs[norient + 1 + o] = h_beam_off[o];
         hs[2 * (norient + 1) + o] = h_ext_off[o];
     }
-    PBT_CUDA_TRY(cudaMemcpyAsync(S.refbase, hs, (norient + 1) * 8, cudaMemcpyHostToDevice, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(S.beam_off, hs + norient + 1, (norient + 1) * 8,
-                                 cudaMemcpyHostToDevice, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(S.ext_off, hs + 2 * (norient + 1), (norient + 1) * 8,
-                                 cudaMemcpyHostToDevice, st));
+    PBT_CUDA_TRY(cudaMemcpyAsync(rb, hs, 3 * (norient + 1) * 8, cudaMemcpyHostToDevice, st));
     if (!ctx->capturing) {
         PBT_CUDA_TRY(cudaEventRecord(ctx->stage_ev, st));
         ctx->stage_pending = true;
     }
-    PBT_CUDA_TRY(cudaMemsetAsync(S.err, 0, 16, st));  // error flags and epsmax
-    // rotation low parts: zero in a pair's unused half (an odd record count)
-    PBT_CUDA_TRY(cudaMemsetAsync(S.rlo, 0, (size_t)(nrec2 / 2) * 3 * sizeof(float2), st));
-    RefSrc src{d_beam, d_ext, S.beam_off, S.ext_off, S.refbase, norient};
-    const int th = 256;
-    k2_count_kernel<<<(unsigned)((nrefs + 1 + th - 1) / th), th, 0, st>>>(src, nrefs, d_face_off,
-                                                                          nfaces, cnt, S.err);
-    PBT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, scan_tmp, cnt, S.start, (int)(nrefs + 1), st));
+    if (!uniform) {
+        const int th = 256;
+        k2_count_kernel<<<(unsigned)((nrefs + 1 + th - 1) / th), th, 0, st>>>(src, nrefs, d_face_off,
+                                                                              nfaces, cnt, &flags->err);
+        PBT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(base + o_tmp, scan_tmp, cnt, (int64_t *)(base + o_start),
+                                                   (int)(nrefs + 1), st));
+        ctx->launches += 2;
+    }
     const double waveno = 2.0 * kPiRef / lambda;
+    // 64 threads: a short list's set-up is one chain of FP64 steps a thread, spread over
+    // the SMs
+    const int th = 64;
     if (nrefs > 0)
         k2_setup_kernel<<<(unsigned)((nrefs + th - 1) / th), th, 0, st>>>(
-            src, nrefs, d_verts, nverts, d_face_off, d_face_vi, S.start, waveno, lambda, fast_diff,
-            S.recs, S.pairs, S.fovs, S.rlo, S.err, S.epsmax);
-    ctx->launches += 3;
+            src, nrefs, d_verts, nverts, d_face_off, nfaces, d_face_vi, waveno, lambda, fast_diff,
+            S.recs, S.pairs, S.fovs, S.rlo, &flags->err, &flags->epsmax);
+    ctx->launches++;
     PBT_CUDA_TRY(cudaGetLastError());
     return PBT_OK;
 }
@@ -1971,18 +2064,20 @@ int k2_fast_tiles(pbt_ctx *ctx, cudaStream_t st, int64_t tile) {
 
 // Records per work item of the default plan: about eight items per resident CTA
 // (four per SM) for the call's records and bin tiles, in multiples of 64, between
-// 256 and 2,048.  Fewer, larger items cost less per item on large lists; on small
-// grids larger items leave the SMs short of work at the end of the launch (a
-// 31,000-outbeam orientation on 16,290 bins: 2.95 ms at 1,024 records per item,
-// 3.56 ms at 4,096).
+// 256 and 2,048.  Fewer, larger items cost less per item on large lists (24 lists of
+// 3,500 on 361 x 180 bins: 22.2 ms at 1,024, 23.6 at 128); on small grids larger items
+// leave the SMs short of work at the end of the launch (a 31,000-outbeam orientation on
+// 16,290 bins: 2.95 ms at 1,024 records per item, 3.56 ms at 4,096).  A call that does
+// not give every resident CTA an item of 256 takes smaller ones, down to 64 (528
+// outbeams on 6,552 bins, a pass: 147 us at 64, 164 at 128, 205 at 256, 157 at 32).
 int64_t k2_auto_rpi(int64_t nrec, int64_t ntiles, int nsm) {
-    const int64_t want = (int64_t)8 * 4 * std::max(nsm, 1);
-    int64_t r = nrec * ntiles / want;
-    r = (r / 64) * 64;
-    return std::min<int64_t>(2048, std::max<int64_t>(256, r));
+    const int64_t slots = (int64_t)4 * std::max(nsm, 1);
+    const int64_t r = (nrec * ntiles / (8 * slots) / 64) * 64;
+    const int64_t one = (nrec * ntiles / slots / 32) * 32;  // one item per resident CTA
+    return std::min<int64_t>({2048, std::max<int64_t>(256, r), std::max<int64_t>(64, one)});
 }
 
-int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, int64_t no,
+int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags, int64_t o0, int64_t no,
                  int64_t nrefs, double lambda, int fast_diff, K2Plan plan, double *ws,
                  int64_t *seg_rec, int64_t *item_pre, unsigned long long *counter) {
     pbt::NvtxRange nvtx_("pbt: far-field sum (FP32)");
@@ -1995,14 +2090,14 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
         ntiles = g.fast_ntiles;
     }
     if (plan.auto_rpi) plan.rpi = k2_auto_rpi(nrefs, ntiles, ctx->sm_count);
-    k2_plan_kernel<<<1, 32, 0, st>>>(S.start, S.refbase, S.beam_off, o0, no, plan.rpi, ntiles,
-                                     seg_rec, item_pre, counter);
-    ctx->launches++;
-    PBT_CUDA_TRY(cudaMemsetAsync(ws, 0, (size_t)2 * no * 8 * g.nb * sizeof(double), st));
     // split tickets of every (segment, tile)
-    const size_t tk_bytes = (size_t)2 * no * ntiles * sizeof(unsigned);
-    PBT_TRY(ctx->d_tk.ensure(tk_bytes));
-    PBT_CUDA_TRY(cudaMemsetAsync(ctx->d_tk.p, 0, tk_bytes, st));
+    const int64_t ntk = 2 * no * ntiles;
+    PBT_TRY(ctx->d_tk.ensure((size_t)ntk * sizeof(unsigned)));
+    const int64_t zb = std::min<int64_t>((ntk + 8 * K2_PLAN_THREADS - 1) / (8 * K2_PLAN_THREADS), 256);
+    k2_plan_kernel<<<(unsigned)(1 + zb), K2_PLAN_THREADS, 0, st>>>(S.src, o0, no, plan.rpi, ntiles, seg_rec,
+                                                                   item_pre, counter,
+                                                                   ctx->d_tk.as<unsigned>());
+    ctx->launches++;
     const double waveno = 2.0 * kPiRef / lambda;
     K2MainArgs A;
     A.recs = S.recs;
@@ -2023,7 +2118,7 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
     A.ws = ws;
     A.tickets = ctx->d_tk.as<unsigned>();
     A.counter = counter;
-    A.err = S.err;
+    A.err = &flags->err;
     if (plan.variant == 1) {
         K2PkArgs B;
         B.pairs = S.pairs;
@@ -2042,11 +2137,11 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
         B.theta_i = A.theta_i;
         B.hkR = A.hkR;
         B.turns = (float)(0.5 * waveno * kFarR * kInvPi);
-        B.epsmax = S.epsmax;
+        B.epsmax = &flags->epsmax;
         B.ws = ws;
         B.tickets = A.tickets;
         B.counter = counter;
-        B.err = S.err;
+        B.err = &flags->err;
         if (plan.bpt == 1)
             return fast_diff ? k2_launch_pk<1, true>(ctx, st, B) : k2_launch_pk<1, false>(ctx, st, B);
         return fast_diff ? k2_launch_pk<2, true>(ctx, st, B) : k2_launch_pk<2, false>(ctx, st, B);
@@ -2054,12 +2149,6 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, int64_t o0, in
     if (plan.bpt == 1)
         return fast_diff ? k2_launch_main<1, true>(ctx, st, A) : k2_launch_main<1, false>(ctx, st, A);
     return fast_diff ? k2_launch_main<2, true>(ctx, st, A) : k2_launch_main<2, false>(ctx, st, A);
-}
-
-int64_t max_face_nv(const int64_t *h_face_off, int64_t nfaces) {
-    int64_t m = 3;
-    for (int64_t f = 0; f < nfaces; f++) m = std::max(m, h_face_off[f + 1] - h_face_off[f]);
-    return m;
 }
 
 }  // namespace
@@ -2115,12 +2204,6 @@ int k2_check_err(pbt_ctx *ctx, cudaStream_t st, const int *d_err) {
 // epilogue into the sums), finish (averages and phi integrals).
 // h_beam_off / h_ext_off (relative to the run) and h_face_off are host arrays;
 // every other array is device memory.
-namespace {
-__global__ void k2_err_fold_kernel(const int *__restrict__ run_err, int *__restrict__ total) {
-    if (threadIdx.x == 0 && *run_err) atomicOr(total, *run_err);
-}
-}  // namespace
-
 int k2_batch_begin(pbt_ctx *ctx, cudaStream_t st, int64_t norient, int64_t max_run,
                    const pbt_output_params *d_params_per, K2Batch &B) {
     const GridCache &g = ctx->grid;
@@ -2132,20 +2215,27 @@ int k2_batch_begin(pbt_ctx *ctx, cudaStream_t st, int64_t norient, int64_t max_r
     const size_t cap = (size_t)16 << 30;
     B.wchunk = std::max<int64_t>(1, std::min<int64_t>(max_run, (int64_t)(cap / per_orient)));
     const int64_t chunk = B.wchunk;
-    // d_ws: workspace | mu_sum | per-orient red (6) | bs | scale (2) | per-orient params | seg/items
-    const size_t o_ws = 0, o_mu = align_up(o_ws + chunk * per_orient),
-                 o_red = align_up(o_mu + 16 * nb * 8), o_bs = align_up(o_red + 6 * norient * 8),
+    // A grid with too few bins for the SMs spreads the epilogue's orientations over
+    // blockIdx.y, up to 32 ways, each with a Mueller sum of its own.
+    const int64_t eblk = (nb + K2_EPI_THREADS - 1) / K2_EPI_THREADS;
+    B.ny = (int)std::max<int64_t>(1, std::min<int64_t>({(8 * ctx->sm_count + eblk - 1) / eblk, chunk, 32}));
+    // d_ws: workspace | mu_sum | partial sums of it | per-orient red (6) | bs | scale (2) |
+    // per-orient params | seg/items | counter | flags | warps' partial sums
+    const size_t o_ws = 0, o_mu = align_up(o_ws + chunk * per_orient), o_mp = align_up(o_mu + 16 * nb * 8),
+                 o_red = align_up(o_mp + (B.ny > 1 ? (size_t)B.ny * 16 * nb * 8 : 0)),
+                 o_bs = align_up(o_red + 6 * norient * 8),
                  o_sc = align_up(o_bs + norient * 8), o_pp = align_up(o_sc + 2 * norient * 8),
                  o_seg = align_up(o_pp + norient * sizeof(pbt_output_params)),
                  o_it = align_up(o_seg + (2 * chunk + 1) * 8), o_cnt = align_up(o_it + (2 * chunk + 1) * 8),
-                 o_err = align_up(o_cnt + 64),
-                 o_part = align_up(o_err + 64),
-                 o_end = align_up(o_part + (size_t)6 * chunk * ((nb + 255) / 256) * 8);
+                 o_flags = align_up(o_cnt + 64),
+                 o_part = align_up(o_flags + sizeof(K2Flags)),
+                 o_end = align_up(o_part + (size_t)6 * chunk * eblk * (K2_EPI_THREADS / 32) * 8);
     PBT_TRY(ctx->d_ws.ensure(o_end));
     char *base = ctx->d_ws.as<char>();
-    B.err = (int *)(base + o_err);
+    B.flags = base + o_flags;
     B.part = (double *)(base + o_part);
-    PBT_CUDA_TRY(cudaMemsetAsync(B.err, 0, sizeof(int), st));
+    B.mu_part = (double *)(base + o_mp);
+    PBT_CUDA_TRY(cudaMemsetAsync(B.flags, 0, sizeof(K2Flags), st));
     B.ws = (double *)(base + o_ws);
     B.mu_sum = (double *)(base + o_mu);
     B.redo = (double *)(base + o_red);
@@ -2155,10 +2245,7 @@ int k2_batch_begin(pbt_ctx *ctx, cudaStream_t st, int64_t norient, int64_t max_r
     B.seg_rec = (int64_t *)(base + o_seg);
     B.item_pre = (int64_t *)(base + o_it);
     B.counter = (unsigned long long *)(base + o_cnt);
-    PBT_CUDA_TRY(cudaMemsetAsync(B.mu_sum, 0, 16 * nb * 8, st));
-    PBT_CUDA_TRY(cudaMemsetAsync(B.redo, 0, 6 * norient * 8, st));
-    PBT_CUDA_TRY(cudaMemsetAsync(B.bs, 0, norient * 8, st));
-    PBT_CUDA_TRY(cudaMemsetAsync(B.scale, 0, 2 * norient * 8, st));
+    B.first = true;
     return PBT_OK;
 }
 
@@ -2170,44 +2257,46 @@ int k2_batch_add(pbt_ctx *ctx, cudaStream_t st, K2Batch &B, int64_t o0, int64_t 
                  const pbt_output_params *d_params_in) {
     const GridCache &g = ctx->grid;
     const int64_t nb = g.nb, nphi = (int64_t)g.phi.size(), ntheta = (int64_t)g.theta.size();
+    K2Flags *flags = (K2Flags *)B.flags;
     K2Setup S;
-    PBT_TRY(k2_prepare(ctx, st, no, d_beam, h_beam_off, d_ext, h_ext_off, d_verts, nverts,
-                       d_face_off, d_face_vi, nfaces, max_face_nv(h_face_off, nfaces), lambda,
-                       fast_diff, B.plan.variant, S));
+    PBT_TRY(k2_prepare(ctx, st, no, d_beam, h_beam_off, d_ext, h_ext_off, d_verts, nverts, h_face_off,
+                       d_face_off, d_face_vi, nfaces, lambda, fast_diff, B.plan.variant, flags, S));
     const double waveno = 2.0 * kPiRef / lambda;
-    const double *phitab = g.phitab.as<double>(), *sth = g.thtab.as<double>(), *cth = sth + ntheta;
-    (void)sth;
+    const double *phitab = g.phitab.as<double>(), *cth = g.thtab.as<double>() + ntheta;
     const int64_t back_bin = 0 + nphi * g.back_i;
-    const int eb = 256;
+    const int eb = K2_EPI_THREADS;
     const unsigned egrid = (unsigned)((nb + eb - 1) / eb);
+    const int64_t nw = (int64_t)egrid * (eb / 32);
     for (int64_t l0 = 0; l0 < no; l0 += B.wchunk) {
         const int64_t n = std::min(B.wchunk, no - l0);
         const int64_t nrefs =
             (h_beam_off[l0 + n] - h_beam_off[l0]) + (h_ext_off[l0 + n] - h_ext_off[l0]);
-        PBT_TRY(k2_run_chunk(ctx, st, S, l0, n, nrefs, lambda, fast_diff, B.plan, B.ws, B.seg_rec,
+        PBT_TRY(k2_run_chunk(ctx, st, S, flags, l0, n, nrefs, lambda, fast_diff, B.plan, B.ws, B.seg_rec,
                              B.item_pre, B.counter));
         const int64_t og = o0 + l0;  // global orientation of the workspace's first slot
         pbt::NvtxRange nvtx_epi("pbt: epilogue (Mueller, orientation sums)");
+        const int ny = (int)std::min<int64_t>(B.ny, n);
+        const dim3 grid(egrid, (unsigned)ny);
         if (scaling) {
-            k2_scatt_be_kernel<<<egrid, eb, 0, st>>>(B.ws, n, og, nb, nphi, phitab, waveno,
-                                                     g.wbin.as<double>(), B.part);
-            k2_part_sum_kernel<<<(unsigned)((2 * n + 3) / 4), 128, 0, st>>>(B.part, 2 * n, egrid,
-                                                                          B.scale + 2 * og);
+            k2_scatt_be_kernel<<<grid, eb, 0, st>>>(B.ws, B.seg_rec, n, nb, nphi, phitab, waveno,
+                                                    g.wbin.as<double>(), B.part);
+            k2_part_sum_kernel<<<(unsigned)(2 * n), 256, 0, st>>>(B.part, nw, B.scale + 2 * og);
             k2_scale_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(B.scale, d_params_in, og, n);
             ctx->launches += 3;
         }
-        k2_epi_kernel<<<egrid, eb, 0, st>>>(B.ws, n, og, nb, nphi, phitab, cth, waveno,
-                                            g.wbin.as<double>(), back_bin, scaling ? B.scale : nullptr,
-                                            B.mu_sum, B.part, B.bs);
-        k2_part_sum_kernel<<<(unsigned)((6 * n + 3) / 4), 128, 0, st>>>(B.part, 6 * n, egrid,
-                                                                      B.redo + 6 * og);
+        k2_epi_kernel<<<grid, eb, 0, st>>>(B.ws, B.seg_rec, n, og, nb, nphi, phitab, cth, waveno,
+                                           g.wbin.as<double>(), back_bin, scaling ? B.scale : nullptr,
+                                           ny > 1 ? B.mu_part : B.mu_sum, B.first ? 1 : 0, B.part, B.bs);
+        k2_part_sum_kernel<<<(unsigned)(6 * n), 256, 0, st>>>(B.part, nw, B.redo + 6 * og);
         ctx->launches += 2;
+        if (ny > 1) {
+            k2_fold_kernel<<<(unsigned)((16 * nb + 255) / 256), 256, 0, st>>>(B.mu_part, ny, 16 * nb,
+                                                                              B.first ? 1 : 0, B.mu_sum);
+            ctx->launches++;
+        }
+        B.first = false;
         PBT_CUDA_TRY(cudaGetLastError());
     }
-    // the run's error flags (its set-up buffer is reused by the next run)
-    k2_err_fold_kernel<<<1, 32, 0, st>>>(S.err, B.err);
-    ctx->launches++;
-    PBT_CUDA_TRY(cudaGetLastError());
     return PBT_OK;
 }
 
@@ -2216,18 +2305,13 @@ int k2_batch_finish(pbt_ctx *ctx, cudaStream_t st, K2Batch &B, const pbt_output_
                     int check_errors) {
     pbt::NvtxRange nvtx_("pbt: orientation average");
     const GridCache &g = ctx->grid;
-    const int64_t nb = g.nb, nphi = (int64_t)g.phi.size(), ntheta = (int64_t)g.theta.size();
-    const int64_t norient = B.norient;
-    k2_final_kernel<<<(unsigned)((norient + 127) / 128), 128, 0, st>>>(B.redo, B.bs, d_params_in,
-                                                                       norient, B.pp);
-    k2_param_avg_kernel<<<1, 32, 0, st>>>(B.pp, norient, d_params_avg);
-    k2_mu_avg_kernel<<<(unsigned)((16 * nb + 255) / 256), 256, 0, st>>>(
-        B.mu_sum, 16 * nb, 1.0 / (double)norient, (double)norient, d_mueller_avg);
-    k2_phi_int_kernel<<<(unsigned)((16 * ntheta + 127) / 128), 128, 0, st>>>(
-        d_mueller_avg, g.wphi.as<double>(), nphi, ntheta, d_m1d_avg);
-    ctx->launches += 4;
+    const int64_t nphi = (int64_t)g.phi.size(), ntheta = (int64_t)g.theta.size();
+    k2_final_kernel<<<1, 608, 0, st>>>(B.redo, B.bs, d_params_in, B.norient, B.pp, d_params_avg);
+    k2_avg_kernel<<<(unsigned)((16 * ntheta + 7) / 8), 256, 0, st>>>(
+        B.mu_sum, g.wphi.as<double>(), nphi, ntheta, (double)B.norient, d_mueller_avg, d_m1d_avg);
+    ctx->launches += 2;
     PBT_CUDA_TRY(cudaGetLastError());
-    if (check_errors) PBT_TRY(k2_check_err(ctx, st, B.err));
+    if (check_errors) PBT_TRY(k2_check_err(ctx, st, &((K2Flags *)B.flags)->err));
     return PBT_OK;
 }
 
@@ -2258,23 +2342,26 @@ int k2_diff_main_impl(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *d_beam, 
     const K2Plan plan = k2_plan_for(ctx);
     K2Setup S;
     const int64_t hbo[2] = {0, nbeam}, heo[2] = {0, next};
-    PBT_TRY(k2_prepare(ctx, st, 1, d_beam, hbo, d_ext, heo, d_verts, nverts, d_face_off, d_face_vi,
-                       nfaces, max_face_nv(h_face_off, nfaces), lambda, fast_diff, plan.variant, S));
     const size_t o_ws = 0, o_seg = align_up(o_ws + (size_t)2 * 8 * nb * sizeof(double)),
-                 o_it = align_up(o_seg + 3 * 8), o_cnt = align_up(o_it + 3 * 8), o_end = align_up(o_cnt + 64);
+                 o_it = align_up(o_seg + 3 * 8), o_cnt = align_up(o_it + 3 * 8),
+                 o_flags = align_up(o_cnt + 64), o_end = align_up(o_flags + sizeof(K2Flags));
     PBT_TRY(ctx->d_ws.ensure(o_end));
     char *base = ctx->d_ws.as<char>();
     double *ws = (double *)(base + o_ws);
-    PBT_TRY(k2_run_chunk(ctx, st, S, 0, 1, nbeam + next, lambda, fast_diff, plan, ws,
-                         (int64_t *)(base + o_seg), (int64_t *)(base + o_it),
-                         (unsigned long long *)(base + o_cnt)));
+    int64_t *seg_rec = (int64_t *)(base + o_seg);
+    K2Flags *flags = (K2Flags *)(base + o_flags);
+    PBT_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(K2Flags), st));
+    PBT_TRY(k2_prepare(ctx, st, 1, d_beam, hbo, d_ext, heo, d_verts, nverts, h_face_off, d_face_off,
+                       d_face_vi, nfaces, lambda, fast_diff, plan.variant, flags, S));
+    PBT_TRY(k2_run_chunk(ctx, st, S, flags, 0, 1, nbeam + next, lambda, fast_diff, plan, ws, seg_rec,
+                         (int64_t *)(base + o_it), (unsigned long long *)(base + o_cnt)));
     const double waveno = 2.0 * kPiRef / lambda;
     k2_ampl_out_kernel<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(
-        ws, nb, (int64_t)g.phi.size(), g.phitab.as<double>(), g.xyz.as<double>(), waveno, d_afb,
+        ws, seg_rec, nb, (int64_t)g.phi.size(), g.phitab.as<double>(), g.xyz.as<double>(), waveno, d_afb,
         d_afe);
     ctx->launches++;
     PBT_CUDA_TRY(cudaGetLastError());
-    return k2_check_err(ctx, st, S.err);
+    return k2_check_err(ctx, st, &flags->err);
 }
 
 }  // namespace pbt

@@ -227,11 +227,14 @@ struct K2Batch {
     K2Plan plan;
     double *ws = nullptr;
     double *mu_sum = nullptr, *redo = nullptr, *bs = nullptr, *scale = nullptr;
-    double *part = nullptr;  // per-block partial sums of the epilogue (6 per orientation and block)
+    double *part = nullptr;  // per-warp partial sums of the epilogue (6 per orientation and warp)
+    double *mu_part = nullptr;  // ny partial Mueller sums of the epilogue (ny > 1)
+    int ny = 1;
+    bool first = true;       // mu_sum holds nothing yet
     pbt_output_params *pp = nullptr;
     int64_t *seg_rec = nullptr, *item_pre = nullptr;
     unsigned long long *counter = nullptr;
-    int *err = nullptr;
+    void *flags = nullptr;   // error flags and the bound of |com| / R, over all runs
 };
 int k2_batch_begin(pbt_ctx *ctx, cudaStream_t st, int64_t norient, int64_t max_run,
                    const pbt_output_params *d_params_per, K2Batch &B);

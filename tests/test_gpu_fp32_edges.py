@@ -121,3 +121,41 @@ def test_batch_odd_segments(ctx):
     a = ctx.diff_batch(beams, exts, V, geo, th, ph, LAM, pin, precision="fp32")
     b = ctx.diff_batch(beams, exts, V, geo, th, ph, LAM, pin, precision="fp64")
     assert mueller_rel_err(a[0], b[0]) <= 1e-4
+
+
+@pytest.mark.parametrize("norient,nt,nphi", [(1, 5, 3), (3, 41, 33), (40, 7, 5), (70, 16, 16)])
+@pytest.mark.parametrize("corners", [3, 4, 0])
+@pytest.mark.parametrize("scaling", [False, True])
+def test_many_orientations(ctx, norient, nt, nphi, corners, scaling):
+    """Epilogue over several orientation groups, lists of triangles, of quads and mixed, some of
+    them empty: FP32 average and per-orientation parameters against the FP64 path (1e-4 of a
+    bin's M11, 1e-5 of the cross sections, the package's bars)."""
+    rng = np.random.default_rng(norient + corners)
+    nf = 12
+    nv = np.full(nf, corners) if corners else rng.integers(3, 7, size=nf)
+    verts, faces = [], []
+    for n in nv:
+        e = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        ang = 2 * np.pi * (np.arange(n) + rng.uniform(0, 0.5, size=n)) / n
+        faces.append(list(range(len(verts) + 1, len(verts) + n + 1)))
+        verts += list(rng.uniform(-3, 3, size=3) + np.cos(ang)[:, None] * e[0] + np.sin(ang)[:, None] * e[1])
+    geo = abt_b200.make_geometry(np.array(verts), faces)
+    beams = [outbeams(int(m), rng, nf) for m in rng.integers(1, 12, size=norient)]
+    exts = [outbeams(int(m), rng, nf, prop=(0, 0, -1)) for m in rng.integers(1, 9, size=norient)]
+    if norient > 2 and not scaling:
+        exts[1] = exts[1][:0]
+        beams[2] = beams[2][:0]
+    V = [geo["verts"]] * norient
+    pin = np.array([abt_b200.params(abs=0.3, geo_cross_sec=10.0, beam_energy_out=2.0)] * norient,
+                   dtype=abt_b200.PARAMS_DTYPE)
+    th = np.linspace(3.0, 180.0, nt) * abt_b200.PI_REF / 180.0
+    ph = (0.3 + np.arange(nphi) * 360.0 / nphi) * abt_b200.PI_REF / 180.0
+    a = ctx.diff_batch(beams, exts, V, geo, th, ph, LAM, pin, precision="fp32", scaling=scaling)
+    b = ctx.diff_batch(beams, exts, V, geo, th, ph, LAM, pin, precision="fp64", scaling=scaling)
+    assert mueller_rel_err(a[0], b[0]) <= 1e-4
+    for x, y in ((a[2], b[2]), (a[3], b[3])):
+        u, v = (np.atleast_1d(p).view(np.float64).reshape(-1, 18) for p in (x, y))
+        assert np.array_equal(np.isnan(u), np.isnan(v))
+        # the parameters but the back-scattering one (a single bin's M11, under the Mueller bar)
+        cols = [c for c in range(18) if c != 9]
+        np.testing.assert_allclose(u[:, cols], v[:, cols], rtol=1e-5, atol=1e-5)
