@@ -98,11 +98,9 @@ int check_grid_ready(pbt_ctx *ctx) {
 }
 
 template <class T>
-int upload(DevBuf &buf, const T *src, size_t n, cudaStream_t st, size_t off_bytes = 0) {
+int upload(pbt_ctx *ctx, DevBuf &buf, const T *src, size_t n, cudaStream_t st, size_t off_bytes = 0) {
     PBT_TRY(buf.ensure(off_bytes + std::max<size_t>(n * sizeof(T), 16)));
-    if (n) PBT_CUDA_TRY(cudaMemcpyAsync(buf.as<char>() + off_bytes, src, n * sizeof(T),
-                                        cudaMemcpyHostToDevice, st));
-    return PBT_OK;
+    return n ? copy_to_device(ctx, buf.as<char>() + off_bytes, src, n * sizeof(T), st) : PBT_OK;
 }
 
 size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -120,8 +118,8 @@ int fp64_diff_main_device(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam
     // external diffraction: fov forced to pi/2, src/diff_mod.f90:797
     PBT_TRY(k1_build_facets(ext, next, kPiRef / 2.0, verts, nverts, face_off, face_vi, nfaces,
                             lambda, fac, edges));
-    PBT_TRY(upload(ctx->d_fac, fac.data(), fac.size(), st));
-    PBT_TRY(upload(ctx->d_edge, edges.data(), edges.size(), st));
+    PBT_TRY(upload(ctx, ctx->d_fac, fac.data(), fac.size(), st));
+    PBT_TRY(upload(ctx, ctx->d_edge, edges.data(), edges.size(), st));
     PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), nbeam, next, ctx->d_edge.as<K1Edge>(), lambda,
                       fast_diff, d_afb, d_afe));
     // the host vectors are released at return: finish the copies first
@@ -144,11 +142,10 @@ int upload_geometry(pbt_ctx *ctx, cudaStream_t st, const double *verts, int64_t 
                  o_end = al(o_v + (size_t)norient * 3 * nverts * 8);
     PBT_TRY(ctx->d_in.ensure(o_end));
     char *b = ctx->d_in.as<char>();
-    PBT_CUDA_TRY(cudaMemcpyAsync(b + o_fo, face_off, (nfaces + 1) * 8, cudaMemcpyHostToDevice, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(b + o_fv, face_vi, nvi * 8, cudaMemcpyHostToDevice, st));
+    PBT_TRY(copy_to_device(ctx, b + o_fo, face_off, (nfaces + 1) * 8, st));
+    PBT_TRY(copy_to_device(ctx, b + o_fv, face_vi, nvi * 8, st));
     if (verts)  // else the caller copies the orientations' blocks
-        PBT_CUDA_TRY(cudaMemcpyAsync(b + o_v, verts, (size_t)norient * 3 * nverts * 8,
-                                     cudaMemcpyHostToDevice, st));
+        PBT_TRY(copy_to_device(ctx, b + o_v, verts, (size_t)norient * 3 * nverts * 8, st));
     G.face_off = (const int64_t *)(b + o_fo);
     G.face_vi = (const int64_t *)(b + o_fv);
     G.verts = (const double *)(b + o_v);
@@ -217,18 +214,14 @@ extern "C" int pbt_diff_main_c(pbt_ctx *ctx, const pbt_outbeam *beam, int64_t nb
         PBT_TRY(ctx->d_fac.ensure(al((nbeam + 1) * ob) + (next + 1) * ob));
         pbt_outbeam *d_beam = ctx->d_fac.as<pbt_outbeam>();
         pbt_outbeam *d_ext = (pbt_outbeam *)(ctx->d_fac.as<char>() + al((nbeam + 1) * ob));
-        if (nbeam) PBT_CUDA_TRY(cudaMemcpyAsync(d_beam, beam, nbeam * ob, cudaMemcpyHostToDevice, st));
-        if (next) PBT_CUDA_TRY(cudaMemcpyAsync(d_ext, ext, next * ob, cudaMemcpyHostToDevice, st));
+        if (nbeam) PBT_TRY(copy_to_device(ctx, d_beam, beam, nbeam * ob, st));
+        if (next) PBT_TRY(copy_to_device(ctx, d_ext, ext, next * ob, st));
         PBT_TRY(k2_diff_main_impl(ctx, st, d_beam, nbeam, d_ext, next, G.verts, nverts, face_off,
                                   G.face_off, G.face_vi, nfaces, lambda, is_fast_diff ? 1 : 0, d_afb,
                                   d_afe));
     }
-    PBT_CUDA_TRY(cudaMemcpyAsync(ampl_far_beam, d_afb, 8 * nb * sizeof(double),
-                                 cudaMemcpyDeviceToHost, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(ampl_far_ext_diff, d_afe, 8 * nb * sizeof(double),
-                                 cudaMemcpyDeviceToHost, st));
-    PBT_CUDA_TRY(cudaStreamSynchronize(st));
-    return PBT_OK;
+    PBT_TRY(copy_to_host(ctx, ampl_far_beam, d_afb, 8 * nb * sizeof(double), st));
+    return copy_to_host(ctx, ampl_far_ext_diff, d_afe, 8 * nb * sizeof(double), st);
 }
 
 extern "C" int pbt_diffraction_c(pbt_ctx *ctx, const pbt_outbeam *outbeam, const double *verts,
@@ -252,15 +245,12 @@ extern "C" int pbt_diffraction_c(pbt_ctx *ctx, const pbt_outbeam *outbeam, const
     std::vector<K1Edge> edges;
     PBT_TRY(k1_build_facets(outbeam, 1, -1.0, verts, nverts, face_off, face_vi, nfaces, lambda, fac,
                             edges));
-    PBT_TRY(upload(ctx->d_fac, fac.data(), fac.size(), st));
-    PBT_TRY(upload(ctx->d_edge, edges.data(), edges.size(), st));
+    PBT_TRY(upload(ctx, ctx->d_fac, fac.data(), fac.size(), st));
+    PBT_TRY(upload(ctx, ctx->d_edge, edges.data(), edges.size(), st));
     PBT_TRY(ctx->d_out.ensure(8 * nb * sizeof(double)));
     PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), 1, 0, ctx->d_edge.as<K1Edge>(), lambda,
                       is_fast_diff ? 1 : 0, ctx->d_out.as<double>(), nullptr));
-    PBT_CUDA_TRY(cudaMemcpyAsync(amplC, ctx->d_out.p, 8 * nb * sizeof(double),
-                                 cudaMemcpyDeviceToHost, st));
-    PBT_CUDA_TRY(cudaStreamSynchronize(st));
-    return PBT_OK;
+    return copy_to_host(ctx, amplC, ctx->d_out.p, 8 * nb * sizeof(double), st);
 }
 
 extern "C" int pbt_finalise_c(pbt_ctx *ctx, const double *ampl_far_beam,
@@ -283,22 +273,14 @@ extern "C" int pbt_finalise_c(pbt_ctx *ctx, const double *ampl_far_beam,
     PBT_TRY(ctx->d_mu.ensure((16 * nb + 16 * ntheta + 18) * sizeof(double)));
     double *d_afb = ctx->d_out.as<double>(), *d_afe = d_afb + 8 * nb;
     double *d_mu = ctx->d_mu.as<double>(), *d_m1 = d_mu + 16 * nb, *d_p = d_m1 + 16 * ntheta;
-    PBT_CUDA_TRY(cudaMemcpyAsync(d_afb, ampl_far_beam, 8 * nb * sizeof(double),
-                                 cudaMemcpyHostToDevice, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(d_afe, ampl_far_ext_diff, 8 * nb * sizeof(double),
-                                 cudaMemcpyHostToDevice, st));
+    PBT_TRY(copy_to_device(ctx, d_afb, ampl_far_beam, 8 * nb * sizeof(double), st));
+    PBT_TRY(copy_to_device(ctx, d_afe, ampl_far_ext_diff, 8 * nb * sizeof(double), st));
     const pbt_output_params pin = *params;
     PBT_TRY(k3_finalise(ctx, st, d_afb, d_afe, lambda, scaling ? 1 : 0, &pin, d_mu, d_m1, d_p,
                         accumulate ? &ctx->tot : nullptr));
-    if (mueller)
-        PBT_CUDA_TRY(cudaMemcpyAsync(mueller, d_mu, 16 * nb * sizeof(double),
-                                     cudaMemcpyDeviceToHost, st));
-    if (mueller_1d)
-        PBT_CUDA_TRY(cudaMemcpyAsync(mueller_1d, d_m1, 16 * ntheta * sizeof(double),
-                                     cudaMemcpyDeviceToHost, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(params, d_p, sizeof(pbt_output_params), cudaMemcpyDeviceToHost, st));
-    PBT_CUDA_TRY(cudaStreamSynchronize(st));
-    return PBT_OK;
+    if (mueller) PBT_TRY(copy_to_host(ctx, mueller, d_mu, 16 * nb * sizeof(double), st));
+    if (mueller_1d) PBT_TRY(copy_to_host(ctx, mueller_1d, d_m1, 16 * ntheta * sizeof(double), st));
+    return copy_to_host(ctx, params, d_p, sizeof(pbt_output_params), st);
 }
 
 extern "C" int pbt_summation_c(pbt_ctx *ctx, const double *mueller, const double *mueller_1d,
@@ -312,7 +294,7 @@ extern "C" int pbt_summation_c(pbt_ctx *ctx, const double *mueller, const double
     const int64_t nb = ntheta * nphi;
     PBT_TRY(ctx->d_mu.ensure((16 * nb + 16 * ntheta + 18) * sizeof(double)));
     double *d_mu = ctx->d_mu.as<double>(), *d_m1 = d_mu + 16 * nb, *d_p = d_m1 + 16 * ntheta;
-    PBT_CUDA_TRY(cudaMemcpyAsync(d_mu, mueller, 16 * nb * 8, cudaMemcpyHostToDevice, st));
+    PBT_TRY(copy_to_device(ctx, d_mu, mueller, 16 * nb * 8, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(d_m1, mueller_1d, 16 * ntheta * 8, cudaMemcpyHostToDevice, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(d_p, params, sizeof(pbt_output_params), cudaMemcpyHostToDevice, st));
     PBT_TRY(totals_add_device(ctx, ctx->tot, st, d_mu, d_m1, d_p));
@@ -336,7 +318,7 @@ extern "C" int pbt_divide_by_num_orientations_c(pbt_ctx *ctx, int64_t num_orient
     PBT_TRY(ctx->d_mu.ensure((16 * nb + 16 * nt + 18) * sizeof(double)));
     double *d_mu = ctx->d_mu.as<double>(), *d_m1 = d_mu + 16 * nb, *d_p = d_m1 + 16 * nt;
     PBT_TRY(totals_divide_device(ctx, ctx->tot, st, num_orients, d_mu, d_m1, d_p));
-    PBT_CUDA_TRY(cudaMemcpyAsync(mueller_total, d_mu, 16 * nb * 8, cudaMemcpyDeviceToHost, st));
+    PBT_TRY(copy_to_host(ctx, mueller_total, d_mu, 16 * nb * 8, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(mueller_1d_total, d_m1, 16 * nt * 8, cudaMemcpyDeviceToHost, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(params_total, d_p, sizeof(pbt_output_params),
                                  cudaMemcpyDeviceToHost, st));
@@ -456,7 +438,7 @@ int host_batch(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const HostRuns &H
                                              cudaMemcpyDeviceToHost, st));
         }
         PBT_TRY(totals_divide_device(ctx, T, st, norient, d_mu, d_m1, d_p));
-        PBT_CUDA_TRY(cudaMemcpyAsync(mueller_avg, d_mu, 16 * nb * 8, cudaMemcpyDeviceToHost, st));
+        PBT_TRY(copy_to_host(ctx, mueller_avg, d_mu, 16 * nb * 8, st));
         PBT_CUDA_TRY(cudaMemcpyAsync(mueller_1d_avg, d_m1, 16 * ntheta * 8, cudaMemcpyDeviceToHost, st));
         PBT_CUDA_TRY(cudaMemcpyAsync(params_avg, d_p, sizeof(pbt_output_params),
                                      cudaMemcpyDeviceToHost, st));
@@ -580,7 +562,7 @@ int host_batch(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const HostRuns &H
         if (nrun > 1) PBT_CUDA_TRY(cudaEventRecord(ctx->done_ev[slot], st));
     }
     PBT_TRY(k2_batch_finish(ctx, st, B, d_pin, d_mu, d_m1, d_pa, 1));
-    PBT_CUDA_TRY(cudaMemcpyAsync(mueller_avg, d_mu, 16 * nb * 8, cudaMemcpyDeviceToHost, st));
+    PBT_TRY(copy_to_host(ctx, mueller_avg, d_mu, 16 * nb * 8, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(mueller_1d_avg, d_m1, 16 * ntheta * 8, cudaMemcpyDeviceToHost, st));
     PBT_CUDA_TRY(cudaMemcpyAsync(params_avg, d_pa, sizeof(pbt_output_params), cudaMemcpyDeviceToHost,
                                  st));

@@ -2,7 +2,9 @@
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <string.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "pbt_internal.h"
@@ -72,6 +74,96 @@ void HostBuf::release() {
     if (p) cudaFreeHost(p);
     p = nullptr;
     cap = 0;
+}
+
+namespace {
+
+// Whether `p` is plain pageable memory (the driver copies pinned and managed memory best).
+bool pageable(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Pinning the slots costs about as much as ten copies gain, so a context takes them
+// only after kIoRent large copies by the driver.
+bool io_rented(pbt_ctx *ctx) { return ctx->io_copies < kIoRent && ++ctx->io_copies; }
+
+int io_prepare(pbt_ctx *ctx) {
+    PBT_TRY(ctx->h_io.ensure(kIoSlots * kIoChunk));
+    for (int i = 0; i < kIoSlots; i++)
+        if (!ctx->io_ev[i])
+            PBT_CUDA_TRY(cudaEventCreateWithFlags(&ctx->io_ev[i], cudaEventDisableTiming));
+    return PBT_OK;
+}
+
+// memcpy of a chunk, by up to eight threads in 64 KB pieces when the whole copy is
+// kIoPar or more (2.1 MB out: 113 us a call against 186 on one thread).  Smaller ones
+// stay on the calling thread: the threads wait actively for a while afterwards, and a
+// caller with threaded work of its own (the torch operations of a gradient step on
+// 6,000 bins) lost 4 % to them.
+void copy_threads(char *dst, const char *src, size_t n, bool par) {
+    const int64_t piece = 64 << 10, np = (int64_t)((n + piece - 1) / piece);
+#pragma omp parallel for schedule(static) num_threads(8) if (par && np > 1)
+    for (int64_t i = 0; i < np; i++)
+        memcpy(dst + i * piece, src + i * piece, std::min<size_t>(piece, n - i * piece));
+}
+
+}  // namespace
+
+// The driver moves pageable memory through a pinned buffer of its own with one thread:
+// 2.1 MB to the host took 138 us, 8.3 MB 438 us, against 49 and 159 us of transfer.
+// Here the transfer of one chunk runs while the host threads move the chunks before it.
+int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    if (bytes < kIoMin || !pageable(dst) || io_rented(ctx)) {
+        PBT_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+        PBT_CUDA_TRY(cudaStreamSynchronize(st));
+        return PBT_OK;
+    }
+    PBT_TRY(io_prepare(ctx));
+    char *pin = ctx->h_io.as<char>();
+    const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
+    auto size_of = [&](size_t c) { return std::min(kIoChunk, bytes - c * kIoChunk); };
+    for (size_t c = 0; c < nch + kIoSlots - 1; c++) {
+        if (c < nch) {
+            const size_t s = c % kIoSlots;
+            PBT_CUDA_TRY(cudaMemcpyAsync(pin + s * kIoChunk, (const char *)src + c * kIoChunk, size_of(c),
+                                         cudaMemcpyDeviceToHost, st));
+            PBT_CUDA_TRY(cudaEventRecord(ctx->io_ev[s], st));
+        }
+        if (c + 1 >= kIoSlots) {
+            // the oldest chunk in flight; its slot is free for chunk c + 1
+            const size_t d = c + 1 - kIoSlots, s = d % kIoSlots;
+            if (d >= nch) continue;
+            PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
+            copy_threads((char *)dst + d * kIoChunk, pin + s * kIoChunk, size_of(d),
+                         bytes >= kIoPar);
+        }
+    }
+    return PBT_OK;
+}
+
+int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    if (bytes < kIoMin || !pageable(src) || io_rented(ctx)) {
+        PBT_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+        return PBT_OK;
+    }
+    PBT_TRY(io_prepare(ctx));
+    char *pin = ctx->h_io.as<char>();
+    const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
+    for (size_t c = 0; c < nch; c++) {
+        const size_t s = c % kIoSlots, n = std::min(kIoChunk, bytes - c * kIoChunk);
+        // the slot's last transfer, of this copy or of an earlier one
+        PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
+        copy_threads(pin + s * kIoChunk, (const char *)src + c * kIoChunk, n, bytes >= kIoPar);
+        PBT_CUDA_TRY(cudaMemcpyAsync((char *)dst + c * kIoChunk, pin + s * kIoChunk, n,
+                                     cudaMemcpyHostToDevice, st));
+        PBT_CUDA_TRY(cudaEventRecord(ctx->io_ev[s], st));
+    }
+    return PBT_OK;
 }
 
 void timing_begin(pbt_ctx *ctx, cudaStream_t st) {
@@ -246,6 +338,9 @@ extern "C" int pbt_ctx_destroy(pbt_ctx *ctx) {
         ctx->tot.release();
         ctx->btot.release();
         ctx->h_stage.release();
+        ctx->h_io.release();
+        for (cudaEvent_t e : ctx->io_ev)
+            if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
         if (ctx->stage_ev) cudaEventDestroy(ctx->stage_ev);
         for (int i = 0; i < 2; i++) {

@@ -992,19 +992,19 @@ int k4_adjoint(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam, int64_t n
     if (nrec > 0) {
         // the FP64 set-up of each record on the device (the same frame code as the
         // forward's set-up), one thread per record
-        if (nbeam) PBT_CUDA_TRY(cudaMemcpyAsync(d_ob, beam, nbeam * ob, cudaMemcpyHostToDevice, st));
-        if (next) PBT_CUDA_TRY(cudaMemcpyAsync(d_ob + nbeam, ext, next * ob, cudaMemcpyHostToDevice, st));
-        PBT_CUDA_TRY(cudaMemcpyAsync(base + o_vert, verts, 3 * nverts * 8, cudaMemcpyHostToDevice, st));
-        PBT_CUDA_TRY(cudaMemcpyAsync(base + o_fo, face_off, (nfaces + 1) * 8, cudaMemcpyHostToDevice, st));
-        PBT_CUDA_TRY(cudaMemcpyAsync(base + o_fv, face_vi, nvi * 8, cudaMemcpyHostToDevice, st));
+        if (nbeam) PBT_TRY(copy_to_device(ctx, d_ob, beam, nbeam * ob, st));
+        if (next) PBT_TRY(copy_to_device(ctx, d_ob + nbeam, ext, next * ob, st));
+        PBT_TRY(copy_to_device(ctx, base + o_vert, verts, 3 * nverts * 8, st));
+        PBT_TRY(copy_to_device(ctx, base + o_fo, face_off, (nfaces + 1) * 8, st));
+        PBT_TRY(copy_to_device(ctx, base + o_fv, face_vi, nvi * 8, st));
         k4_setup_kernel<<<(unsigned)((nrec + 127) / 128), 128, 0, st>>>(
             d_ob, nbeam, d_ob + nbeam, nrec, (const double *)(base + o_vert), nverts,
             (const int64_t *)(base + o_fo), (const int64_t *)(base + o_fv), k, lambda,
             (K4Rec *)(base + o_rec), (int *)(base + o_kind), (float *)(base + o_fov), d_h);
         PBT_CUDA_TRY(cudaMemsetAsync(base + o_out, 0, nrec * K4_NACC * 8, st));
     }
-    PBT_CUDA_TRY(cudaMemcpyAsync(base + o_ga, gafb, 8 * nb * 8, cudaMemcpyHostToDevice, st));
-    PBT_CUDA_TRY(cudaMemcpyAsync(base + o_gb, gafe, 8 * nb * 8, cudaMemcpyHostToDevice, st));
+    PBT_TRY(copy_to_device(ctx, base + o_ga, gafb, 8 * nb * 8, st));
+    PBT_TRY(copy_to_device(ctx, base + o_gb, gafe, 8 * nb * 8, st));
     k4_prep_kernel<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(
         (const double *)(base + o_ga), (const double *)(base + o_gb), g.xyz.as<double>(),
         g.phitab.as<double>(), nb, nphi, k, (K4Bin *)(base + o_bin),
@@ -1067,10 +1067,10 @@ int k4_adjoint(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam, int64_t n
             d_gamp, d_gamp + 8 * nbeam, d_gv);
     ctx->launches += nrec > 0 ? 2 : 0;
     PBT_CUDA_TRY(cudaGetLastError());
-    PBT_CUDA_TRY(cudaMemcpyAsync(gverts, d_gv, 3 * nverts * 8, cudaMemcpyDeviceToHost, st));
-    if (nbeam) PBT_CUDA_TRY(cudaMemcpyAsync(gbeam, d_gamp, nbeam * 8 * 8, cudaMemcpyDeviceToHost, st));
+    PBT_TRY(copy_to_host(ctx, gverts, d_gv, 3 * nverts * 8, st));
+    if (nbeam) PBT_TRY(copy_to_host(ctx, gbeam, d_gamp, nbeam * 8 * 8, st));
     if (next)
-        PBT_CUDA_TRY(cudaMemcpyAsync(gext, d_gamp + 8 * nbeam, next * 8 * 8, cudaMemcpyDeviceToHost, st));
+        PBT_TRY(copy_to_host(ctx, gext, d_gamp + 8 * nbeam, next * 8 * 8, st));
     PBT_CUDA_TRY(cudaStreamSynchronize(st));
     return PBT_OK;
 }

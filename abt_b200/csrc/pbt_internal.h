@@ -82,6 +82,14 @@ struct HostBuf {
     T *as() const { return static_cast<T *>(p); }
 };
 
+// Pinned staging of large copies between the caller's pageable arrays and the device
+// (kIoSlots slots of kIoChunk bytes a context, allocated on first use).
+constexpr int kIoSlots = 4;
+constexpr size_t kIoChunk = (size_t)512 << 10;
+constexpr size_t kIoMin = (size_t)256 << 10;  // smaller copies go to the driver as they are
+constexpr size_t kIoPar = (size_t)1536 << 10; // copies from here on use several host threads
+constexpr int kIoRent = 8;                    // large copies of a context before it pins them
+
 // ------------------------------------------- reference-exact FP64 records
 // One outgoing facet, prepared for the FP64 kernel (all values formed in the
 // reference's operation order).  384 bytes, in the order the kernel reads it
@@ -158,6 +166,9 @@ struct pbt_ctx {
     pbt::DevBuf d_tk;  // split tickets of the FP32 kernel's (segment, tile) pairs
     pbt::DevBuf d_k1part;  // FP64 drop-in: partial grids of the facet splits (small grids)
     pbt::HostBuf h_stage;
+    pbt::HostBuf h_io;               // pinned slots of copy_to_host / copy_to_device
+    cudaEvent_t io_ev[pbt::kIoSlots] = {};
+    int io_copies = 0;               // large copies left to the driver so far
     cudaEvent_t stage_ev = nullptr;  // last copy out of h_stage (wait before reuse)
     bool stage_pending = false;
     pbt::DevTotals tot;    // user-visible totals (pbt_summation_c / pbt_finalise_c accumulate)
@@ -178,6 +189,10 @@ struct pbt_ctx {
 namespace pbt {
 
 // ----------------------------------------------------------- host helpers
+// Copies on st between the caller's host array and the device.  copy_to_host returns
+// when the data are in dst; copy_to_device when src may be changed.
+int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st);
+int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st);
 int validate_geometry(const double *verts, int64_t nverts, const int64_t *face_off,
                       const int64_t *face_vi, int64_t nfaces);
 int validate_angles(const double *theta, int64_t ntheta, const double *phi, int64_t nphi);

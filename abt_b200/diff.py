@@ -187,7 +187,7 @@ class Context:
         v, fo, fv = _geo(geometry)
         theta = np.ascontiguousarray(theta, dtype=np.float64)
         phi = np.ascontiguousarray(phi, dtype=np.float64)
-        out = np.zeros((len(phi), len(theta), 2, 2), dtype=np.complex128, order="F")
+        out = np.empty((len(phi), len(theta), 2, 2), dtype=np.complex128, order="F")
         check(_lib.lib().pbt_diffraction_c(self._h, ptr(ob), ptr(v), v.shape[0], ptr(fo), ptr(fv),
                                            len(fo) - 1, ptr(theta), len(theta), ptr(phi),
                                            len(phi), float(lam), int(bool(is_fast_diff)),
@@ -211,9 +211,9 @@ class Context:
         shape = (len(phi), len(theta), 2, 2)
         if ga.shape != shape or ge.shape != shape:
             raise ValueError(f"cotangent shape must be {shape}")
-        gv = np.zeros((v.shape[0], 3), order="F")
-        gb = np.zeros((max(len(beam), 1), 8))
-        gx = np.zeros((max(len(ext), 1), 8))
+        gv = np.empty((v.shape[0], 3), order="F")
+        gb = np.empty((max(len(beam), 1), 8))
+        gx = np.empty((max(len(ext), 1), 8))
         check(_lib.lib().pbt_diff_adjoint_c(self._h, ptr(beam), len(beam), ptr(ext), len(ext),
                                             ptr(v), v.shape[0], ptr(fo), ptr(fv), len(fo) - 1,
                                             ptr(theta), len(theta), ptr(phi), len(phi), float(lam),
@@ -231,8 +231,8 @@ class Context:
         afb = np.asfortranarray(ampl_far_beam, dtype=np.complex128)
         afe = np.asfortranarray(ampl_far_ext_diff, dtype=np.complex128)
         p = np.array(params_in, dtype=PARAMS_DTYPE).copy()
-        mu = np.zeros((len(phi), len(theta), 16), order="F")
-        mu1 = np.zeros((len(theta), 16), order="F")
+        mu = np.empty((len(phi), len(theta), 16), order="F")
+        mu1 = np.empty((len(theta), 16), order="F")
         check(_lib.lib().pbt_finalise_c(self._h, afb.ctypes.data, afe.ctypes.data, ptr(theta),
                                         len(theta), ptr(phi), len(phi), float(lam),
                                         int(bool(scaling)), p.ctypes.data, mu.ctypes.data,
@@ -249,8 +249,8 @@ class Context:
 
     def divide_by_num_orientations(self, num_orients, ntheta, nphi):
         """divide_by_num_orientations (src/outputs_mod.f90:13-43) of the device totals."""
-        mu = np.zeros((nphi, ntheta, 16), order="F")
-        mu1 = np.zeros((ntheta, 16), order="F")
+        mu = np.empty((nphi, ntheta, 16), order="F")
+        mu1 = np.empty((ntheta, 16), order="F")
         p = np.zeros((), dtype=PARAMS_DTYPE)
         check(_lib.lib().pbt_divide_by_num_orientations_c(self._h, int(num_orients),
                                                           mu.ctypes.data, mu1.ctypes.data,
