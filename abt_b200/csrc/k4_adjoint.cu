@@ -15,12 +15,12 @@
 // the frame the reference builds from angles (src/diff_mod.f90:200-289,
 // 540-559).  Per facet x bin the kernel recomputes the forward quantities and
 // back-propagates; everything that depends on the bin only through a linear
-// map of per-facet data is accumulated as a per-facet sum over bins (36
+// map of per-facet data is accumulated as a per-facet sum over bins (30
 // floats), so no facet x bin intermediate is stored.  A host pass in FP64 then
 // maps those sums through the frame construction to the vertex gradients.
 //
 // Layout: one warp per record (4 per CTA), lanes striding over a range of
-// bins with the 36 sums in registers; one warp reduction and one FP64 atomic
+// bins with the 30 sums in registers; one warp reduction and one FP64 atomic
 // per (record, bin range) at the end.
 #include <math.h>
 #include <stdlib.h>
@@ -38,10 +38,11 @@ namespace {
 
 constexpr int K4_WARPS = 4;     // records per CTA, one per warp
 constexpr int64_t K4_MAX_LANE_BINS = 1024;  // FP32 terms per lane and accumulator
-constexpr int K4_NACC = 36;     // per-record accumulators
+constexpr int K4_NACC = 30;     // per-record accumulators
 constexpr double kTwoPi4 = 6.283185307179586;
 constexpr double kInv2Pi4 = 0.15915494309189535;
 constexpr double kMagic4 = 6755399441055744.0;
+constexpr double kFracMagic4 = 1572864.0;  // 1.5 * 2^20: an FP64 unit of 2^-32
 constexpr float kClampSq4 = (float)(1.0 - (double)0.999999f * (double)0.999999f);
 
 // accumulator layout
@@ -49,23 +50,21 @@ enum {
     A_AMP = 0,     // 8: cotangent of amp' (re, im) x 4
     A_TKX = 8,     // 3: sum theta_bar_j * kxx
     A_TKY = 11,    // 3: sum theta_bar_j * kyy
-    A_WU = 14,     // 9: sum w_bar (x) u   (row-major, R_bar contribution)
-    A_EA = 23,     // 3: sum ea_bar
-    A_P2 = 26,     // 3: prop2 cotangent
-    A_INC = 29,    // 3: incidence-in-frame cotangent
-    A_CU = 32,     // 3: sum of (c-direct coefficient) x u, the u-parallel part of c_bar
-    A_CE = 35,     // 1: sum of the coefficient of 2 c / R^2 in c_bar
+    A_R = 14,      // 9: cotangent of the frame's entries at fixed prop2 and vertices (row-major)
+    A_P2 = 23,     // 3: prop2 cotangent
+    A_C = 26,      // 3: cotangent of the centre at fixed frame, but for
+    A_CE = 29,     // 1: the coefficient of 2 c / R^2 in it
 };
 
-// packed accumulator pairs: (TKX_j, TKY_j) and (WU_i0, WU_i1)
-// and the two Karczewski-Wolf bin sums (sum ee_bar s, sum X) that the
-// record's constants scale into A_P2 at the end
-enum { P_TK = 0, P_WU01 = 3, P_KW = 6, K4_NPAIR = 7 };
+// Inside the bin loop A_AMP holds the amplitude sums in the circular basis, A_P2 + 2 the
+// sum of dd_bar s, and A_EE (not written out) that of ee_bar s; the record's constants
+// scale them into A_AMP and A_P2 at the end.
+enum { A_EE = K4_NACC, K4_NSUM };
 
 // Fields in groups of four floats on 16-byte boundaries, in the order the
 // bin loop reads them, so that the shared-memory reads can be 16 bytes wide.
 struct __align__(16) K4Rec {
-    double kc[3];
+    double kc[3];            // k com / (2 pi)
     double pad0;
     float eps[3], b;
     float R[9], ea[3];
@@ -77,12 +76,14 @@ struct __align__(16) K4Rec {
 };
 static_assert(sizeof(K4Rec) == 208, "K4Rec layout");
 
-// Per-bin input in HBM: the unit bin direction in FP64, 32 B (two 16-byte
+// Per-bin input in HBM: the unit bin direction in FP64 and FP32, 48 B (three 16-byte
 // loads).  The forward-bodge direction (same phi, first row above 1 degree)
 // is read from the same table inside the (rare) bodge branch.
 struct __align__(16) K4Bin {
-    double ux, uy, uz, pad;
+    double ux, uy, uz;
+    float fx, fy, fz, pad[3];
 };
+static_assert(sizeof(K4Bin) == 48, "K4Bin layout");
 
 struct Bin4 {
     double ux, uy, uz;
@@ -91,14 +92,7 @@ struct Bin4 {
     int64_t o;     // bin index
     float2 G[4];   // cotangent of S' (pre-T, common phase removed) for the record's kind,
                    // circular basis of the columns: H+_1, H-_1, H+_2, H-_2
-    float2 Gm[4];  // -i G
 };
-
-__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 
 __device__ __forceinline__ float rcp4(float x) {
     float r;
@@ -198,12 +192,11 @@ __device__ __forceinline__ void dd_grad(float t0, float t1, float t2, float2 &g,
         // E = i e^{ic} sinc(h) = sc n with n = i e^{ic} = (-s, c); dE/dc = i E = sc (i n),
         // i n = (-c, -s); dE/dh = dsc n.  g = (E2 - E1) / D,
         // dg/dlo = (g - (iE1 - H1)/2) / D, dg/dhi = ((iE2 + H2)/2 - g) / D
-        const float2 n1 = make_float2(-s1, c1), n2 = make_float2(-s2, c2);
-        const float2 in1 = make_float2(-c1, -s1), in2 = make_float2(-c2, -s2);
-        const float2 iD2 = bc2(iD);
-        g = mul2(fma2(bc2(sc2), n2, mul2(bc2(-sc1), n1)), iD2);
-        dlo = mul2(fma2(bc2(0.5f * dsc1), n1, fma2(bc2(-0.5f * sc1), in1, g)), iD2);
-        dhi = mul2(fma2(bc2(0.5f * dsc2), n2, fma2(bc2(0.5f * sc2), in2, make_float2(-g.x, -g.y))), iD2);
+        g = make_float2(iD * fmaf(sc1, s1, -sc2 * s2), iD * fmaf(sc2, c2, -sc1 * c1));
+        dlo = make_float2(iD * fmaf(0.5f, fmaf(sc1, c1, -dsc1 * s1), g.x),
+                          iD * fmaf(0.5f, fmaf(dsc1, c1, sc1 * s1), g.y));
+        dhi = make_float2(iD * fmaf(-0.5f, fmaf(dsc2, s2, sc2 * c2), -g.x),
+                          iD * fmaf(0.5f, fmaf(dsc2, c2, -sc2 * s2), -g.y));
     }
     if (D < 0.25f) dd_series(lo, mid, hi, g, dlo, dhi);
 }
@@ -272,22 +265,26 @@ __device__ __forceinline__ Dir4 dir4(const K4Rec &r, float fx, float fy, float f
     return d;
 }
 
-// Back-propagate a cotangent kb of the aperture-frame direction into the
-// frame outer product and ea accumulators; returns the cotangents of
+// Back-propagate a cotangent kb of the aperture-frame direction k = R (u opa2 - e opa)
+// (general bin step) into the frame and centre accumulators; returns the cotangents of
 // a = u.c/R (ab) and b = |c|^2/R^2 (bb) for the caller's c terms.
 __device__ __forceinline__ void dir4_back(const K4Rec &r, const Dir4 &d, const float kb[3], float fx,
-                                          float fy, float fz, float *acc, float2 *accP, float &ab,
+                                          float fy, float fz, float iRf, float *acc, float &ab,
                                           float &bb) {
-    const float2 u01 = make_float2(fx, fy);
+    const float x0 = fmaf(fx, d.opa2, -r.eps[0] * d.opa), x1 = fmaf(fy, d.opa2, -r.eps[1] * d.opa),
+                x2 = fmaf(fz, d.opa2, -r.eps[2] * d.opa);
     float opa2b = 0.0f, opab = 0.0f;
     for (int i = 0; i < 3; i++) {
-        const float wb = kb[i] * d.opa2;
         opa2b = fmaf(kb[i], d.w[i], opa2b);
         opab = fmaf(-kb[i], r.ea[i], opab);
-        accP[P_WU01 + i] = fma2(bc2(wb), u01, accP[P_WU01 + i]);
-        acc[A_WU + 3 * i + 2] = fmaf(wb, fz, acc[A_WU + 3 * i + 2]);
-        acc[A_EA + i] = fmaf(-kb[i], d.opa, acc[A_EA + i]);
+        acc[A_R + 3 * i] = fmaf(kb[i], x0, acc[A_R + 3 * i]);
+        acc[A_R + 3 * i + 1] = fmaf(kb[i], x1, acc[A_R + 3 * i + 1]);
+        acc[A_R + 3 * i + 2] = fmaf(kb[i], x2, acc[A_R + 3 * i + 2]);
     }
+    // e = c / R
+    const float oR = -d.opa * iRf;
+    for (int j = 0; j < 3; j++)
+        acc[A_C + j] = fmaf(oR, fmaf(r.R[6 + j], kb[2], fmaf(r.R[3 + j], kb[1], r.R[j] * kb[0])), acc[A_C + j]);
     ab = opab + opa2b * fmaf(3.0f, d.a, 1.0f);
     bb = -0.5f * opa2b;
 }
@@ -295,161 +292,176 @@ __device__ __forceinline__ void dir4_back(const K4Rec &r, const Dir4 &d, const f
 // Cotangents through the polarisation block and the amplitudes: g_bar, A_bar
 // and B_bar from the bin's cotangent G, and the amplitude sums.
 __device__ __forceinline__ void w_back(const K4Rec &r, const Bin4 &B, float2 g, float A, float Bm,
-                                       float2 *accA, float2 &gb, float &Ab, float &Bb) {
+                                       float *acc, float2 &gb, float &Ab, float &Bb) {
     const float2 *u = reinterpret_cast<const float2 *>(r.amp);
-    // H conj(u) = Re(u) H + Im(u) (-i H)
-    const float2 Sp = fma2(bc2(u[0].x), B.G[0], fma2(bc2(u[0].y), B.Gm[0],
-                           fma2(bc2(u[2].x), B.G[2], mul2(bc2(u[2].y), B.Gm[2]))));
-    const float2 Sn = fma2(bc2(u[1].x), B.G[1], fma2(bc2(u[1].y), B.Gm[1],
-                           fma2(bc2(u[3].x), B.G[3], mul2(bc2(u[3].y), B.Gm[3]))));
-    const float2 Ss = add2(Sp, Sn), Sd = sub2(Sp, Sn);
-    gb = make_float2(fmaf(A, Ss.x, -Bm * Sd.y), fmaf(A, Ss.y, Bm * Sd.x));
-    Ab = fmaf(g.x, Ss.x, g.y * Ss.y);
-    Bb = fmaf(g.y, Sd.x, -g.x * Sd.y);
-    {
-        const float gyB = g.y * Bm, gyA = g.y * A;
-        // conj(g z+) and conj(g z-); H w = Re(w) H - Im(w) (-i H)
-        const float wpr = fmaf(g.x, A, gyB), wpi = fmaf(g.x, Bm, -gyA);
-        const float wnr = fmaf(g.x, A, -gyB), wni = fmaf(-g.x, Bm, -gyA);
-        accA[0] = fma2(bc2(wpr), B.G[0], fma2(bc2(-wpi), B.Gm[0], accA[0]));
-        accA[1] = fma2(bc2(wnr), B.G[1], fma2(bc2(-wni), B.Gm[1], accA[1]));
-        accA[2] = fma2(bc2(wpr), B.G[2], fma2(bc2(-wpi), B.Gm[2], accA[2]));
-        accA[3] = fma2(bc2(wnr), B.G[3], fma2(bc2(-wni), B.Gm[3], accA[3]));
+    // S+- = sum_j H+-_j conj(u+-_j)
+    auto sum2 = [&](int j) {
+        const float2 h = B.G[j], v = u[j], h2 = B.G[j + 2], v2 = u[j + 2];
+        return make_float2(fmaf(h.x, v.x, fmaf(h.y, v.y, fmaf(h2.x, v2.x, h2.y * v2.y))),
+                           fmaf(h.y, v.x, fmaf(-h.x, v.y, fmaf(h2.y, v2.x, -h2.x * v2.y))));
+    };
+    const float2 Sp = sum2(0), Sn = sum2(1);
+    const float sx = Sp.x + Sn.x, sy = Sp.y + Sn.y, dx = Sp.x - Sn.x, dy = Sp.y - Sn.y;
+    gb = make_float2(fmaf(A, sx, -Bm * dy), fmaf(A, sy, Bm * dx));
+    Ab = fmaf(g.x, sx, g.y * sy);
+    Bb = fmaf(g.y, dx, -g.x * dy);
+    // u+-_j_bar += H+-_j w+-, w+- = conj(g z+-)
+    const float gyB = g.y * Bm, gyA = g.y * A;
+    const float2 w[2] = {make_float2(fmaf(g.x, A, gyB), fmaf(g.x, Bm, -gyA)),
+                         make_float2(fmaf(g.x, A, -gyB), fmaf(-g.x, Bm, -gyA))};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 h = B.G[j], v = w[j & 1];
+        acc[A_AMP + 2 * j] = fmaf(v.x, h.x, fmaf(-v.y, h.y, acc[A_AMP + 2 * j]));
+        acc[A_AMP + 2 * j + 1] = fmaf(v.x, h.y, fmaf(v.y, h.x, acc[A_AMP + 2 * j + 1]));
     }
 }
 
-// Cotangents of the phases t_j, the aperture wave vector and the bin direction,
-// given those of kx, ky, kz from the polarisation block (kxb, kyb, kzb).
-__device__ __forceinline__ void phase_back(const K4Rec &r, const Bin4 &B, const Dir4 &d, float2 g,
-                                           float2 dlo, float2 dhi, float2 gb, const float (&t)[3],
-                                           float kxx, float kyy, float kxb, float kyb, float kzb,
-                                           float k, float hkR, float iRf, float *acc, float2 *accP) {
-    // phases: t_j = ph + kxx xa_j + kyy ya_j.  t_bar = Re(conj(g_bar) dg/dt),
-    // assigned by rank (ties broken by index); phb = sum_j t_bar_j = Re(conj(g_bar) i g).
+// Cotangents of the phases t_j = ph + kxx xa_j + kyy ya_j: the vertex and prop2 sums,
+// and the cotangents of kxx, kyy and ph.
+__device__ __forceinline__ void phase_back(const K4Rec &r, float2 g, float2 dlo, float2 dhi, float2 gb,
+                                           const float (&t)[3], float kxx, float kyy, float *acc,
+                                           float &kxxb, float &kyyb, float &phb) {
+    // t_bar = Re(conj(g_bar) dg/dt), assigned by rank (g is symmetric, so equal phases
+    // have equal derivatives); phb = sum_j t_bar_j = Re(conj(g_bar) i g).
     const float tlo = fmaf(gb.x, dlo.x, gb.y * dlo.y), thi = fmaf(gb.x, dhi.x, gb.y * dhi.y);
-    const float phb = fmaf(gb.y, g.x, -gb.x * g.y);
+    phb = fmaf(gb.y, g.x, -gb.x * g.y);
     const float tmid = phb - tlo - thi;
-    // rank 0 (lowest) / 2 (highest) of each t_j, ties broken by index
-    const bool c01 = t[1] < t[0], c02 = t[2] < t[0], c12 = t[2] < t[1];
-    const bool is_lo[3] = {!c01 && !c02, c01 && !c12, c02 && c12};
-    const bool is_hi[3] = {c01 && c02, !c01 && c12, !c02 && !c12};
-    float kxxb = 0.0f, kyyb = 0.0f;
-    const float2 kk2 = make_float2(kxx, kyy);
+    const float lo = fminf(fminf(t[0], t[1]), t[2]), hi = fmaxf(fmaxf(t[0], t[1]), t[2]);
+    kxxb = 0.0f;
+    kyyb = 0.0f;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-        const float tb = is_lo[j] ? tlo : (is_hi[j] ? thi : tmid);
+        const float tb = t[j] == lo ? tlo : (t[j] == hi ? thi : tmid);
         kxxb = fmaf(tb, r.xa[j], kxxb);
         kyyb = fmaf(tb, r.ya[j], kyyb);
-        accP[P_TK + j] = fma2(bc2(tb), kk2, accP[P_TK + j]);
+        acc[A_TKX + j] = fmaf(tb, kxx, acc[A_TKX + j]);
+        acc[A_TKY + j] = fmaf(tb, kyy, acc[A_TKY + j]);
     }
-    // kxx = k p2x - k kx ; kyy = k p2y - k ky
-    kxb = fmaf(-k, kxxb, kxb);
-    kyb = fmaf(-k, kyyb, kyb);
-    acc[A_P2 + 0] += kxxb;  // times k after the loop
+    acc[A_P2 + 0] += kxxb;  // kxx = k p2x - k kx ; times k after the loop
     acc[A_P2 + 1] += kyyb;
-    const float kb3[3] = {kxb, kyb, kzb};
-    float ab, bb;
-    dir4_back(r, d, kb3, B.fx, B.fy, B.fz, acc, accP, ab, bb);
-    // ph = hkR (b - a^2)(1 + a) - rf with rf = k u.c (mod 2 pi), a = u.c/R, b = |c|^2/R^2:
-    // c_bar = (ab + phb dph/da) u / R - phb k u + (bb + phb dph/db) 2 c / R^2
-    const float dpa = hkR * fmaf(-2.0f * d.a, d.opa, fmaf(-d.a, d.a, r.b));
-    const float dpb = hkR * d.opa;
-    const float cu = fmaf(fmaf(phb, dpa, ab), iRf, -k * phb);
-    acc[A_CU + 0] = fmaf(cu, B.fx, acc[A_CU + 0]);
-    acc[A_CU + 1] = fmaf(cu, B.fy, acc[A_CU + 1]);
-    acc[A_CU + 2] = fmaf(cu, B.fz, acc[A_CU + 2]);
-    acc[A_CE] += fmaf(phb, dpb, bb);
 }
 
-// The bin step outside the clamps and the forward bodge (a bin away from the
-// poles, |ky| <= 0.999999 and kx^2 + kz^2 above the floor): the general step
-// below with kyc = ky, tt = kx^2 + kz^2 and q = k, its branches left out.
-__device__ __forceinline__ void k4_main(const K4Rec &r, const Bin4 &B, const Dir4 &d, float kx,
-                                        float ky, float kz, float kxx, float kyy,
-                                        const float (&t)[3], float tt, float k, float hkR,
-                                        float iRf, float *acc, float2 *accA, float2 *accP) {
+// Centre cotangent of the far-field phase ph = hkR (b - a^2)(1 + a) - k u.c and of
+// a = u.c/R, b = |c|^2/R^2: (ab + phb dph/da) u / R - phb k u + (bb + phb dph/db) 2 c / R^2.
+// Returns the coefficient of u.
+__device__ __forceinline__ float centre_back(float a, float b, float phb, float ab, float bb, float k,
+                                             float hkR, float iRf, float *acc) {
+    const float opa = 1.0f + a;
+    const float dpa = hkR * fmaf(-2.0f * a, opa, fmaf(-a, a, b));
+    acc[A_CE] += fmaf(phb, hkR * opa, bb);
+    return fmaf(fmaf(phb, dpa, ab), iRf, -k * phb);
+}
+
+// The bin step outside the clamps and the forward bodge (a bin away from the poles,
+// |ky| <= 0.999999 and kx^2 + kz^2 above the floor).  With (a, b, c) = u opa2 - e opa the
+// unit direction from the facet in the lab frame, k = R (a, b, c), and the scattering
+// plane's normal h = inc x k = (b, -a, 0), the polarisation block is
+//   A = sc (P D + Q E),  B = sc (P E - Q D),  sc = 1 / (|h| t),  t = kx^2 + kz^2,
+//   P = y . h = y0 b - y1 a,  Q = y2 |h|^2 - c (y0 a + y1 b)  (y the frame's second axis),
+//   D = kw1 t - hicf kz,  E = -hicf kx ky
+// (|k| = 1 and Ky = 0 up to rounding, as in the forward kernel).  Its backward needs no
+// h in the aperture frame, and the cotangents of the frame's entries and of the
+// centre are formed directly in the lab frame.
+__device__ __forceinline__ void k4_main(const K4Rec &r, const Bin4 &B, float al, float opa, float a, float b,
+                                        float c, float kx, float ky, float kz, float u, float ph, float tt,
+                                        float k, float hkR, float iRf, float *acc) {
+    const float kxx = fmaf(-k, kx, r.kp[0]), kyy = fmaf(-k, ky, r.kp[1]);
+    float t[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) t[j] = fmaf(kyy, r.ya[j], fmaf(kxx, r.xa[j], ph));
     float2 g, dlo, dhi;
     dd_grad_main(t[0], t[1], t[2], g, dlo, dhi);
-    const float rs = rsqrt4(tt), s = tt * rs;
-    const float e = rs * r.hicf, kxky = kx * ky;
-    const float dd = fmaf(r.kw1, s, -kz * e);
-    const float ee = fmaf(r.kw2, s, -kxky * e);
-    const float hr[3] = {fmaf(r.inc[1], kz, -r.inc[2] * ky), fmaf(r.inc[2], kx, -r.inc[0] * kz),
-                         fmaf(r.inc[0], ky, -r.inc[1] * kx)};
-    const float hn = rsqrt4(fmaf(hr[2], hr[2], fmaf(hr[1], hr[1], hr[0] * hr[0])));
-    // hr is normal to k and |k| = 1 to third order in |c|/R, so the general
-    // p = hn (hr1 s - (ky/s) hr . (kx, 0, kz)) is hn hr1 / s, the forward kernel's
-    // form; rr = hn (hr2 kx - hr0 kz) / s.
-    const float f = hn * rs;
-    const float R0 = fmaf(hr[2], kx, -hr[0] * kz);
-    const float pp = f * hr[1], rr = f * R0;
-    const float A = fmaf(pp, dd, rr * ee), Bm = fmaf(pp, ee, -rr * dd);
+    const float y0 = r.R[3], y1 = r.R[4], y2 = r.R[5];
+    const float hn2 = fmaf(a, a, b * b);
+    const float P = fmaf(y0, b, -y1 * a), Q = fmaf(y2, hn2, -c * u);
+    const float D = fmaf(r.kw1, tt, -r.hicf * kz), E = -r.hicf * (kx * ky);
+    const float ht = hn2 * tt;
+    const float sc = rsqrt4(ht * tt), rht = rcp4(ht);
+    const float A = sc * fmaf(P, D, Q * E), Bm = sc * fmaf(P, E, -Q * D);
     float2 gb;
     float Ab, Bb;
-    w_back(r, B, g, A, Bm, accA, gb, Ab, Bb);
-    const float ppb = fmaf(Ab, dd, Bb * ee), rrb = fmaf(Ab, ee, -Bb * dd);
-    const float ddb = fmaf(Ab, pp, -Bb * rr), eeb = fmaf(Ab, rr, Bb * pp);
-    // f = hn rs: f_bar = pp_bar hr1 + rr_bar R0; hn_bar = f_bar rs, rs_bar = f_bar hn
-    const float fb = fmaf(ppb, hr[1], rrb * R0);
-    const float R0b = rrb * f;
-    const float hn3 = -(fb * rs) * (hn * hn * hn);  // d hn / d hr_i = -hn^3 hr_i
-    const float hrb[3] = {fmaf(-R0b, kz, hn3 * hr[0]), fmaf(ppb, f, hn3 * hr[1]),
-                          fmaf(R0b, kx, hn3 * hr[2])};
-    float kxb = R0b * hr[2];
-    float kzb = -R0b * hr[0];
-    float kyb = 0.0f;
-    const float sbm = -(fb * hn) * (rs * rs);  // rs = 1/s
-    // h = inc x k
-    kxb += hrb[1] * r.inc[2] - hrb[2] * r.inc[1];
-    kyb += hrb[2] * r.inc[0] - hrb[0] * r.inc[2];
-    kzb += hrb[0] * r.inc[1] - hrb[1] * r.inc[0];
-    acc[A_INC + 0] += ky * hrb[2] - kz * hrb[1];
-    acc[A_INC + 1] += kz * hrb[0] - kx * hrb[2];
-    acc[A_INC + 2] += kx * hrb[1] - ky * hrb[0];
-    // Karczewski-Wolf dd, ee (see k4_eval)
-    const float dde = ddb * e, eee = eeb * e;
-    kxb = fmaf(-eee, ky, kxb);
-    kyb = fmaf(-eee, kx, kyb);
-    kzb -= dde;
-    const float X = fmaf(dde, kz, eee * kxky);
-    const float sb = sbm + fmaf(ddb, r.kw1, fmaf(eeb, r.kw2, rs * X));
-    acc[A_P2 + 2] = fmaf(ddb, s, acc[A_P2 + 2]);
-    accP[P_KW].x = fmaf(eeb, s, accP[P_KW].x);
-    accP[P_KW].y += X;
-    const float ttb = 0.5f * sb * rs;  // s = sqrt(tt)
-    kxb = fmaf(2.0f * kx, ttb, kxb);
-    kzb = fmaf(2.0f * kz, ttb, kzb);
-    phase_back(r, B, d, g, dlo, dhi, gb, t, kxx, kyy, kxb, kyb, kzb, k, hkR, iRf, acc, accP);
+    w_back(r, B, g, A, Bm, acc, gb, Ab, Bb);
+    const float Wr = fmaf(Ab, A, Bb * Bm) * rht;  // sc sc_bar / (|h|^2 t)
+    const float Mb = Ab * sc, Nb = Bb * sc;
+    const float Pb = fmaf(Mb, D, Nb * E), Qb = fmaf(Mb, E, -Nb * D);
+    const float Db = fmaf(Mb, P, -Nb * Q), Eb = fmaf(Mb, Q, Nb * P);
+    // sc = |h|^-1 t^-1: the cotangents of |h|^2 (doubled) and of t
+    const float h2 = fmaf(-Wr, tt, 2.0f * Qb * y2);
+    const float t2 = 2.0f * fmaf(-Wr, hn2, Db * r.kw1);
+    acc[A_P2 + 2] = fmaf(Db, tt, acc[A_P2 + 2]);
+    acc[A_EE] = fmaf(Eb, tt, acc[A_EE]);
+    const float hD = r.hicf * Db, hE = r.hicf * Eb;
+    float kxxb, kyyb, phb;
+    phase_back(r, g, dlo, dhi, gb, t, kxx, kyy, acc, kxxb, kyyb, phb);
+    const float kxb = fmaf(-k, kxxb, fmaf(t2, kx, -hE * ky));
+    const float kyb = fmaf(-k, kyyb, -hE * kx);
+    const float kzb = fmaf(t2, kz, -hD);
+    // frame: k = R (a, b, c), and the second axis in P, Q and u = y0 a + y1 b
+    const float ub = -Qb * c, e1 = kyb + ub;
+    acc[A_R + 0] = fmaf(kxb, a, acc[A_R + 0]);
+    acc[A_R + 1] = fmaf(kxb, b, acc[A_R + 1]);
+    acc[A_R + 3] = fmaf(e1, a, fmaf(Pb, b, acc[A_R + 3]));
+    acc[A_R + 4] = fmaf(e1, b, fmaf(-Pb, a, acc[A_R + 4]));
+    acc[A_R + 6] = fmaf(kzb, a, acc[A_R + 6]);
+    acc[A_R + 7] = fmaf(kzb, b, acc[A_R + 7]);
+    acc[A_R + 2] = fmaf(kxb, c, acc[A_R + 2]);
+    acc[A_R + 5] = fmaf(kyb, c, fmaf(Qb, hn2, acc[A_R + 5]));
+    acc[A_R + 8] = fmaf(kzb, c, acc[A_R + 8]);
+    // lab direction
+    const float da = fmaf(h2, a, fmaf(-y1, Pb, fmaf(y0, e1, fmaf(r.R[0], kxb, r.R[6] * kzb))));
+    const float db = fmaf(h2, b, fmaf(y0, Pb, fmaf(y1, e1, fmaf(r.R[1], kxb, r.R[7] * kzb))));
+    const float dc = fmaf(-Qb, u, fmaf(y2, kyb, fmaf(r.R[2], kxb, r.R[8] * kzb)));
+    // (a, b, c) = u opa2 - e opa: to first order in e, al_bar = (a, b, c) . (da, db, dc)
+    // and b_bar = -al_bar / 2 (both enter the centre's cotangent divided by R)
+    const float alb = fmaf(dc, c, fmaf(db, b, da * a));
+    const float cu = centre_back(al, r.b, phb, alb, -0.5f * alb, k, hkR, iRf, acc);
+    const float oR = -opa * iRf;
+    acc[A_C + 0] = fmaf(oR, da, fmaf(cu, B.fx, acc[A_C + 0]));
+    acc[A_C + 1] = fmaf(oR, db, fmaf(cu, B.fy, acc[A_C + 1]));
+    acc[A_C + 2] = fmaf(oR, dc, fmaf(cu, B.fz, acc[A_C + 2]));
 }
 
 // Cotangent contributions of one (record, bin).
-template <bool FAST>
+template <bool FAST, bool WIDE>
 __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, float hkR, float iRf,
                                         float cosfov, const float *p0, const K4Bin *__restrict__ bins,
-                                        int64_t nphi, int64_t theta_i, float *acc, float2 *accA,
-                                        float2 *accP) {
-    // forward
-    const double ka = fma(B.uz, r.kc[2], fma(B.uy, r.kc[1], B.ux * r.kc[0]));
-    const double nq = fma(ka, kInv2Pi4, kMagic4) - kMagic4;
-    const float rf = (float)fma(-nq, kTwoPi4, ka);
-    const Dir4 d = dir4(r, B.fx, B.fy, B.fz);
-    if (FAST) {
-        const float dx = fmaf(B.fx, d.opa, -r.eps[0]), dy = fmaf(B.fy, d.opa, -r.eps[1]),
-                    dz = fmaf(B.fz, d.opa, -r.eps[2]);
-        if (fmaf(dz, p0[2], fmaf(dy, p0[1], dx * p0[0])) < cosfov) return;
+                                        int64_t nphi, int64_t theta_i, float *acc) {
+    // forward: k u.c modulo 2 pi as a fixed-point fraction of a turn (2^-32 units), the low
+    // word of the FP64 sum added to 1.5 * 2^20; beyond 2^18 turns (WIDE) the nearest
+    // integer is taken off first
+    float fr;
+    if (!WIDE) {
+        fr = (float)__double2loint(fma(B.uz, r.kc[2], fma(B.uy, r.kc[1], fma(B.ux, r.kc[0], kFracMagic4))));
+    } else {
+        const double ka = fma(B.uz, r.kc[2], fma(B.uy, r.kc[1], B.ux * r.kc[0]));
+        fr = (float)((ka - ((ka + kMagic4) - kMagic4)) * 4294967296.0);
     }
-    const float ph = fmaf(hkR * fmaf(-d.a, d.a, r.b), d.opa, -rf);
+    const float al = fmaf(B.fz, r.eps[2], fmaf(B.fy, r.eps[1], B.fx * r.eps[0]));
+    const float opa = 1.0f + al;
+    const float opa2 = fmaf(al, fmaf(1.5f, al, 1.0f), fmaf(-0.5f, r.b, 1.0f));
+    const float a = fmaf(B.fx, opa2, -r.eps[0] * opa), b = fmaf(B.fy, opa2, -r.eps[1] * opa),
+                c = fmaf(B.fz, opa2, -r.eps[2] * opa);
+    if (FAST) {
+        if (fmaf(c, p0[2], fmaf(b, p0[1], a * p0[0])) < cosfov) return;
+    }
+    const float ph = fmaf(hkR * fmaf(-al, al, r.b), opa, fr * (float)(-kTwoPi4 / 4294967296.0));
+    {
+        const float u = fmaf(r.R[4], b, r.R[3] * a);
+        const float mx = fmaf(r.R[2], c, fmaf(r.R[1], b, r.R[0] * a)), my = fmaf(r.R[5], c, u),
+                    mz = fmaf(r.R[8], c, fmaf(r.R[7], b, r.R[6] * a));
+        const float tr = fmaf(mx, mx, mz * mz);
+        if (!B.pole && tr > kClampSq4) {
+            k4_main(r, B, al, opa, a, b, c, mx, my, mz, u, ph, tr, k, hkR, iRf, acc);
+            return;
+        }
+    }
+    // near a pole or on the clamp: the general step, in the aperture frame
+    const Dir4 d = dir4(r, B.fx, B.fy, B.fz);
     const float kx = d.k[0], ky = d.k[1], kz = d.k[2];
     const float kxx = fmaf(-k, kx, r.kp[0]), kyy = fmaf(-k, ky, r.kp[1]);
     float t[3];
     for (int j = 0; j < 3; j++) t[j] = fmaf(kyy, r.ya[j], fmaf(kxx, r.xa[j], ph));
-    {
-        const float tr = fmaf(kx, kx, kz * kz);
-        if (!B.pole && tr > kClampSq4 && fabsf(ky) <= 0.999999f) {
-            k4_main(r, B, d, kx, ky, kz, kxx, kyy, t, tr, k, hkR, iRf, acc, accA, accP);
-            return;
-        }
-    }
     float2 g, dlo, dhi;
     dd_grad(t[0], t[1], t[2], g, dlo, dhi);
     const bool yclamp = !(fabsf(ky) <= 0.999999f);
@@ -476,9 +488,9 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
     float hx = 0.0f, hy = 0.0f, hz = 0.0f;
     if (bodge) {
         const K4Bin hb = bins[B.o % nphi + nphi * theta_i];
-        hx = (float)hb.ux;
-        hy = (float)hb.uy;
-        hz = (float)hb.uz;
+        hx = hb.fx;
+        hy = hb.fy;
+        hz = hb.fz;
         dh = dir4(r, hx, hy, hz);
         q[0] = dh.k[0];
         q[1] = dh.k[1];
@@ -516,7 +528,7 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
     //   u+-_j_bar = H+-_j conj(g z+-)
     float2 gb;
     float Ab, Bb;
-    w_back(r, B, g, A, Bm, accA, gb, Ab, Bb);
+    w_back(r, B, g, A, Bm, acc, gb, Ab, Bb);
     // A = pp dd + rr ee, B = pp ee - rr dd
     const float ppb = fmaf(Ab, dd, Bb * ee), rrb = fmaf(Ab, ee, -Bb * dd);
     const float ddb = fmaf(Ab, pp, -Bb * rr), eeb = fmaf(Ab, rr, Bb * pp);
@@ -564,16 +576,17 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
     qb[0] = hrb[1] * r.inc[2] - hrb[2] * r.inc[1];
     qb[1] = hrb[2] * r.inc[0] - hrb[0] * r.inc[2];
     qb[2] = hrb[0] * r.inc[1] - hrb[1] * r.inc[0];
-    acc[A_INC + 0] += q[1] * hrb[2] - q[2] * hrb[1];
-    acc[A_INC + 1] += q[2] * hrb[0] - q[0] * hrb[2];
-    acc[A_INC + 2] += q[0] * hrb[1] - q[1] * hrb[0];
+    // inc = -R z: its cotangent into the frame's third column
+    acc[A_R + 2] -= q[1] * hrb[2] - q[2] * hrb[1];
+    acc[A_R + 5] -= q[2] * hrb[0] - q[0] * hrb[2];
+    acc[A_R + 8] -= q[0] * hrb[1] - q[1] * hrb[0];
     if (bodge) {
         float abh, bbh;
-        dir4_back(r, dh, qb, hx, hy, hz, acc, accP, abh, bbh);
+        dir4_back(r, dh, qb, hx, hy, hz, iRf, acc, abh, bbh);
         const float ch = abh * iRf;
-        acc[A_CU + 0] = fmaf(ch, hx, acc[A_CU + 0]);
-        acc[A_CU + 1] = fmaf(ch, hy, acc[A_CU + 1]);
-        acc[A_CU + 2] = fmaf(ch, hz, acc[A_CU + 2]);
+        acc[A_C + 0] = fmaf(ch, hx, acc[A_C + 0]);
+        acc[A_C + 1] = fmaf(ch, hy, acc[A_C + 1]);
+        acc[A_C + 2] = fmaf(ch, hz, acc[A_C + 2]);
         acc[A_CE] += bbh;
     } else {
         kxb += qb[0];
@@ -582,10 +595,9 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
     }
     // Karczewski-Wolf dd, ee as above.  With X = (dd_bar kz + ee_bar kx ky) e:
     //   s_bar += kw1 dd_bar + kw2 ee_bar + X / s
-    //   p2_bar: z -cf/2 dd_bar s, x Ky cf/2 ee_bar s,
-    //           y Kx cf/2 ee_bar s + Ky cf^2 (kw1 dd_bar s + kw2 ee_bar s + X)
-    // (cf = 1/sqrt(1 - Ky^2)); the bin sums of dd_bar s, ee_bar s and X are
-    // scaled by the record's constants after the loop.
+    //   p2_bar: z -cf/2 dd_bar s, x Ky cf/2 ee_bar s, y Kx cf/2 ee_bar s
+    // (cf = 1/sqrt(1 - Ky^2); y's further terms carry Ky, zero up to rounding); the bin
+    // sums of dd_bar s and ee_bar s are scaled by the record's constants after the loop.
     const float dde = ddb * e, eee = eeb * e;
     kxb = fmaf(-eee, kyc, kxb);
     kycb = fmaf(-eee, kx, kycb);
@@ -593,24 +605,38 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
     const float X = fmaf(dde, kz, eee * kxkyc);
     const float sb = sbm + fmaf(ddb, r.kw1, fmaf(eeb, r.kw2, rs * X));
     acc[A_P2 + 2] = fmaf(ddb, s, acc[A_P2 + 2]);
-    accP[P_KW].x = fmaf(eeb, s, accP[P_KW].x);
-    accP[P_KW].y += X;
+    acc[A_EE] = fmaf(eeb, s, acc[A_EE]);
     if (!floored) {
         const float ttb = 0.5f * sb * rs;  // s = sqrt(tt)
         kxb = fmaf(2.0f * kx, ttb, kxb);
         kzb = fmaf(2.0f * kz, ttb, kzb);
     }
     float kyb = yclamp ? 0.0f : kycb;
-    phase_back(r, B, d, g, dlo, dhi, gb, t, kxx, kyy, kxb, kyb, kzb, k, hkR, iRf, acc, accP);
+    float kxxb, kyyb, phb, ab, bb;
+    phase_back(r, g, dlo, dhi, gb, t, kxx, kyy, acc, kxxb, kyyb, phb);
+    const float kb3[3] = {fmaf(-k, kxxb, kxb), fmaf(-k, kyyb, kyb), kzb};
+    dir4_back(r, d, kb3, B.fx, B.fy, B.fz, iRf, acc, ab, bb);
+    const float cu = centre_back(al, r.b, phb, ab, bb, k, hkR, iRf, acc);
+    acc[A_C + 0] = fmaf(cu, B.fx, acc[A_C + 0]);
+    acc[A_C + 1] = fmaf(cu, B.fy, acc[A_C + 1]);
+    acc[A_C + 2] = fmaf(cu, B.fz, acc[A_C + 2]);
 }
 
 // One warp per record, K4_WARPS records per CTA; blockIdx.y selects a range
-// of bins.  Each lane walks the range with stride 32 and keeps the 36 sums of
+// of bins.  Each lane walks the range with stride 32 and keeps the 30 sums of
 // its record in registers (FP32, at most K4_MAX_LANE_BINS terms), so the warp
-// reduction and the FP64 atomic into out[record][36] happen once per
+// reduction and the FP64 atomic into out[record][30] happen once per
 // (record, range).  The warps of a CTA walk the same bins, which the L1 serves.
-template <bool FAST, int MINB>
-__global__ void __launch_bounds__(K4_WARPS * 32, MINB) k4_adjoint_kernel(
+//
+// Bound: issue (78 % of the slots; 366 instructions a facet and bin, 272 of them on the
+// FMA pipe).  In the aperture frame, with the sums of the incidence direction and of the
+// centre's frame components kept apart (36 sums, 168 registers, three CTAs per SM), a
+// plate of 30,968 triangles x 16,290 bins took 7.32 ms; in the lab frame 6.92 (30 sums,
+// 128 registers, four CTAs), with scalar instead of packed FP32x2 operations, whose
+// broadcast operands cost a move each, 6.63, and with the phase's reduction in fixed
+// point 6.59.
+template <bool FAST, bool WIDE>
+__global__ void __launch_bounds__(K4_WARPS * 32, 4) k4_adjoint_kernel(
     const K4Rec *__restrict__ recs, const int *__restrict__ kinds, const float *__restrict__ fovdat,
     int64_t nrec, const K4Bin *__restrict__ bins, const float4 *__restrict__ gbin, int64_t nb,
     int64_t nphi, int64_t theta_i, int64_t chunk, float k, float hkR, float iRf, float pole_cos,
@@ -635,26 +661,22 @@ __global__ void __launch_bounds__(K4_WARPS * 32, MINB) k4_adjoint_kernel(
         p0[2] = fovdat[4 * rec + 2];
         cosfov = fovdat[4 * rec + 3];
     }
-    float acc[K4_NACC];
-    float2 accA[4], accP[K4_NPAIR];
+    float acc[K4_NSUM];
 #pragma unroll
-    for (int q = 0; q < K4_NACC; q++) acc[q] = 0.0f;
-#pragma unroll
-    for (int q = 0; q < K4_NPAIR; q++) accP[q] = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int q = 0; q < 4; q++) accA[q] = make_float2(0.0f, 0.0f);
+    for (int q = 0; q < K4_NSUM; q++) acc[q] = 0.0f;
     const int64_t o0 = (int64_t)blockIdx.y * chunk, o1 = min(nb, o0 + chunk);
     for (int64_t o = o0 + lane; o < o1; o += 32) {
         Bin4 B;
         const double2 *pb = reinterpret_cast<const double2 *>(bins + o);
-        const double2 q0 = pb[0], q1 = pb[1];
+        const double2 q0 = pb[0];
+        const int4 q1 = reinterpret_cast<const int4 *>(pb)[1];  // uz, fx, fy
         B.ux = q0.x;
         B.uy = q0.y;
-        B.uz = q1.x;
-        B.fx = (float)B.ux;
-        B.fy = (float)B.uy;
-        B.fz = (float)B.uz;
-        B.pole = !(fabs(B.uz) < (double)pole_cos);
+        B.uz = __hiloint2double(q1.y, q1.x);
+        B.fx = __int_as_float(q1.z);
+        B.fy = __int_as_float(q1.w);
+        B.fz = bins[o].fz;
+        B.pole = !(fabsf(B.fz) < pole_cos);
         B.o = o;
         const float4 *pg = G + 2 * o;
         const float4 g0 = pg[0], g1 = pg[1];
@@ -662,35 +684,25 @@ __global__ void __launch_bounds__(K4_WARPS * 32, MINB) k4_adjoint_kernel(
         B.G[1] = make_float2(g0.z, g0.w);
         B.G[2] = make_float2(g1.x, g1.y);
         B.G[3] = make_float2(g1.z, g1.w);
-#pragma unroll
-        for (int c = 0; c < 4; c++) B.Gm[c] = make_float2(B.G[c].y, -B.G[c].x);
-        k4_eval<FAST>(r, B, k, hkR, iRf, cosfov, p0, bins, nphi, theta_i, acc, accA, accP);
+        k4_eval<FAST, WIDE>(r, B, k, hkR, iRf, cosfov, p0, bins, nphi, theta_i, acc);
     }
     // amplitude sums back from the circular basis: a1j_bar = u+_j_bar + u-_j_bar,
     // a2j_bar = i (u-_j_bar - u+_j_bar)
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        const float2 up = accA[2 * j], un = accA[2 * j + 1];
-        acc[A_AMP + 4 * j] = up.x + un.x;
-        acc[A_AMP + 4 * j + 1] = up.y + un.y;
-        acc[A_AMP + 4 * j + 2] = up.y - un.y;
-        acc[A_AMP + 4 * j + 3] = un.x - up.x;
-    }
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-        acc[A_TKX + j] = accP[P_TK + j].x;
-        acc[A_TKY + j] = accP[P_TK + j].y;
-        acc[A_WU + 3 * j] += accP[P_WU01 + j].x;
-        acc[A_WU + 3 * j + 1] += accP[P_WU01 + j].y;
+        float *v = acc + A_AMP + 4 * j;
+        const float2 up = make_float2(v[0], v[1]), un = make_float2(v[2], v[3]);
+        v[0] = up.x + un.x;
+        v[1] = up.y + un.y;
+        v[2] = up.y - un.y;
+        v[3] = un.x - up.x;
     }
     {
-        // A_P2 held (sum kxx_bar, sum kyy_bar, sum dd_bar s) and P_KW (sum ee_bar s, sum X)
+        // A_P2 held sum kxx_bar, sum kyy_bar and sum dd_bar s
         const float cf = r.cf, Kx = r.p2[0], Ky = r.p2[1];
-        const float q1 = acc[A_P2 + 2], q2 = accP[P_KW].x, q3 = accP[P_KW].y;
-        acc[A_P2 + 0] = fmaf(k, acc[A_P2 + 0], 0.5f * Ky * cf * q2);
-        acc[A_P2 + 1] = fmaf(k, acc[A_P2 + 1],
-                             fmaf(0.5f * Kx * cf, q2, Ky * cf * cf * fmaf(r.kw1, q1, fmaf(r.kw2, q2, q3))));
-        acc[A_P2 + 2] = -0.5f * cf * q1;
+        acc[A_P2 + 0] = fmaf(k, acc[A_P2 + 0], 0.5f * Ky * cf * acc[A_EE]);
+        acc[A_P2 + 1] = fmaf(k, acc[A_P2 + 1], 0.5f * Kx * cf * acc[A_EE]);
+        acc[A_P2 + 2] *= -0.5f * cf;
     }
 #pragma unroll
     for (int q = 0; q < K4_NACC; q++) {
@@ -717,7 +729,10 @@ __global__ void k4_prep_kernel(const double *__restrict__ gafb, const double *__
     bn.ux = X * ir;
     bn.uy = Y * ir;
     bn.uz = Zc * ir;
-    bn.pad = 0.0;
+    bn.fx = (float)bn.ux;
+    bn.fy = (float)bn.uy;
+    bn.fz = (float)bn.uz;
+    bn.pad[0] = bn.pad[1] = bn.pad[2] = 0.0f;
     bins[o] = bn;
     double sK, cK;
     sincos(k * rho, &sK, &cK);
@@ -795,7 +810,7 @@ __global__ void k4_setup_kernel(const pbt_outbeam *__restrict__ beam, int64_t nb
         const double As = 0.5 * ((xa[1] - xa[0]) * (ya[2] - ya[0]) - (xa[2] - xa[0]) * (ya[1] - ya[0]));
         const double cpre = 2.0 * As / lambda * fr.sign;
         for (int c = 0; c < 3; c++) {
-            r.kc[c] = k * fr.com[c];
+            r.kc[c] = k * fr.com[c] * kInv2Pi4;
             r.eps[c] = (float)(fr.com[c] / Rf);
             r.ea[c] = (float)(ea[c] / Rf);
             r.p2[c] = (float)fr.prop2[c];
@@ -843,7 +858,7 @@ __global__ void k4_setup_kernel(const pbt_outbeam *__restrict__ beam, int64_t nb
         fovd[4 * q + 3] = (float)cos(fov);
     }
 
-// Thread per record: the record's 36 sums mapped through the frame
+// Thread per record: the record's 30 sums mapped through the frame
 // construction (z = -n, x = unit(p - (p.n) n), y = z x x, n = unit(e0 x e1),
 // c = mean(v)) to its three vertices (added with FP64 atomics) and to its
 // amplitude (gamp: 8 doubles, the outbeam's ampl order).
@@ -855,7 +870,6 @@ __global__ void k4_map_kernel(const double *__restrict__ acc, const Host4 *__res
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nrec) return;
     const double Rf = kFarR;
-    const double inc[3] = {0, 0, -1};
         const double *A = &acc[q * K4_NACC];
         const Host4 &h = H[q];
         const pbt_outbeam &ob = q < nbeam ? beam[q] : ext[q - nbeam];
@@ -889,8 +903,7 @@ __global__ void k4_map_kernel(const double *__restrict__ acc, const Host4 *__res
         double Rb[3][3];
         for (int a = 0; a < 3; a++)
             for (int b = 0; b < 3; b++)
-                Rb[a][b] = A[A_WU + 3 * a + b] + A[A_EA + a] * h.c[b] / Rf +
-                           A[A_INC + a] * inc[b] + A[A_P2 + a] * h.p[b];
+                Rb[a][b] = A[A_R + 3 * a + b] + A[A_P2 + a] * h.p[b];
         double eb[3][3];
         for (int j = 0; j < 3; j++)
             for (int b = 0; b < 3; b++) {
@@ -898,11 +911,8 @@ __global__ void k4_map_kernel(const double *__restrict__ acc, const Host4 *__res
                 Rb[1][b] += yab[j] * h.e[j][b];
                 eb[j][b] = xab[j] * h.R[0][b] + yab[j] * h.R[1][b];
             }
-        // c_bar = direct + R^T ea_bar / Rf
         double cb[3];
-        for (int b = 0; b < 3; b++)
-            cb[b] = A[A_CU + b] + A[A_CE] * 2.0 * h.c[b] / (Rf * Rf) +
-                    (h.R[0][b] * A[A_EA + 0] + h.R[1][b] * A[A_EA + 1] + h.R[2][b] * A[A_EA + 2]) / Rf;
+        for (int b = 0; b < 3; b++) cb[b] = A[A_C + b] + A[A_CE] * 2.0 * h.c[b] / (Rf * Rf);
         // frame: z = -n, x = unit(p - (p.n) n), y = z x x
         double n[3] = {-h.R[2][0], -h.R[2][1], -h.R[2][2]}, xh[3] = {h.R[0][0], h.R[0][1], h.R[0][2]};
         double zb[3] = {Rb[2][0], Rb[2][1], Rb[2][2]}, xb[3] = {Rb[0][0], Rb[0][1], Rb[0][2]},
@@ -1028,14 +1038,8 @@ int k4_adjoint(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam, int64_t n
         vmax2 = std::max(vmax2, x * x + y * y + z * z);
     }
     const float pole_cos = (float)(0.999 - 2.0 * sqrt(vmax2) / Rf - 1e-5);
+    const bool wide = !(k * sqrt(vmax2) * kInv2Pi4 < 262144.0);  // see k4_eval
     timing_begin(ctx, st);
-    // Minimum CTAs per SM for the register budget: 3 (168 registers, a few
-    // bytes of spill) by default; PBT_K4_MINB=1|2|4 selects another build.
-    static const int minb = [] {
-        const char *e = getenv("PBT_K4_MINB");
-        const int v = e ? atoi(e) : 3;
-        return (v == 1 || v == 2 || v == 4) ? v : 3;
-    }();
     if (nrec > 0) {
         auto launch = [&](auto kern) {
             kern<<<grid, K4_WARPS * 32, 0, st>>>(
@@ -1044,17 +1048,10 @@ int k4_adjoint(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam, int64_t n
                 g.theta_i, chunk, (float)k,
                 (float)(0.5 * k * Rf), (float)(1.0 / Rf), pole_cos, (double *)(base + o_out));
         };
-        if (fast_diff) {
-            if (minb == 1) launch(k4_adjoint_kernel<true, 1>);
-            else if (minb == 2) launch(k4_adjoint_kernel<true, 2>);
-            else if (minb == 4) launch(k4_adjoint_kernel<true, 4>);
-            else launch(k4_adjoint_kernel<true, 3>);
-        } else {
-            if (minb == 1) launch(k4_adjoint_kernel<false, 1>);
-            else if (minb == 2) launch(k4_adjoint_kernel<false, 2>);
-            else if (minb == 4) launch(k4_adjoint_kernel<false, 4>);
-            else launch(k4_adjoint_kernel<false, 3>);
-        }
+        if (fast_diff)
+            wide ? launch(k4_adjoint_kernel<true, true>) : launch(k4_adjoint_kernel<true, false>);
+        else
+            wide ? launch(k4_adjoint_kernel<false, true>) : launch(k4_adjoint_kernel<false, false>);
     }
     timing_end(ctx, st);
     ctx->launches += nrec > 0 ? 2 : 1;
