@@ -122,8 +122,8 @@ int fp64_diff_main_device(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *beam
     PBT_TRY(upload(ctx, ctx->d_edge, edges.data(), edges.size(), st));
     PBT_TRY(k1_launch(ctx, st, ctx->d_fac.as<K1Facet>(), nbeam, next, ctx->d_edge.as<K1Edge>(), lambda,
                       fast_diff, d_afb, d_afe));
-    // the host vectors are released at return: finish the copies first
-    PBT_CUDA_TRY(cudaStreamSynchronize(st));
+    // No wait: copies from pageable memory return once they are staged, so the host
+    // vectors may go, and the host prepares the next orientation of a batch beside the sum.
     return PBT_OK;
 }
 
@@ -423,25 +423,28 @@ int host_batch(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const HostRuns &H
         PBT_TRY(totals_ensure(T, ntheta, nphi, st));
         PBT_TRY(totals_reset(T, st));
         PBT_TRY(ctx->d_out.ensure(2 * 8 * nb * sizeof(double)));
-        PBT_TRY(ctx->d_mu.ensure((16 * nb + 16 * ntheta + 18) * sizeof(double)));
+        // d_mu: mueller | m1d | averaged params | per-orientation params, copied at the end:
+        // a copy to the host after each orientation would wait for its sum
+        PBT_TRY(ctx->d_mu.ensure((16 * nb + 16 * ntheta + 18 * (norient + 1)) * sizeof(double)));
         double *d_afb = ctx->d_out.as<double>(), *d_afe = d_afb + 8 * nb;
         double *d_mu = ctx->d_mu.as<double>(), *d_m1 = d_mu + 16 * nb, *d_p = d_m1 + 16 * ntheta;
+        double *d_per = d_p + 18;
         for (int64_t o = 0; o < norient; o++) {
             PBT_TRY(fp64_diff_main_device(ctx, st, H.beam[o], beam_off[o + 1] - beam_off[o],
                                           H.ext[o], ext_off[o + 1] - ext_off[o], H.verts[o],
                                           nverts, face_off, face_vi, nfaces, lambda,
                                           is_fast_diff ? 1 : 0, d_afb, d_afe));
             PBT_TRY(k3_finalise(ctx, st, d_afb, d_afe, lambda, scaling ? 1 : 0, &params_in[o], d_mu,
-                                d_m1, d_p, &T));
-            if (params_per_orient)
-                PBT_CUDA_TRY(cudaMemcpyAsync(&params_per_orient[o], d_p, sizeof(pbt_output_params),
-                                             cudaMemcpyDeviceToHost, st));
+                                d_m1, d_per + 18 * o, &T));
         }
         PBT_TRY(totals_divide_device(ctx, T, st, norient, d_mu, d_m1, d_p));
         PBT_TRY(copy_to_host(ctx, mueller_avg, d_mu, 16 * nb * 8, st));
         PBT_CUDA_TRY(cudaMemcpyAsync(mueller_1d_avg, d_m1, 16 * ntheta * 8, cudaMemcpyDeviceToHost, st));
         PBT_CUDA_TRY(cudaMemcpyAsync(params_avg, d_p, sizeof(pbt_output_params),
                                      cudaMemcpyDeviceToHost, st));
+        if (params_per_orient)
+            PBT_CUDA_TRY(cudaMemcpyAsync(params_per_orient, d_per, norient * sizeof(pbt_output_params),
+                                         cudaMemcpyDeviceToHost, st));
         PBT_CUDA_TRY(cudaStreamSynchronize(st));
         return PBT_OK;
     }

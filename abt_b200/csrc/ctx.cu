@@ -147,7 +147,7 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
 }
 
 int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st) {
-    if (bytes < kIoMin || !pageable(src) || io_rented(ctx)) {
+    if (bytes < kIoMinUp || !pageable(src) || io_rented(ctx)) {
         PBT_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return PBT_OK;
     }
