@@ -978,16 +978,19 @@ __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
     b = make_float2(v.z, v.w);
 }
 
-template <bool FAST, bool WIDE>
+// GENERAL: the step with its rare branch (poles, forward bodge, clamp of ky).  Otherwise
+// the main step alone, which lowers tmin to the smallest kx^2 + kz^2: at or below the
+// clamp's the caller takes the general step instead.  WIDE: far-field phases of any size.
+template <bool FAST, bool GENERAL, bool WIDE>
 __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const BinPk &B,
-                                        float2 (&acc)[8], float2 hkRh,
+                                        float2 (&acc)[8], float2 hkRh, float &tmin,
                                         const float4 &hb, bool lo_ok, bool hi_ok,
                                         const double *__restrict__ xyz, int64_t nb,
                                         const float2 *__restrict__ rl) {
     // far-field half phase per facet, k u.c / 2 modulo pi, as a fixed-point fraction of
     // pi (2^-32 units): added to 1.5 * 2^20 the FP64 sum's low word is that fraction, so
     // the reduction costs no operation of its own (each of the three steps rounds to
-    // 2^-32 pi = 7e-10 rad).  That holds up to 2^19 half turns; records beyond (kWide, a
+    // 2^-32 pi = 7e-10 rad).  That holds up to 2^19 half turns; records beyond (WIDE, a
     // launch with k |com| above 1.6e6) subtract the nearest integer.
     float2 fr;
     {
@@ -1075,8 +1078,9 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     float2 P1 = fma2(r3, b, neg2(mul2(r4, a)));
     float2 R1 = fma2(r5, hn2, neg2(mul2(c, u)));
     float2 kzc = P.kzc;
-    const bool cx = tr.x <= kOneMinusClampSq, cy = tr.y <= kOneMinusClampSq;
-    if (B.pole || cx || cy) {
+    const bool cx = GENERAL && tr.x <= kOneMinusClampSq, cy = GENERAL && tr.y <= kOneMinusClampSq;
+    if (!GENERAL) tmin = fminf(tmin, fminf(tr.x, tr.y));
+    if (GENERAL && (B.pole || cx || cy)) {
         float2 r0, r1, r2, r6, r7, r8, q3, q4, q5, q9;
         ld22(&P.R[0], r0, r1);
         ld22(&P.R[2], r2, q3);
@@ -1362,6 +1366,12 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
         for (int q = 0; q < BPT; q++)
 #pragma unroll
             for (int c = 0; c < 8; c++) sum(q, c) = 0.0;
+        [[maybe_unused]] bool general = wide;
+        if constexpr (FAST) {
+#pragma unroll
+            for (int q = 0; q < BPT; q++) general = general || bd[q].pole;
+            general = __any_sync(0xffffffffu, general);
+        }
         bool failed = false;
         for (int c = 0; c < I.nchunk; c++) {
             if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&full[st]), phase))) {
@@ -1398,14 +1408,10 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                 if (c == I.nchunk - 1 && (I.edge & 2)) patch(n - 1, 0, 1);
             }
             float2 acc[BPT][8];
-#pragma unroll
-            for (int q = 0; q < BPT; q++)
-#pragma unroll
-                for (int cc = 0; cc < 8; cc++) acc[q][cc] = bc2(0.0f);
+            [[maybe_unused]] unsigned pm0 = 0, keep[2] = {0, 0};
             if (FAST) {
                 // the tile cull of the stage's 2n records, two per lane: a record
                 // whose field of view misses the warp's bins adds nothing
-                unsigned keep[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int r = h * 32 + lane;
@@ -1430,39 +1436,55 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     x = (x | (x >> 8)) & 0x0000FFFFu;
                     return x;
                 };
-                const unsigned pm0 = pairs_of(keep[0]) | (pairs_of(keep[1]) << 16);
-                auto pairs = [&](auto w) {
+                pm0 = pairs_of(keep[0]) | (pairs_of(keep[1]) << 16);
+            }
+            // Without the field-of-view test every lane adds (the edge pairs are patched
+            // above; a bin beyond nb is never written out).
+            float tmin = 1.0f;
+            auto pairs = [&](auto general_, auto wide_) {
+                constexpr bool G = decltype(general_)::value, WD = decltype(wide_)::value;
+#pragma unroll
+                for (int q = 0; q < BPT; q++)
+#pragma unroll
+                    for (int cc = 0; cc < 8; cc++) acc[q][cc] = bc2(0.0f);
+                if constexpr (FAST) {
                     for (unsigned pm = pm0; pm; pm &= pm - 1u) {
                         const int j = __ffs(pm) - 1;
                         const unsigned m = (j & 16 ? keep[1] : keep[0]) >> (2 * (j & 15));
                         const K2Fov *fv = P.fovs + 2 * (I.p0 + c * CH + j);
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<true, decltype(w)::value>(
-                                sbuf[st][j], fv, bd[q], acc[q], hkRh, s_hb[q][tid],
-                                (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0, P.xyz, P.nb,
-                                P.rlo + (I.p0 + c * CH + j) * 3);
+                            k2_pair<true, G, WD>(sbuf[st][j], fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
+                                                 (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0,
+                                                 P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
                     }
-                };
-                if (wide)
-                    pairs(std::true_type());
-                else
-                    pairs(std::false_type());
-            } else {
-                // without the field-of-view test every lane adds (the edge pairs are
-                // patched above; a bin beyond nb is never written out)
-                auto pairs = [&](auto w) {
+                } else {
                     for (int j = 0; j < n; j++)
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<false, decltype(w)::value>(
-                                sbuf[st][j], nullptr, bd[q], acc[q], hkRh, s_hb[q][tid], true, true,
-                                P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
-                };
-                if (wide)
-                    pairs(std::true_type());
-                else
-                    pairs(std::false_type());
+                            k2_pair<false, G, WD>(sbuf[st][j], nullptr, bd[q], acc[q], hkRh, tmin,
+                                                  s_hb[q][tid], true, true, P.xyz, P.nb,
+                                                  P.rlo + (I.p0 + c * CH + j) * 3);
+                }
+            };
+            if constexpr (FAST) {
+                // With the field-of-view test the main step goes without its rare branch: a
+                // warp with a bin near the poles takes the general loop (of any phase, too),
+                // and one that meets the clamp of ky (a 0.08 degree cone) does the chunk
+                // again: 13.25 -> 12.9 ms on 16 lists of 3,500 polygons.  The full sum gains
+                // nothing by it (216.1 against 216.5 ms; its main step alone, wrong at the
+                // poles, 210.2), and small grids, with more of their tiles at the poles,
+                // lose 1-3 %.
+                bool again = general;
+                if (!general) {
+                    pairs(std::false_type(), std::false_type());
+                    again = __any_sync(0xffffffffu, tmin <= kOneMinusClampSq);
+                }
+                if (again) pairs(std::true_type(), std::true_type());
+            } else if (wide) {
+                pairs(std::true_type(), std::true_type());
+            } else {
+                pairs(std::true_type(), std::false_type());
             }
 #pragma unroll
             for (int q = 0; q < BPT; q++)
