@@ -32,12 +32,13 @@
 //   in which the sums are kept; the basis change and the rotation T(phi), which
 //   depends on the bin alone, are applied once at the end.
 //
-// Bound: FP64 pipe (65 % of cycles; 399 instructions a triangle and bin, 207 of them
+// Bound: FP64 pipe (65 % of cycles; 360 instructions a triangle and bin, 196 of them
 // FP64, against 1,813 with every operation of the reference).  A triangle list of
-// 2,582 x 32,580 bins takes 1.62 ms (5.2e10 facet-bin/s), the operation-by-operation
-// kernel took 6.92 ms.  The facet records go through shared memory, three stages of 16
-// and one barrier a stage: read from global memory they cost 38 % of the issue slots
-// in load waits; a private stage per warp, without barriers, measured 3 % slower.
+// 2,582 x 32,580 bins takes 1.51 ms (5.6e10 facet-bin/s), the operation-by-operation
+// kernel took 6.92 ms (1.59 ms with quadrant polynomials in place of the table of
+// roots).  The facet records go through shared memory, three stages of 16 and one
+// barrier a stage: read from global memory they cost 38 % of the issue slots in load
+// waits; a private stage per warp, without barriers, measured 3 % slower.
 //
 // The file is built with -fmad=false: a multiply-add is fused only where fma()
 // is written.  Facet frames come from the host (host_setup.cpp); the bin grid
@@ -94,38 +95,29 @@ __device__ __forceinline__ double rsqrt_n(double x) {
     const double e = fma(-(x * y), y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
-// x = n pi/2 + r for |x| < 2^30: pi/2 in two parts, each product fused, so r is good
-// to 1e-16 absolute.  Returns r; q = n modulo 2^32.
-__device__ __forceinline__ double reduce_n(double x, int *q) {
-    const double t = fma(x, 0.6366197723675814, 6755399441055744.0);
-    *q = __double2loint(t);
+// e^{ix} from a table of the 128th roots of unity and short polynomials: x = n h + r, h =
+// 2 pi / 128 in two parts (each product fused, so r is good to 1e-16 absolute for
+// |x| < 2^30), and e^{ir} on |r| <= h/2 from minimax fits (Remez exchange in 50 digits:
+// 3e-17 for sin, 3e-20 for cos - 1).  15 FP64 operations; the quadrant form with
+// polynomials to r^13 and r^14 takes 20 and as many selects and sign changes again, the
+// library's checks for huge arguments too and reads its coefficients from memory.
+constexpr int kRoots = 128;
+__device__ __forceinline__ double reduce_n(double x, int *n32) {
+    const double t = fma(x, 20.371832715762604, 6755399441055744.0);
+    *n32 = __double2loint(t);  // n modulo 2^32
     const double n = t - 6755399441055744.0;
-    return fma(-n, 6.123233995736766e-17, fma(-n, 1.5707963267948966, x));
+    return fma(-n, 1.9135106236677394e-18, fma(-n, 0.04908738521234052, x));
 }
-// sin and cos of x + qk pi/2, |x| < 2^30: minimax polynomials in r^2 on [0, pi^2/16]
-// (Remez exchange in 50 digits: 3e-18 relative for sin, 1.5e-19 absolute for cos).
-// The library's form checks for huge arguments and reads its coefficients from
-// memory.
-__device__ __forceinline__ void sincos_n(double x, int qk, double *sn, double *cs) {
-    int q;
-    const double r = reduce_n(x, &q);
-    q += qk;
+// e^{i (x + nk h)}, roots[k] = (cos, sin)(k h)
+__device__ __forceinline__ void sincos_n(double x, int nk, const double2 *roots, double *sn, double *cs) {
+    int n;
+    const double r = reduce_n(x, &n);
+    const double2 w = roots[(n + nk) & (kRoots - 1)];
     const double z = r * r;
-    double p = fma(z, 1.589679568451575e-10, -2.5050758115840255e-08);
-    p = fma(z, p, 2.7557313691921887e-06);
-    p = fma(z, p, -0.00019841269829807819);
-    p = fma(z, p, 0.008333333333322413);
-    p = fma(z, p, -0.16666666666666632);
-    double c = fma(z, -1.1367981880469046e-11, 2.0875897738682843e-09);
-    c = fma(z, c, -2.7557315738613277e-07);
-    c = fma(z, c, 2.4801587294628004e-05);
-    c = fma(z, c, -0.001388888888888284);
-    c = fma(z, c, 0.04166666666666665);
-    const double s0 = fma(r * z, p, r), c0 = fma(z, fma(z, c, -0.5), 1.0);
-    const double a = (q & 1) ? c0 : s0, b = (q & 1) ? s0 : c0;
-    // signs: sin turns with bit 1 of q, cos with bit 1 of q + 1
-    *sn = __hiloint2double(__double2hiint(a) ^ ((q & 2) << 30), __double2loint(a));
-    *cs = __hiloint2double(__double2hiint(b) ^ (((q + 1) & 2) << 30), __double2loint(b));
+    const double s = fma(r * z, fma(z, 0.008333155366073453, -0.16666666662958388), r);
+    const double c = z * fma(z, fma(z, -0.0013888601850806472, 0.041666666656641586), -0.499999999999999);
+    *cs = fma(-w.y, s, fma(w.x, c, w.x));
+    *sn = fma(w.x, s, fma(w.y, c, w.y));
 }
 
 // contour_integral for one bin (src/diff_mod.f90:357-428), operation by operation
@@ -226,6 +218,9 @@ __device__ __forceinline__ void k1_stage(K1Facet *dst, const K1Facet *src, int n
 template <bool FAST>
 __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P) {
     __shared__ K1Facet sfac[K1_NST][K1_CH];
+    __shared__ double2 s_root[kRoots];  // see sincos_n; the first stage's barrier publishes it
+    static_assert(K1_THREADS == kRoots, "one root a thread");
+    sincospi(threadIdx.x * (2.0 / kRoots), &s_root[threadIdx.x].y, &s_root[threadIdx.x].x);
     const int kind = (int)blockIdx.y >= P.split[0];
     const int run = (int)blockIdx.y - (kind ? P.split[0] : 0);
     const int64_t fb = P.first[kind] + run * P.run[kind];
@@ -310,11 +305,11 @@ __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P)
                 const double z3h = v5.x * xh + v5.y * yh + v6.x * zh;
                 polar_ref(F, kx, ky, kz, x3h / rh, y3h / rh, z3h / rh, &A, &B);
             }
-            // aperture integral; the phase bvs = n pi/2 + rK joins each vertex phase
+            // aperture integral; the phase bvs = nK h + rK joins each vertex phase
             const int nv = (int)F->nv;
             const double kxx = fma(-waveno, kx, v1.y), kyy = fma(-waveno, ky, v6.y);
-            int qK;
-            const double rK = reduce_n(bvs, &qK);
+            int nK;
+            const double rK = reduce_n(bvs, &nK);
             Z g;
             // a lower bound of min |omega| * min(|kxx|, |kyy|) from the high words; the
             // contour also takes the reference's floor of 1e-6 under |kxx| and |kyy|
@@ -332,9 +327,9 @@ __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P)
                 if (!contour) {
                     const double2 p0 = v[12], p1 = v[13], p2 = v[14];
                     double s0, c0, s1, c1, s2, c2;
-                    sincos_n(fma(kyy, p0.y, fma(kxx, p0.x, rK)), qK, &s0, &c0);
-                    sincos_n(fma(kyy, p1.y, fma(kxx, p1.x, rK)), qK, &s1, &c1);
-                    sincos_n(fma(kyy, p2.y, fma(kxx, p2.x, rK)), qK, &s2, &c2);
+                    sincos_n(fma(kyy, p0.y, fma(kxx, p0.x, rK)), nK, s_root, &s0, &c0);
+                    sincos_n(fma(kyy, p1.y, fma(kxx, p1.x, rK)), nK, s_root, &s1, &c1);
+                    sincos_n(fma(kyy, p2.y, fma(kxx, p2.x, rK)), nK, s_root, &s2, &c2);
                     // i sum_j e_j / prod (d_j - d_k) = -i (e_0 w1 + e_1 w2 + e_2 w0) / (w0 w1 w2)
                     const double t = v7.y * rcp_n(w0 * w1 * wl);
                     g.re = fma(s2, w0, fma(s1, wl, s0 * w1)) * t;
@@ -350,7 +345,7 @@ __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P)
                 if (!contour) {
                     double s0, c0, sp, cp;
                     g = {0, 0};
-                    sincos_n(fma(kyy, E[0].yj, fma(kxx, E[0].xj, rK)), qK, &s0, &c0);
+                    sincos_n(fma(kyy, E[0].yj, fma(kxx, E[0].xj, rK)), nK, s_root, &s0, &c0);
                     sp = s0;
                     cp = c0;
                     for (int q = 0; q < nv; q++) {
@@ -358,7 +353,7 @@ __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P)
                         const double w = fma(-kyy, E[q].dy, kdx) * rcp_n(fma(kyy, E[q].dy, kdx));
                         double sn = s0, cn = c0;
                         if (q + 1 < nv)
-                            sincos_n(fma(kyy, E[q + 1].yj, fma(kxx, E[q + 1].xj, rK)), qK, &sn, &cn);
+                            sincos_n(fma(kyy, E[q + 1].yj, fma(kxx, E[q + 1].xj, rK)), nK, s_root, &sn, &cn);
                         g.re = fma(w, sn - sp, g.re);
                         g.im = fma(w, cp - cn, g.im);
                         sp = sn;
