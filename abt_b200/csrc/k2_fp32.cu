@@ -171,6 +171,33 @@ __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const 
     for (int q = 0; q < 8; q++) put(P.amp[q], (float)uc[q]);
 }
 
+// A record's field-of-view data: prop0, fov and the facet centre.
+__device__ __forceinline__ K2Fov make_fov(const double *prop0, double fov, const double *com) {
+    K2Fov fv;
+    fv.p0[0] = (float)prop0[0];
+    fv.p0[1] = (float)prop0[1];
+    fv.p0[2] = (float)prop0[2];
+    fv.cos_fov = (float)cos(fov);
+    // the per-bin test uses the direction from the facet centre: it is
+    // within |c|/R of the direction from the origin; 2|c|/R + 1e-5 rad
+    // also covers the FP32 rounding of both tests
+    const double cn = sqrt(com[0] * com[0] + com[1] * com[1] + com[2] * com[2]);
+    const double fovm = fov + 2.0 * cn / kFarR + 1e-5;
+    fv.fovm = (float)fovm;
+    fv.cos_fovm = (float)cos(fovm);
+    fv.sin_fovm = (float)sin(fovm);
+    // FP32 test error: second-order parallax (< 3 |c/R|^2) and rounding (< 8e-7)
+    const double e2 = (cn / kFarR) * (cn / kFarR);
+    fv.tol = (float)(3.0 * e2 + 8e-7);
+    for (int c = 0; c < 3; c++) {
+        fv.com[c] = com[c];
+        fv.p0d[c] = prop0[c];
+    }
+    fv.cos_fovd = cos(fov);
+    fv.pad = 0.0;
+    return fv;
+}
+
 __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restrict__ verts,
                                 int64_t nverts, const int64_t *__restrict__ face_off,
                                 int64_t nfaces, const int64_t *__restrict__ face_vi, double waveno, double lambda, int fast_diff,
@@ -298,33 +325,114 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
             recs[r0 + t] = rec;
         }
         if (fast_diff) {
-            K2Fov fv;
-            const double fov = kind ? kPiRef / 2.0 : ob->fov;
-            fv.p0[0] = (float)prop0[0];
-            fv.p0[1] = (float)prop0[1];
-            fv.p0[2] = (float)prop0[2];
-            fv.cos_fov = (float)cos(fov);
-            // the per-bin test uses the direction from the facet centre: it is
-            // within |c|/R of the direction from the origin; 2|c|/R + 1e-5 rad
-            // also covers the FP32 rounding of both tests
-            const double cn = sqrt(fr.com[0] * fr.com[0] + fr.com[1] * fr.com[1] +
-                                   fr.com[2] * fr.com[2]);
-            const double fovm = fov + 2.0 * cn / kFarR + 1e-5;
-            fv.fovm = (float)fovm;
-            fv.cos_fovm = (float)cos(fovm);
-            fv.sin_fovm = (float)sin(fovm);
-            // FP32 test error: second-order parallax (< 3 |c/R|^2) and rounding (< 8e-7)
-            const double e2 = (cn / kFarR) * (cn / kFarR);
-            fv.tol = (float)(3.0 * e2 + 8e-7);
-            for (int c = 0; c < 3; c++) {
-                fv.com[c] = fr.com[c];
-                fv.p0d[c] = prop0[c];
-            }
-            fv.cos_fovd = cos(fov);
-            fv.pad = 0.0;
-            fovs[r0 + t] = fv;
+            fovs[r0 + t] = make_fov(prop0, kind ? kPiRef / 2.0 : ob->fov, fr.com);
         }
     }
+}
+
+// Thread per outbeam g: its half of facet pair g / 2 (K2Poly and its vertices, `stride`
+// bytes a pair).  Both threads of a pair look up both faces for the fans' common length.
+__global__ void k2_setup_poly_kernel(RefSrc S, int64_t nrefs, const double *__restrict__ verts,
+                                     int64_t nverts, const int64_t *__restrict__ face_off,
+                                     int64_t nfaces, const int64_t *__restrict__ face_vi, double waveno,
+                                     double lambda, int fast_diff, int nvmax, char *__restrict__ polys,
+                                     int64_t stride, K2Fov *__restrict__ fovs, float2 *__restrict__ rlo,
+                                     int *__restrict__ err, unsigned *__restrict__ epsmax) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= nrefs) return;
+    int64_t o, o2;
+    int kind, kind2;
+    const pbt_outbeam *ob = ref_lookup(S, g, o, kind);
+    auto corners = [&](const pbt_outbeam *b) {
+        return b->fi < 1 || b->fi > nfaces ? 0 : (int)(face_off[b->fi] - face_off[b->fi - 1]);
+    };
+    int nv = corners(ob);
+    if (nv == 0) atomicOr(err, 1);
+    if (nv > kMaxPolyVerts) atomicOr(err, 2);  // larger faces are not supported in FP32
+    if (nv > nvmax) nv = 0;
+    const int64_t g2 = g ^ 1;
+    const int nv2 = g2 < nrefs ? corners(ref_lookup(S, g2, o2, kind2)) : 0;
+    const int m = max(max(nv, nv2 > nvmax ? 0 : nv2), 3) - 2;
+    K2Poly &P = *reinterpret_cast<K2Poly *>(polys + (g >> 1) * stride);
+    K2PolyVertex *pv = reinterpret_cast<K2PolyVertex *>(&P + 1);
+    const int h = (int)(g & 1);
+    auto put = [h](float2 &dst, double v) {
+        if (h)
+            dst.y = (float)v;
+        else
+            dst.x = (float)v;
+    };
+    P.m = m;  // the same value from both threads
+    FacetFrame fr;
+    double vx[kMaxPolyVerts], vy[kMaxPolyVerts], vz[kMaxPolyVerts], sign = 1.0;
+    if (nv > 0) {
+        const int64_t fb = face_off[ob->fi - 1];
+        const double *V = verts + o * 3 * nverts;
+        for (int i = 0; i < nv; i++) {
+            const int64_t vi = face_vi[fb + i] - 1;
+            vx[i] = V[vi];
+            vy[i] = V[vi + nverts];
+            vz[i] = V[vi + 2 * nverts];
+        }
+        facet_frame(vx, vy, vz, nv, ob->prop_out, ob->vk7, fr, nullptr, nullptr, nullptr);
+        sign = fr.sign;
+    } else {
+        // no face: a record that adds nothing
+        fr = FacetFrame{};
+        fr.R.m[0][0] = fr.R.m[1][1] = fr.R.m[2][2] = 1.0;
+    }
+    const double *com = fr.com;
+    const double R = kFarR, c2 = com[0] * com[0] + com[1] * com[1] + com[2] * com[2];
+    atomicMax(epsmax, __float_as_uint((float)(sqrt(c2) / R * (1.0 + 1e-6)) + 1e-30f));
+    const double Ky = fr.prop2[1], cf2 = 1.0 / (1.0 - Ky * Ky);
+    for (int c = 0; c < 3; c++) {
+        P.kc[c][h] = 0.5 * kInvPi * waveno * com[c];
+        put(P.eps[c], com[c] / R);
+    }
+    put(P.b, c2 / (R * R));
+    for (int q = 0; q < 9; q++) put(P.R[q], fr.R.m[q / 3][q % 3]);
+    put(P.nKx, -fr.prop2[0]);
+    put(P.kzc, -fr.prop2[2] * cf2);
+    for (int i = 0; i < 3; i++) {
+        put(rlo[(g >> 1) * 3 + i], fr.R.m[1][i] - (double)(float)fr.R.m[1][i]);
+        // an odd list: the last pair's unused half
+        if (g == nrefs - 1 && !h) rlo[(g >> 1) * 3 + i].y = 0.0f;
+    }
+    // amplitude (2 i / lambda) sign ampl in the circular basis, times sqrt(1 - Ky^2) / 4
+    const double cpre = nv > 0 ? 2.0 / lambda * sign : 0.0, sk = 0.25 / sqrt(cf2);
+    for (int b = 0; b < 2; b++) {
+        double am[4];  // (1,b), (2,b) re/im
+        for (int q = 0; q < 2; q++) {
+            am[2 * q] = -cpre * ob->ampl[4 * b + 2 * q + 1];
+            am[2 * q + 1] = cpre * ob->ampl[4 * b + 2 * q];
+        }
+        put(P.amp[4 * b], sk * (am[0] - am[3]));
+        put(P.amp[4 * b + 1], sk * (am[1] + am[2]));
+        put(P.amp[4 * b + 2], sk * (am[0] + am[3]));
+        put(P.amp[4 * b + 3], sk * (am[1] - am[2]));
+    }
+    double x0 = 0, y0 = 0, xp = 0, yp = 0;
+    for (int j = 0; j < m + 2; j++) {
+        double x = xp, y = yp, w = 0.0;
+        if (j < nv) {
+            const double d[3] = {vx[j] - com[0], vy[j] - com[1], vz[j] - com[2]};
+            double r[3];
+            mv33(fr.R, d, r);
+            x = r[0];
+            y = r[1];
+            if (j == 0) {
+                x0 = x;
+                y0 = y;
+            }
+            if (j >= 2) w = 0.5 * ((xp - x0) * (y - y0) - (x - x0) * (yp - y0));
+        }
+        put(pv[j].vx, -0.5 * waveno * x);
+        put(pv[j].vy, -0.5 * waveno * y);
+        put(pv[j].w, w);
+        xp = x;
+        yp = y;
+    }
+    if (fast_diff) fovs[g] = make_fov(ob->prop_out, kind ? kPiRef / 2.0 : ob->fov, com);
 }
 
 // Per orientation chunk [o0, o0+no): segment records and work-item prefix (block 0, a
@@ -931,11 +1039,10 @@ __device__ __forceinline__ TriF tri_front(float2 t1, float2 t2, float2 t3) {
     return F;
 }
 
-__device__ __forceinline__ void tri_back(const TriF &F, float2 hn2, float2 tt, float2 &gx, float2 &gy) {
+// scr = sc / (p12 Dh); twice_sc() is formed only where the Taylor series needs it.
+template <class Sc>
+__device__ __forceinline__ void tri_back(const TriF &F, float2 scr, Sc twice_sc, float2 &gx, float2 &gy) {
     const float2 Dh = F.Dh;
-    const float2 q = mul2(mul2(F.p12, Dh), tt);
-    const float2 hq = mul2(hn2, mul2(q, q));
-    const float2 scr = make_float2(rsqrt_fz(hq.x), rsqrt_fz(hq.y));
     gx = mul2(fma2(F.S1, F.s1, neg2(mul2(F.S2, F.s2))), scr);
     gy = mul2(fma2(F.S2, F.k2, neg2(mul2(F.S1, F.k1))), scr);
     // (uniform over the warp: the lanes that need it select)
@@ -954,8 +1061,7 @@ __device__ __forceinline__ void tri_back(const TriF &F, float2 hn2, float2 tt, f
         const float2 q4 = fma2(yc, q3, ya4);
         const float2 q5 = fma2(yc, q4, mul2(ya4, ya));
         const float2 q6 = fma2(yc, q5, mul2(ya4, ya2));
-        const float2 ht = mul2(mul2(hn2, tt), tt);
-        const float2 tsc = make_float2(2.0f * rsqrt_fz(ht.x), 2.0f * rsqrt_fz(ht.y));
+        const float2 tsc = twice_sc();
         const float2 re = mul2(tsc, fma2(q6, bc2(1.0f / 630.0f),
                                          fma2(q4, bc2(-1.0f / 45.0f), fma2(q2, bc2(1.0f / 6.0f), bc2(-0.5f)))));
         const float2 im = mul2(tsc, fma2(q5, bc2(-2.0f / 315.0f),
@@ -970,6 +1076,13 @@ __device__ __forceinline__ void tri_back(const TriF &F, float2 hn2, float2 tt, f
     }
 }
 
+// 2 g for each lane, g the second divided difference alone
+__device__ __forceinline__ void tri_poly(float2 t1, float2 t2, float2 t3, float2 &gx, float2 &gy) {
+    const TriF F = tri_front(t1, t2, t3);
+    const float2 q = mul2(F.p12, F.Dh);
+    tri_back(F, make_float2(rcp_approx(q.x), rcp_approx(q.y)), [] { return make_float2(2.0f, 2.0f); }, gx, gy);
+}
+
 // Two adjacent float2 fields of a record pair from one 16-byte shared-memory load
 // (every such field pair of K2Pair starts on a 16-byte boundary).
 __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
@@ -981,8 +1094,8 @@ __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
 // GENERAL: the step with its rare branch (poles, forward bodge, clamp of ky).  Otherwise
 // the main step alone, which lowers tmin to the smallest kx^2 + kz^2: at or below the
 // clamp's the caller takes the general step instead.  WIDE: far-field phases of any size.
-template <bool FAST, bool GENERAL, bool WIDE>
-__device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const BinPk &B,
+template <bool FAST, bool GENERAL, bool WIDE, class PairT>
+__device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const BinPk &B,
                                         float2 (&acc)[8], float2 hkRh, float &tmin,
                                         const float4 &hb, bool lo_ok, bool hi_ok,
                                         const double *__restrict__ xyz, int64_t nb,
@@ -1043,9 +1156,10 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     // the divided difference's phases, sort, sines and cosines: independent of
     // the polarisation block and its rare branch, so formed ahead of the branch
     // (one basic block with the direction arithmetic for the scheduler)
-    TriF tf;
-    {
-        const float2 dx = add2(kx, nKx);
+    constexpr bool POLY = std::is_same<PairT, K2Poly>::value;
+    const float2 dx = add2(kx, nKx);
+    [[maybe_unused]] TriF tf;
+    if constexpr (!POLY) {
         float2 vx0, vx1, vx2, vy0, vy1, vy2;
         ld22(&P.vx[0], vx0, vx1);
         ld22(&P.vx[2], vx2, vy0);
@@ -1169,7 +1283,38 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
     // aperture integral on the half phases, its second half (the normalisation
     // sc needs the polarisation block's |h| and tt): 2 sc g
     float2 gx, gy;
-    tri_back(tf, hn2, tt, gx, gy);
+    if constexpr (!POLY) {
+        const float2 q = mul2(mul2(tf.p12, tf.Dh), tt);
+        const float2 hq = mul2(hn2, mul2(q, q));
+        tri_back(tf, make_float2(rsqrt_fz(hq.x), rsqrt_fz(hq.y)), [&] {
+            const float2 ht = mul2(mul2(hn2, tt), tt);
+            return make_float2(2.0f * rsqrt_fz(ht.x), 2.0f * rsqrt_fz(ht.y));
+        }, gx, gy);
+    } else {
+        // the fan's triangles share all of the above; their areas weight them
+        const float4 *v = reinterpret_cast<const float4 *>(&P + 1);  // vx, vy | w, pad
+        auto phase = [&](int j) {
+            const float4 q = v[2 * j];
+            return fma2(ky, make_float2(q.z, q.w), fma2(dx, make_float2(q.x, q.y), ph));
+        };
+        const float2 t0 = phase(0);
+        float2 tp = phase(1);
+        gx = gy = bc2(0.0f);
+        const int m = P.m;
+#pragma unroll 1
+        for (int j = 2; j < m + 2; j++) {
+            const float2 tn = phase(j), w = *reinterpret_cast<const float2 *>(&v[2 * j + 1]);
+            float2 ax, ay;
+            tri_poly(t0, tp, tn, ax, ay);
+            gx = fma2(w, ax, gx);
+            gy = fma2(w, ay, gy);
+            tp = tn;
+        }
+        const float2 ht = mul2(mul2(hn2, tt), tt);
+        const float2 sc = make_float2(rsqrt_fz(ht.x), rsqrt_fz(ht.y));
+        gx = mul2(gx, sc);
+        gy = mul2(gy, sc);
+    }
     // [[A, B], [-B, A]] is diagonal in the circular basis: with z = A - iB the
     // columns' u+ take z, their u- take conj(z).  q+ = g z, q- = g conj(z).
     const float2 gyB = mul2(gy, Bc), gxB = mul2(gx, Bc);
@@ -1209,6 +1354,7 @@ __device__ __forceinline__ void k2_pair(const K2Pair &P, const K2Fov *fv, const 
 // four CTAs per SM); 32 with the field-of-view cull, whose per-stage keep masks are
 // two 32-bit ballot words of the stage's 64 records.
 constexpr int K2P_CH_FULL = 44, K2P_CH_FOV = 32;
+constexpr int kPolyStage = 44 * 288;  // bytes a stage of polygons: 29 pairs of up to 6 vertices
 
 // The record's per-bin test passes no bin of the tile when the angle between
 // prop0 and the tile centre exceeds fovm + psi (fovm includes the parallax
@@ -1222,6 +1368,8 @@ __device__ __forceinline__ bool cone_culled(const K2Fov &f, const K2Cone &t) {
 struct K2PkArgs {
     const float2 *rlo;  // R_1 - (float)R_1, pair layout (3 per pair)
     const K2Pair *pairs;
+    const char *polys;  // polygons: K2Poly and vertices, stride bytes a pair
+    int stride, chunk;  // and pairs per shared-memory stage
     const K2Fov *fovs;
     const int *perm;        // is_fast_diff: tile-major bin order (-1: padding)
     const K2Cone *cones;    // is_fast_diff: cone of each warp's 32 bins
@@ -1250,11 +1398,19 @@ struct K2PkArgs {
 // With the field-of-view test each warp culls the stage's records against the cone of
 // its own 4 x 8 bins (13.3 ms; 14.9 with one 8 x 16 cone for the CTA, on 16 lists of
 // 3,500 polygons x 64,979 bins).
-template <int BPT, bool FAST>
+// POLY: facets of up to 16 vertices as one record each (K2Poly): the direction, the
+// polarisation block and the phase once a facet, a divided difference for each triangle
+// of its fan.  16 lists of 3,500 facets of 3-6 vertices with the field-of-view test: 9.85
+// ms against 12.75 as fans.
+template <int BPT, bool FAST, bool POLY>
 __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kernel(K2PkArgs P) {
-    constexpr int CH = FAST ? K2P_CH_FOV : K2P_CH_FULL;
+    using PairT = std::conditional_t<POLY, K2Poly, K2Pair>;
+    constexpr int CHT = FAST ? K2P_CH_FOV : K2P_CH_FULL;
+    const int CH = POLY ? P.chunk : CHT;
     constexpr int NW = K2_THREADS / 32;
-    __shared__ __align__(128) K2Pair sbuf[K2_NST][CH];
+    __shared__ __align__(128) char sbuf[K2_NST][POLY ? kPolyStage : CHT * sizeof(K2Pair)];
+    const int stride = POLY ? P.stride : (int)sizeof(K2Pair);
+    auto pair_at = [&](int s, int j) -> PairT & { return *reinterpret_cast<PairT *>(sbuf[s] + j * stride); };
     __shared__ __align__(8) uint64_t full[K2_NST], empty[K2_NST];
     __shared__ float4 s_hb[BPT][K2_THREADS];  // forward-bodge bin directions of this CTA's bins
     // the item's FP64 sums, a column per thread: in registers (two bins a thread) they
@@ -1295,7 +1451,8 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
         auto load = [&](int c, int s) {
             const int n = min(CH, I.npair - c * CH);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            bulk_load(smem_u32(&sbuf[s][0]), P.pairs + I.p0 + c * CH, (uint32_t)(n * sizeof(K2Pair)),
+            const char *src = POLY ? P.polys : reinterpret_cast<const char *>(P.pairs);
+            bulk_load(smem_u32(sbuf[s]), src + (I.p0 + c * CH) * stride, (uint32_t)(n * stride),
                       smem_u32(&full[s]));
         };
         if (tid == 0) {
@@ -1384,17 +1541,20 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                 // record of another item or the array's padding: that half takes a
                 // copy of the pair's other record with zero amplitude, so the pair
                 // loop needs no per-pair range test.  Every warp writes the same
-                // values for itself: 3 FP64 phases, then the 30 float2 fields from
-                // eps on (the last 8 are the amplitudes).
+                // values for itself: 3 FP64 phases, then the float2 fields from eps on
+                // (8 of them the amplitudes; a polygon's length m belongs to both halves,
+                // its vertices follow).
                 auto patch = [&](int j, int src, int dst) {
-                    K2Pair &Q = sbuf[st][j];
-                    for (int t = lane; t < 33; t += 32) {
+                    PairT &Q = pair_at(st, j);
+                    float2 *f = &Q.eps[0];
+                    const int amp0 = (int)(&Q.amp[0] - f);
+                    const int nf = (stride - (int)((char *)f - (char *)&Q)) / 8;
+                    for (int t = lane; t < 3 + nf; t += 32) {
                         if (t < 3) {
                             Q.kc[t][dst] = Q.kc[t][src];
-                        } else {
-                            float2 *f = &Q.eps[0];
+                        } else if (!POLY || t - 3 != amp0 - 1) {
                             const int i = t - 3;
-                            const float v = i >= 22 ? 0.0f : (src ? f[i].y : f[i].x);
+                            const float v = i >= amp0 && i < amp0 + 8 ? 0.0f : (src ? f[i].y : f[i].x);
                             if (dst)
                                 f[i].y = v;
                             else
@@ -1454,7 +1614,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                         const K2Fov *fv = P.fovs + 2 * (I.p0 + c * CH + j);
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<true, G, WD>(sbuf[st][j], fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
+                            k2_pair<true, G, WD>(pair_at(st, j), fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
                                                  (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0,
                                                  P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
                     }
@@ -1462,7 +1622,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     for (int j = 0; j < n; j++)
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<false, G, WD>(sbuf[st][j], nullptr, bd[q], acc[q], hkRh, tmin,
+                            k2_pair<false, G, WD>(pair_at(st, j), nullptr, bd[q], acc[q], hkRh, tmin,
                                                   s_hb[q][tid], true, true, P.xyz, P.nb,
                                                   P.rlo + (I.p0 + c * CH + j) * 3);
                 }
@@ -1851,6 +2011,8 @@ K2Plan k2_plan_for(const pbt_ctx *ctx) {
 struct K2Setup {
     K2Rec *recs = nullptr;
     K2Pair *pairs = nullptr;
+    char *polys = nullptr;  // facet pairs of polygons, poly_stride bytes each
+    int64_t poly_stride = 0;
     K2Fov *fovs = nullptr;
     float2 *rlo = nullptr;  // R_1 - (float)R_1 per record (the y row), pair layout (3 per pair)
     RefSrc src{};
@@ -1883,14 +2045,21 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
                const int64_t *h_beam_off, const pbt_outbeam *d_ext, const int64_t *h_ext_off,
                const double *d_verts, int64_t nverts, const int64_t *h_face_off,
                const int64_t *d_face_off, const int64_t *d_face_vi, int64_t nfaces, double lambda,
-               int fast_diff, int variant, K2Flags *flags, K2Setup &S) {
+               int fast_diff, const K2Plan &plan, K2Flags *flags, K2Setup &S) {
     pbt::NvtxRange nvtx_("pbt: set-up (records)");
     const int64_t nrefs = h_beam_off[norient] + h_ext_off[norient];
     const FaceRange nv = face_range(h_face_off, nfaces);
-    const int64_t max_recs = std::max<int64_t>(1, nrefs * std::max<int64_t>(1, nv.hi - 2));
+    const int variant = plan.variant;
+    // One record a facet (k2_main_pk_kernel's POLY) from 1.2 triangles a face on, one a
+    // triangle of the fan below and with the other plans.  Measured on 6 lists of 3,500
+    // facets, 361 x 180 bins, quads among triangles: 10 % quads 6.97 ms (facets) against
+    // 6.71 (fans), 20 % 7.49 against 7.51, all quads 9.31 against 12.08.
+    const bool poly = variant == 1 && plan.bpt == 1 && nv.hi > 3 && 5 * h_face_off[nfaces] >= 16 * nfaces;
+    const int64_t nvp = std::min<int64_t>(nv.hi, kMaxPolyVerts);
+    const int64_t max_recs = std::max<int64_t>(1, nrefs * (poly ? 1 : std::max<int64_t>(1, nv.hi - 2)));
     // Faces of one vertex count (triangles nearly always): outbeam g's records start at
-    // g (nv - 2), so the count and its scan (three launches) are for mixed faces only.
-    const bool uniform = nv.lo == nv.hi;
+    // g (nv - 2), so the count and its scan (three launches) are for mixed fans only.
+    const bool uniform = poly || nv.lo == nv.hi;
     size_t scan_tmp = 0;
     if (!uniform)
         cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr,
@@ -1910,14 +2079,18 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     src.ext_off = rb + 2 * (norient + 1);
     src.norient = norient;
     src.start = uniform ? nullptr : (int64_t *)(base + o_start);
-    src.per = nv.lo - 2;
+    src.per = poly ? 1 : nv.lo - 2;
+    S.poly_stride = poly ? (int64_t)(sizeof(K2Poly) + nvp * sizeof(K2PolyVertex)) : 0;
     // records (or record pairs; an even count so the last pair is whole)
     const int64_t nrec2 = (max_recs + 1) & ~(int64_t)1;
-    const size_t rec_bytes = variant ? (size_t)(nrec2 / 2) * sizeof(K2Pair) : (size_t)max_recs * sizeof(K2Rec);
+    const size_t rec_bytes = poly      ? (size_t)(nrec2 / 2) * S.poly_stride
+                             : variant ? (size_t)(nrec2 / 2) * sizeof(K2Pair)
+                                       : (size_t)max_recs * sizeof(K2Rec);
     const size_t fov_bytes = fast_diff ? align_up(nrec2 * sizeof(K2Fov)) : 0;
     PBT_TRY(ctx->d_rec.ensure(align_up(rec_bytes) + fov_bytes + (size_t)(nrec2 / 2) * 3 * sizeof(float2)));
     S.recs = variant ? nullptr : ctx->d_rec.as<K2Rec>();
-    S.pairs = variant ? ctx->d_rec.as<K2Pair>() : nullptr;
+    S.pairs = variant && !poly ? ctx->d_rec.as<K2Pair>() : nullptr;
+    S.polys = poly ? ctx->d_rec.as<char>() : nullptr;
     S.fovs = fast_diff ? (K2Fov *)(ctx->d_rec.as<char>() + align_up(rec_bytes)) : nullptr;
     S.rlo = (float2 *)(ctx->d_rec.as<char>() + align_up(rec_bytes) + fov_bytes);
     // host-side offsets -> device (pinned staging; the previous call's copy
@@ -1951,7 +2124,11 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     // 64 threads: a short list's set-up is one chain of FP64 steps a thread, spread over
     // the SMs
     const int th = 64;
-    if (nrefs > 0)
+    if (nrefs > 0 && poly)
+        k2_setup_poly_kernel<<<(unsigned)((nrefs + th - 1) / th), th, 0, st>>>(
+            src, nrefs, d_verts, nverts, d_face_off, nfaces, d_face_vi, waveno, lambda, fast_diff, (int)nvp,
+            S.polys, S.poly_stride, S.fovs, S.rlo, &flags->err, &flags->epsmax);
+    else if (nrefs > 0)
         k2_setup_kernel<<<(unsigned)((nrefs + th - 1) / th), th, 0, st>>>(
             src, nrefs, d_verts, nverts, d_face_off, nfaces, d_face_vi, waveno, lambda, fast_diff,
             S.recs, S.pairs, S.fovs, S.rlo, &flags->err, &flags->epsmax);
@@ -1979,18 +2156,18 @@ int k2_launch_main(pbt_ctx *ctx, cudaStream_t st, const K2MainArgs &A) {
     return PBT_OK;
 }
 
-template <int BPT, bool FAST>
+template <int BPT, bool FAST, bool POLY>
 int k2_launch_pk(pbt_ctx *ctx, cudaStream_t st, const K2PkArgs &A) {
     static const int occ = [] {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k2_main_pk_kernel<BPT, FAST>, K2_THREADS,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k2_main_pk_kernel<BPT, FAST, POLY>, K2_THREADS,
                                                           0) != cudaSuccess)
             (void)cudaGetLastError();
         return n > 0 ? n : 1;
     }();
     const int grid = ctx->sm_count * occ;
     timing_begin(ctx, st);
-    k2_main_pk_kernel<BPT, FAST><<<grid, K2_THREADS, 0, st>>>(A);
+    k2_main_pk_kernel<BPT, FAST, POLY><<<grid, K2_THREADS, 0, st>>>(A);
     timing_end(ctx, st);
     ctx->launches++;
     PBT_CUDA_TRY(cudaGetLastError());
@@ -2144,6 +2321,9 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags
     if (plan.variant == 1) {
         K2PkArgs B;
         B.pairs = S.pairs;
+        B.polys = S.polys;
+        B.stride = (int)S.poly_stride;
+        B.chunk = S.polys ? std::min(fast_diff ? K2P_CH_FOV : K2P_CH_FULL, (int)(kPolyStage / S.poly_stride)) : 0;
         B.rlo = S.rlo;
         B.fovs = S.fovs;
         B.perm = cull ? g.fast_perm.as<int>() : nullptr;
@@ -2164,9 +2344,11 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags
         B.tickets = A.tickets;
         B.counter = counter;
         B.err = &flags->err;
+        if (S.polys)
+            return fast_diff ? k2_launch_pk<1, true, true>(ctx, st, B) : k2_launch_pk<1, false, true>(ctx, st, B);
         if (plan.bpt == 1)
-            return fast_diff ? k2_launch_pk<1, true>(ctx, st, B) : k2_launch_pk<1, false>(ctx, st, B);
-        return fast_diff ? k2_launch_pk<2, true>(ctx, st, B) : k2_launch_pk<2, false>(ctx, st, B);
+            return fast_diff ? k2_launch_pk<1, true, false>(ctx, st, B) : k2_launch_pk<1, false, false>(ctx, st, B);
+        return fast_diff ? k2_launch_pk<2, true, false>(ctx, st, B) : k2_launch_pk<2, false, false>(ctx, st, B);
     }
     if (plan.bpt == 1)
         return fast_diff ? k2_launch_main<1, true>(ctx, st, A) : k2_launch_main<1, false>(ctx, st, A);
@@ -2282,7 +2464,7 @@ int k2_batch_add(pbt_ctx *ctx, cudaStream_t st, K2Batch &B, int64_t o0, int64_t 
     K2Flags *flags = (K2Flags *)B.flags;
     K2Setup S;
     PBT_TRY(k2_prepare(ctx, st, no, d_beam, h_beam_off, d_ext, h_ext_off, d_verts, nverts, h_face_off,
-                       d_face_off, d_face_vi, nfaces, lambda, fast_diff, B.plan.variant, flags, S));
+                       d_face_off, d_face_vi, nfaces, lambda, fast_diff, B.plan, flags, S));
     const double waveno = 2.0 * kPiRef / lambda;
     const double *phitab = g.phitab.as<double>(), *cth = g.thtab.as<double>() + ntheta;
     const int64_t back_bin = 0 + nphi * g.back_i;
@@ -2374,7 +2556,7 @@ int k2_diff_main_impl(pbt_ctx *ctx, cudaStream_t st, const pbt_outbeam *d_beam, 
     K2Flags *flags = (K2Flags *)(base + o_flags);
     PBT_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(K2Flags), st));
     PBT_TRY(k2_prepare(ctx, st, 1, d_beam, hbo, d_ext, heo, d_verts, nverts, h_face_off, d_face_off,
-                       d_face_vi, nfaces, lambda, fast_diff, plan.variant, flags, S));
+                       d_face_vi, nfaces, lambda, fast_diff, plan, flags, S));
     PBT_TRY(k2_run_chunk(ctx, st, S, flags, 0, 1, nbeam + next, lambda, fast_diff, plan, ws, seg_rec,
                          (int64_t *)(base + o_it), (unsigned long long *)(base + o_cnt)));
     const double waveno = 2.0 * kPiRef / lambda;

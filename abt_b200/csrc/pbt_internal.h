@@ -89,7 +89,7 @@ constexpr size_t kIoChunk = (size_t)512 << 10;
 constexpr size_t kIoMin = (size_t)256 << 10;  // smaller results go to the driver as they are
 constexpr size_t kIoMinUp = (size_t)64 << 10; // smaller uploads too (from here on they wait for the stream there)
 constexpr size_t kIoPar = (size_t)1536 << 10; // copies from here on use several host threads
-constexpr int kIoRent = 8;                    // large copies of a context before it pins them
+constexpr int kIoRent = 24;                   // large copies of a context before it pins them
 
 // ------------------------------------------- reference-exact FP64 records
 // One outgoing facet, prepared for the FP64 kernel (all values formed in the

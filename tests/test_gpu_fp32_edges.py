@@ -159,3 +159,54 @@ def test_many_orientations(ctx, norient, nt, nphi, corners, scaling):
         # the parameters but the back-scattering one (a single bin's M11, under the Mueller bar)
         cols = [c for c in range(18) if c != 9]
         np.testing.assert_allclose(u[:, cols], v[:, cols], rtol=1e-5, atol=1e-5)
+
+
+def _polygon_mesh(rng, nv):
+    verts, faces = [], []
+    for n in nv:
+        e = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        ang = 2 * np.pi * (np.arange(n) + rng.uniform(0, 0.5, size=n)) / n
+        faces.append(list(range(len(verts) + 1, len(verts) + n + 1)))
+        verts += list(rng.uniform(-4, 4, size=3) + np.cos(ang)[:, None] * e[0] + np.sin(ang)[:, None] * e[1])
+    return abt_b200.make_geometry(np.array(verts), faces)
+
+
+@pytest.mark.parametrize("nv", [[4] * 30, [16] * 30, [3, 5] * 15, [3] * 25 + [16] * 5, [3] * 29 + [4],
+                                list(range(3, 17)) * 2 + [3, 3], [3] * 29 + [40]])
+@pytest.mark.parametrize("counts", [(1, 2), (57, 58), (130, 31)])
+@pytest.mark.parametrize("fast", [False, True])
+def test_polygon_records(ctx, nv, counts, fast):
+    """Facets of 3 to 16 vertices as one record each or as fans, neighbours of unequal length,
+    lists that begin and end within a pair and a stage (a face of 40 vertices that no outbeam
+    uses beside them): 2e-5 of the largest amplitude of the FP64 drop-in, off the forward row
+    (facets of radius 1, FP32 phases near 25 rad)."""
+    rng = np.random.default_rng(len(nv) + sum(counts))
+    geo = _polygon_mesh(rng, nv)
+    usable = np.nonzero(np.asarray(nv) <= 16)[0] + 1
+    beam, ext = outbeams(counts[0], rng, 1), outbeams(counts[1], rng, 1, prop=(0, 0, -1))
+    for ob in (beam, ext):
+        ob["fi"] = rng.choice(usable, size=len(ob))
+    th = np.linspace(4.0, 180.0, 23) * abt_b200.PI_REF / 180.0
+    ph = (0.3 + np.arange(35) * 360.0 / 35) * abt_b200.PI_REF / 180.0
+    ref = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=fast, precision="fp64")
+    for rpi in (None, 33):
+        if rpi:
+            ctx.set_plan(1, 1, rpi)
+        got = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=fast, precision="fp32")
+        ctx.set_plan(-1)
+        for g, r in zip(got, ref):
+            assert rel_err(g, r) <= 2e-5
+            if fast:
+                assert np.array_equal(g == 0, r == 0)
+
+
+def test_too_many_vertices(ctx):
+    """A face above 16 vertices is refused in FP32 when an outbeam uses it."""
+    rng = np.random.default_rng(1)
+    th, ph = _grid(9, 8)
+    for nv in ([4, 4, 17], [3] * 20 + [17]):
+        geo = _polygon_mesh(rng, nv)
+        ob = outbeams(3, rng, 1)
+        ob["fi"] = len(nv)
+        with pytest.raises(abt_b200.PbtError):
+            ctx.diff_main(ob, None, geo, th, ph, LAM, precision="fp32")
