@@ -23,11 +23,11 @@
 //   contour itself, so both agree to 1e-11 everywhere.  Facets with a clamped
 //   edge slope (:379-382) always take it.
 // * The polarisation block (karczewski :124-198 and the scattering-plane
-//   rotation :628-658) reduces, away from the forward bodge and the clamp of
-//   ky, to A = sc (P d + Q e), B = sc (P e - Q d) with d = -(Kz t + kz), e = -kx ky,
+//   rotation :628-658) reduces, away from the clamp of ky, to A = sc (P d + Q e), B = sc (P e - Q d) with d = -(Kz t + kz), e = -kx ky,
 //   t = kx^2 + kz^2, h = (b, -a, 0) the incidence direction times the unit
 //   direction (a, b, c) from the facet, P = y . h, Q = y_z |h|^2 - c (y_x a + y_y b)
-//   (y the aperture frame's second axis) and sc = 1 / (2 |h| t).
+//   (y the aperture frame's second axis) and sc = 1 / (2 |h| t); in the forward bodge
+//   (:630-633) with h from another bin, not normal to (a, b, c).
 // * [[A, B], [-B, A]] is diagonal in the columns' circular basis u+- = a1 +- i a2,
 //   in which the sums are kept; the basis change and the rotation T(phi), which
 //   depends on the bin alone, are applied once at the end.
@@ -286,16 +286,33 @@ __global__ void __launch_bounds__(K1_THREADS, K1_MINB) k1_kernel(const K1Args P)
             const double kx = x3 * ir, ky = y3 * ir, kz = z3 * ir;
             const double a = x1 * ir, b = y1 * ir, c = z1 * ir;
             double A, B;
-            if (fabs(c) < kLit0_999 - 1e-9 && fabs(ky) < kLit0_999999) {
-                const double hn2 = fma(a, a, b * b), tt = fma(kx, kx, kz * kz);
-                const double Pp = fma(R3, b, -(R4 * a));
-                const double Q = fma(R5, hn2, -(c * fma(R4, b, R3 * a)));
+            const double fc = fabs(c);
+            // the reference's roundings decide next to the bodge's limit (:630)
+            if (fabs(fc - kLit0_999) > 1e-9 && fabs(ky) < kLit0_999999) {
+                const double tt = fma(kx, kx, kz * kz);
+                double hn2, Pp, Q;
+                if (fc < kLit0_999) {
+                    hn2 = fma(a, a, b * b);
+                    Pp = fma(R3, b, -(R4 * a));
+                    Q = fma(R5, hn2, -(c * fma(R4, b, R3 * a)));
+                } else {
+                    // forward bodge: h = (p, q, 0) from the bin at the same phi and theta
+                    // index theta_i, no longer normal to k:
+                    // P = y . h - ky (h . k), Q = -y . (k x h)
+                    const int64_t oh = i + P.nphi * P.theta_i;
+                    const double xh = P.xyz[oh] - v0.x, yh = P.xyz[nb + oh] - v0.y,
+                                 zh = P.xyz[2 * nb + oh] - v1.x;
+                    const double ih = rsqrt_n(fma(zh, zh, fma(yh, yh, xh * xh)));
+                    const double p = yh * ih, q = -(xh * ih);
+                    hn2 = fma(p, p, q * q);
+                    Pp = fma(R4, q, R3 * p) - ky * fma(q, b, p * a);
+                    Q = fma(c, fma(R3, q, -(R4 * p)), -(R5 * fma(a, q, -(b * p))));
+                }
                 const double d = -fma(v7.x, tt, kz), e = -(kx * ky);
                 const double sc = 0.5 * rsqrt_n((hn2 * tt) * tt);
                 A = sc * fma(Pp, d, Q * e);
                 B = sc * fma(Pp, e, -(Q * d));
             } else {
-                // forward bodge: the bin at the same phi and theta index theta_i
                 const int64_t oh = i + P.nphi * P.theta_i;
                 const double xh = P.xyz[oh] - F->com[0], yh = P.xyz[nb + oh] - F->com[1],
                              zh = P.xyz[2 * nb + oh] - F->com[2];

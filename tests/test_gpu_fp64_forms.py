@@ -83,3 +83,17 @@ def test_clamped_slopes(ctx):
     geo = abt_b200.make_geometry(v, [[1, 2, 3], [4, 6, 5]])
     beam = outbeams(4, rng, 2, prop=(np.sin(0.4), 0.0, -np.cos(0.4)))
     _check(ctx, geo, beam, beam[:0], *_grid(lo=5.0), 0.532)
+
+
+@pytest.mark.parametrize("lo,hi", [(0.0, 3.2), (1.0, 2.6), (176.8, 180.0)])
+def test_forward_bodge(ctx, lo, hi):
+    """Rows on both sides of the forward bodge's limit, acos(0.999) = 2.56 degrees from the
+    incidence axis, in both hemispheres, and the rows at the axis itself."""
+    rng = np.random.default_rng(31)
+    geo, _, _ = W.synthetic_beam_list(n_beams=1, facets_per_beam=6, seed=9, cube=4.0)
+    th = np.linspace(lo, hi, 33) * abt_b200.PI_REF / 180.0
+    ph = (0.3 + np.arange(7) * 51.0) * abt_b200.PI_REF / 180.0
+    tilt = (np.sin(0.3), 0.0, -np.cos(0.3))
+    for sign in (1, -1):
+        prop = tuple(sign * x for x in tilt)
+        _check(ctx, geo, outbeams(5, rng, 6, prop=prop), outbeams(3, rng, 6, prop=prop), th, ph, 0.532)
