@@ -938,12 +938,15 @@ __global__ void __launch_bounds__(K2_THREADS, 2) k2_main_kernel(K2MainArgs P) {
 // Bound: issue.  Over the pair loop the FMA pipe's cycles (an FFMA2 holds it two)
 // and the other instructions add up to 88 % of the cycles, at 16 and 20 warps per SM
 // alike, so only fewer operations help.  200,000 triangles x 259,560 bins take
-// 217.9 ms: 244.8 before the lab-frame normal (no R s + R e, no h in the aperture
+// 213.0 ms: 244.8 before the lab-frame normal (no R s + R e, no h in the aperture
 // frame; 227.8), the sinc series formed by every lane instead of behind a vote
-// (224.1), and the fixed-point phase with the item's state and sums in shared memory
-// (217.9; with CTA barriers between the stages or the sums in registers 224-226, five
-// CTAs per SM with 96 registers 228).  One operation less in the second-order terms
-// ((u - eps) opa2, no 1 + al) came out of the compiler slower, 221.7 ms.
+// (224.1), the fixed-point phase with the item's state and sums in shared memory
+// (215.9; with CTA barriers between the stages or the sums in registers 224-226, five
+// CTAs per SM with 96 registers 228), and the steps of their own for warps away from
+// the incidence axis, at it, and on the clamp of ky (213.0; 24 lists of 3,300 facets
+// within 13 um x 64,980 bins 22.0 -> 21.1 ms, 1 % of it by Near, 2 % by the Pole step
+// in place of Full).  One operation less in the second-order terms ((u - eps) opa2, no
+// 1 + al) came out of the compiler slower, 221.7 ms.
 
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 // the special-function unit's approximations with subnormal inputs flushed
@@ -1091,10 +1094,21 @@ __device__ __forceinline__ void ld22(const float2 *p, float2 &a, float2 &b) {
     b = make_float2(v.z, v.w);
 }
 
-// GENERAL: the step with its rare branch (poles, forward bodge, clamp of ky).  Otherwise
-// the main step alone, which lowers tmin to the smallest kx^2 + kz^2: at or below the
-// clamp's the caller takes the general step instead.  WIDE: far-field phases of any size.
-template <bool FAST, bool GENERAL, bool WIDE, class PairT>
+// How far a launch's facet centres lie from the origin.  Near: |com| / R up to 2^-14
+// (61 um); the second order of the direction from a facet centre, below 1.5 |com|^2 / R^2
+// = 5.6e-9, is then under a tenth of FP32's half ulp and left out.  Wide: half phases
+// k |com| / 2 from 2^18 pi on, beyond the fixed-point form of the far-field phase.
+enum class Reach { Near, Mid, Wide };
+__device__ __forceinline__ Reach k2_reach(float epsmax, float turns) {
+    if (!(turns * epsmax < 262144.0f)) return Reach::Wide;
+    return epsmax <= 6.1035156e-5f ? Reach::Near : Reach::Mid;
+}
+
+// Main: the step without the forward bodge and the clamp of ky; Pole: with the bodge, for
+// warps with a bin near the incidence axis; both lower tmin to the smallest kx^2 + kz^2:
+// at or below the clamp's the caller takes the Full step, with a branch for either.
+enum class Step { Main, Pole, Full };
+template <bool FAST, Step STEP, Reach REACH, class PairT>
 __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const BinPk &B,
                                         float2 (&acc)[8], float2 hkRh, float &tmin,
                                         const float4 &hb, bool lo_ok, bool hi_ok,
@@ -1103,14 +1117,14 @@ __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const B
     // far-field half phase per facet, k u.c / 2 modulo pi, as a fixed-point fraction of
     // pi (2^-32 units): added to 1.5 * 2^20 the FP64 sum's low word is that fraction, so
     // the reduction costs no operation of its own (each of the three steps rounds to
-    // 2^-32 pi = 7e-10 rad).  That holds up to 2^19 half turns; records beyond (WIDE, a
-    // launch with k |com| above 1.6e6) subtract the nearest integer.
+    // 2^-32 pi = 7e-10 rad).  That holds up to 2^19 half turns; records beyond (Wide)
+    // subtract the nearest integer.
     float2 fr;
     {
         const double2 k0 = *reinterpret_cast<const double2 *>(&P.kc[0][0]);
         const double2 k1 = *reinterpret_cast<const double2 *>(&P.kc[1][0]);
         const double2 k2 = *reinterpret_cast<const double2 *>(&P.kc[2][0]);
-        if (!WIDE) {
+        if (REACH != Reach::Wide) {
             fr.x = (float)__double2loint(fma(B.uz, k2.x, fma(B.uy, k1.x, fma(B.ux, k0.x, kFracMagic))));
             fr.y = (float)__double2loint(fma(B.uz, k2.y, fma(B.uy, k1.y, fma(B.ux, k0.y, kFracMagic))));
         } else {
@@ -1125,21 +1139,28 @@ __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const B
     ld22(&P.eps[0], eps0, eps1);
     ld22(&P.eps[2], eps2, pb);
     const float2 al = fma2(B.fz, eps2, fma2(B.fy, eps1, mul2(B.fx, eps0)));  // u . eps
-    // with y = b - al^2: half phase hkRh y (1 + al) - pi 2^-32 fr, and
-    // opa2 = 1 + al + 1.5 al^2 - 0.5 b = (1 + al) - 0.5 y + al^2
+    // with y = b - al^2: half phase hkRh y (1 + al) - pi 2^-32 fr
     const float2 opa = add2(one, al);
     const float2 y = fma2(neg2(al), al, pb);
     const float2 ph = fma2(fr, bc2((float)(-kPi / 4294967296.0)), mul2(mul2(hkRh, y), opa));
     const float2 opa2 = fma2(al, al, fma2(bc2(-0.5f), y, opa));
     // The unit direction from the facet centre in the lab frame, (a, b, c) = u opa2 -
-    // eps opa, and k = R (a, b, c) in the aperture frame.  The normal of the
+    // eps opa with opa2 = 1 + al + 1.5 al^2 - 0.5 b = (1 + al) - 0.5 y + al^2, or u opa -
+    // eps for Near, and k = R (a, b, c) in the aperture frame.  The normal of the
     // scattering plane, h = inc x k with inc = (0, 0, -1), is (b, -a, 0): formed from
     // the lab components it has no cancellation of nearly parallel unit vectors near
     // the forward and backward directions, where a and b are small and known to full
     // FP32 precision.
-    const float2 a = fma2(B.fx, opa2, neg2(mul2(eps0, opa)));
-    const float2 b = fma2(B.fy, opa2, neg2(mul2(eps1, opa)));
-    const float2 c = fma2(B.fz, opa2, neg2(mul2(eps2, opa)));
+    float2 a, b, c;
+    if (REACH == Reach::Near) {
+        a = fma2(B.fx, opa, neg2(eps0));
+        b = fma2(B.fy, opa, neg2(eps1));
+        c = fma2(B.fz, opa, neg2(eps2));
+    } else {
+        a = fma2(B.fx, opa2, neg2(mul2(eps0, opa)));
+        b = fma2(B.fy, opa2, neg2(mul2(eps1, opa)));
+        c = fma2(B.fz, opa2, neg2(mul2(eps2, opa)));
+    }
     float2 r3, r4, r5, nKx, kx, ky, kz, u;
     {
         float2 r0, r1, r2, r6, r7, r8;
@@ -1192,9 +1213,26 @@ __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const B
     float2 P1 = fma2(r3, b, neg2(mul2(r4, a)));
     float2 R1 = fma2(r5, hn2, neg2(mul2(c, u)));
     float2 kzc = P.kzc;
-    const bool cx = GENERAL && tr.x <= kOneMinusClampSq, cy = GENERAL && tr.y <= kOneMinusClampSq;
-    if (!GENERAL) tmin = fminf(tmin, fminf(tr.x, tr.y));
-    if (GENERAL && (B.pole || cx || cy)) {
+    constexpr bool FULL = STEP == Step::Full;
+    const bool cx = FULL && tr.x <= kOneMinusClampSq, cy = FULL && tr.y <= kOneMinusClampSq;
+    if (!FULL) tmin = fminf(tmin, fminf(tr.x, tr.y));
+    if (STEP == Step::Pole) {
+        // the forward bodge (src/diff_mod.f90:630-633): h = (bb, -ba, 0) from the direction
+        // (ba, bb, .) to the bodge's bin, no longer normal to k: P1 = y . h - ky (h . k),
+        // R1 = -y . (k x h)
+        const bool bx = !(fabsf(c.x) < 0.999f), by = !(fabsf(c.y) < 0.999f);
+        const float2 ux = bc2(hb.x), uy = bc2(hb.y), uz = bc2(hb.z);
+        const float2 ah = fma2(uz, eps2, fma2(uy, eps1, mul2(ux, eps0)));
+        const float2 oh = add2(one, ah);
+        const float2 oh2 = fma2(ah, fma2(bc2(1.5f), ah, one), fma2(bc2(-0.5f), pb, one));
+        const float2 ba = fma2(ux, oh2, neg2(mul2(eps0, oh)));
+        const float2 bb = fma2(uy, oh2, neg2(mul2(eps1, oh)));
+        const float2 hk = fma2(bb, a, neg2(mul2(ba, b)));
+        P1 = sel2(bx, by, fma2(r3, bb, neg2(fma2(r4, ba, mul2(ky, hk)))), P1);
+        R1 = sel2(bx, by, fma2(r5, fma2(a, ba, mul2(b, bb)), neg2(mul2(c, fma2(r4, bb, mul2(r3, ba))))), R1);
+        hn2 = sel2(bx, by, fma2(ba, ba, mul2(bb, bb)), hn2);
+    }
+    if (FULL && (B.pole || cx || cy)) {
         float2 r0, r1, r2, r6, r7, r8, q3, q4, q5, q9;
         ld22(&P.R[0], r0, r1);
         ld22(&P.R[2], r2, q3);
@@ -1350,6 +1388,13 @@ __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const B
     }
 }
 
+using MainC = std::integral_constant<Step, Step::Main>;
+using PoleC = std::integral_constant<Step, Step::Pole>;
+using FullC = std::integral_constant<Step, Step::Full>;
+using NearC = std::integral_constant<Reach, Reach::Near>;
+using MidC = std::integral_constant<Reach, Reach::Mid>;
+using WideC = std::integral_constant<Reach, Reach::Wide>;
+
 // Record pairs per shared-memory stage: 44 for the full sum (three stages, 44 KB,
 // four CTAs per SM); 32 with the field-of-view cull, whose per-stage keep masks are
 // two 32-bit ballot words of the stage's 64 records.
@@ -1444,7 +1489,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
     // bins with |uz| below pole_cos are out of reach of the forward bodge for every
     // record: |inc . k - (-uz)| <= 2 |com| / R for the direction k from a facet centre
     const float pole_cos = 0.999f - 2.0f * __uint_as_float(*P.epsmax) - 1e-5f;
-    const bool wide = !(P.turns * __uint_as_float(*P.epsmax) < 262144.0f);  // see k2_pair
+    const Reach reach = k2_reach(__uint_as_float(*P.epsmax), P.turns);
     for (;;) {
         auto after = [](int s, int n) { return s + n >= K2_NST ? s + n - K2_NST : s + n; };
         // chunk c of the item into its stage (s its index); thread 0 only
@@ -1523,12 +1568,10 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
         for (int q = 0; q < BPT; q++)
 #pragma unroll
             for (int c = 0; c < 8; c++) sum(q, c) = 0.0;
-        [[maybe_unused]] bool general = wide;
-        if constexpr (FAST) {
+        bool pole = false;
 #pragma unroll
-            for (int q = 0; q < BPT; q++) general = general || bd[q].pole;
-            general = __any_sync(0xffffffffu, general);
-        }
+        for (int q = 0; q < BPT; q++) pole = pole || bd[q].pole;
+        pole = __any_sync(0xffffffffu, pole);
         bool failed = false;
         for (int c = 0; c < I.nchunk; c++) {
             if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&full[st]), phase))) {
@@ -1601,8 +1644,9 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             // Without the field-of-view test every lane adds (the edge pairs are patched
             // above; a bin beyond nb is never written out).
             float tmin = 1.0f;
-            auto pairs = [&](auto general_, auto wide_) {
-                constexpr bool G = decltype(general_)::value, WD = decltype(wide_)::value;
+            auto pairs = [&](auto step_, auto reach_) {
+                constexpr Step ST = decltype(step_)::value;
+                constexpr Reach RE = decltype(reach_)::value;
 #pragma unroll
                 for (int q = 0; q < BPT; q++)
 #pragma unroll
@@ -1614,7 +1658,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                         const K2Fov *fv = P.fovs + 2 * (I.p0 + c * CH + j);
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<true, G, WD>(pair_at(st, j), fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
+                            k2_pair<true, ST, RE>(pair_at(st, j), fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
                                                  (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0,
                                                  P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
                     }
@@ -1622,30 +1666,24 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     for (int j = 0; j < n; j++)
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<false, G, WD>(pair_at(st, j), nullptr, bd[q], acc[q], hkRh, tmin,
+                            k2_pair<false, ST, RE>(pair_at(st, j), nullptr, bd[q], acc[q], hkRh, tmin,
                                                   s_hb[q][tid], true, true, P.xyz, P.nb,
                                                   P.rlo + (I.p0 + c * CH + j) * 3);
                 }
             };
-            if constexpr (FAST) {
-                // With the field-of-view test the main step goes without its rare branch: a
-                // warp with a bin near the poles takes the general loop (of any phase, too),
-                // and one that meets the clamp of ky (a 0.08 degree cone) does the chunk
-                // again: 13.25 -> 12.9 ms on 16 lists of 3,500 polygons.  The full sum gains
-                // nothing by it (216.1 against 216.5 ms; its main step alone, wrong at the
-                // poles, 210.2), and small grids, with more of their tiles at the poles,
-                // lose 1-3 %.
-                bool again = general;
-                if (!general) {
-                    pairs(std::false_type(), std::false_type());
-                    again = __any_sync(0xffffffffu, tmin <= kOneMinusClampSq);
-                }
-                if (again) pairs(std::true_type(), std::true_type());
-            } else if (wide) {
-                pairs(std::true_type(), std::true_type());
-            } else {
-                pairs(std::true_type(), std::false_type());
+            // A warp that meets the clamp of ky (a 0.08 degree cone around a facet's second
+            // axis) does the chunk again.
+            bool again = reach == Reach::Wide;
+            if (!again) {
+                if (pole)
+                    pairs(PoleC(), MidC());
+                else if (reach == Reach::Near)
+                    pairs(MainC(), NearC());
+                else
+                    pairs(MainC(), MidC());
+                again = __any_sync(0xffffffffu, tmin <= kOneMinusClampSq);
             }
+            if (again) pairs(FullC(), WideC());
 #pragma unroll
             for (int q = 0; q < BPT; q++)
 #pragma unroll

@@ -210,3 +210,25 @@ def test_too_many_vertices(ctx):
         ob["fi"] = len(nv)
         with pytest.raises(abt_b200.PbtError):
             ctx.diff_main(ob, None, geo, th, ph, LAM, precision="fp32")
+
+
+@pytest.mark.parametrize("offset", [0.0, 55.0, 68.0, 160.0])
+@pytest.mark.parametrize("rows", [(0.1, 3.2), (176.8, 179.9), (20.0, 160.0)])
+@pytest.mark.parametrize("corners", [3, 5])
+@pytest.mark.parametrize("fast", [False, True])
+def test_reach_and_poles(ctx, offset, rows, corners, fast):
+    """Facet centres within 61 um of the origin (the step without the direction's second order)
+    and beyond, in rows around the forward bodge's limit (2.56 degrees from the axis) and away
+    from it: 2e-5 of the largest amplitude of the FP64 drop-in (20 facets of radius 1)."""
+    rng = np.random.default_rng(int(offset) + corners)
+    geo = _polygon_mesh(rng, [corners] * 20)
+    geo["verts"] = np.asfortranarray(geo["verts"] + offset / np.sqrt(3.0) * np.array([1.0, -1.0, 1.0]))
+    beam, ext = outbeams(35, rng, 20), outbeams(18, rng, 20, prop=(np.sin(0.3), 0, -np.cos(0.3)))
+    th = np.linspace(*rows, 23) * abt_b200.PI_REF / 180.0
+    ph = (0.3 + np.arange(35) * 360.0 / 35) * abt_b200.PI_REF / 180.0
+    got = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=fast, precision="fp32")
+    ref = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=fast, precision="fp64")
+    for g, r in zip(got, ref):
+        assert rel_err(g, r) <= 2e-5
+        if fast:
+            assert np.array_equal(g == 0, r == 0)
