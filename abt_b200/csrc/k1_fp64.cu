@@ -23,8 +23,8 @@
 //   contour itself, so both agree to 1e-11 everywhere.  Facets with a clamped
 //   edge slope (:379-382) always take it.
 // * The polarisation block (karczewski :124-198 and the scattering-plane
-//   rotation :628-658) reduces, away from the clamp of ky, to A = sc (P d + Q e), B = sc (P e - Q d) with d = -(Kz t + kz), e = -kx ky,
-//   t = kx^2 + kz^2, h = (b, -a, 0) the incidence direction times the unit
+//   rotation :628-658) reduces, away from the clamp of ky, to A = sc (P d + Q e),
+//   B = sc (P e - Q d) with d = -(Kz t + kz), e = -kx ky, t = kx^2 + kz^2, h = (b, -a, 0) the incidence direction times the unit
 //   direction (a, b, c) from the facet, P = y . h, Q = y_z |h|^2 - c (y_x a + y_y b)
 //   (y the aperture frame's second axis) and sc = 1 / (2 |h| t); in the forward bodge
 //   (:630-633) with h from another bin, not normal to (a, b, c).
@@ -34,11 +34,12 @@
 //
 // Bound: FP64 pipe (65 % of cycles; 360 instructions a triangle and bin, 196 of them
 // FP64, against 1,813 with every operation of the reference).  A triangle list of
-// 2,582 x 32,580 bins takes 1.51 ms (5.6e10 facet-bin/s), the operation-by-operation
+// 2,582 x 32,580 bins takes 1.42 ms (5.9e10 facet-bin/s), the operation-by-operation
 // kernel took 6.92 ms (1.59 ms with quadrant polynomials in place of the table of
-// roots).  The facet records go through shared memory, three stages of 16 and one
-// barrier a stage: read from global memory they cost 38 % of the issue slots in load
-// waits; a private stage per warp, without barriers, measured 3 % slower.
+// roots, 1.51 ms with the forward bodge in the aperture frame).  The facet records go
+// through shared memory, three stages of 16 and one barrier a stage: read from global
+// memory they cost 38 % of the issue slots in load waits; a private stage per warp,
+// without barriers, measured 3 % slower.
 //
 // The file is built with -fmad=false: a multiply-add is fused only where fma()
 // is written.  Facet frames come from the host (host_setup.cpp); the bin grid
@@ -457,8 +458,8 @@ int k1_launch(pbt_ctx *ctx, cudaStream_t st, const K1Facet *d_fac, int64_t n0, i
     // runs of at least 16 over blockIdx.y (at most 64 runs a list), both lists in one
     // launch, each run into a partial grid of its own.  They are summed in run order, so
     // the result is deterministic; it differs from the one-run order by rounding.
-    // Measured on 1,700 + 882 triangles x 32,580 bins: 5 waves 2.57 ms, 8 waves 2.36,
-    // 16 waves 2.10 (four CTAs an SM); 16 waves 1.66, 24 waves 1.62, 40 waves 1.59 (five).
+    // Measured on 1,700 + 882 triangles x 32,580 bins: 10 waves 1.48 ms, 14 1.45, 18 1.43,
+    // 24 1.42, 32 1.41 with the sum of the partial grids, which takes 37 us of it.
     const int64_t resident = (int64_t)ctx->sm_count * K1_MINB;
     const int64_t all = std::max<int64_t>(n0 + n1, 1);
     const int64_t runs = (K1_WAVES * resident + blocks - 1) / blocks;

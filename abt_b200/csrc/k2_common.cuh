@@ -29,16 +29,21 @@ static_assert(sizeof(K2Rec) == 176, "K2Rec must be 176 bytes");
 // Per-record field-of-view test data (is_fast_diff only): prop0 and cos(fov)
 // for the per-bin test; fovm = fov + a parallax margin with its cosine and
 // sine for the per-tile cull (a tile whose cone lies beyond fovm is skipped).
-// When the FP32 per-bin test is within tol of the threshold the FP64 test of
-// the reference (facet centre com, prop0, cos(fov)) decides, with the same
-// rounding as the FP64 drop-in.
 struct __align__(16) K2Fov {
     float p0[3];
     float cos_fov;
     float cos_fovm, sin_fovm, fovm, tol;
-    double com[3], p0d[3], cos_fovd, pad;
 };
-static_assert(sizeof(K2Fov) == 96, "K2Fov must be 96 bytes");
+static_assert(sizeof(K2Fov) == 32, "K2Fov must be 32 bytes");
+
+// When the FP32 per-bin test is within tol of the threshold the FP64 test of
+// the reference (facet centre com, prop0, cos(fov)) decides, with the same
+// rounding as the FP64 drop-in.  An array of its own: the sum reads it in few bins, and
+// the 32 bytes of K2Fov for every one.
+struct __align__(16) K2FovExact {
+    double com[3], p0[3], cos_fov, pad;
+};
+static_assert(sizeof(K2FovExact) == 64, "K2FovExact must be 64 bytes");
 
 // Cone of a bin tile (is_fast_diff only): unit centre direction and the
 // largest angle psi of a tile bin from it.

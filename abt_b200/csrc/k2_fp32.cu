@@ -68,7 +68,7 @@ struct BinDev {
 
 // The field-of-view test of the FP64 drop-in for bin `bin` (src/diff_mod.f90:593-603):
 // x1 = X - com, dot(x1/r1, prop0) >= cos(fov), each operation rounded once.
-__device__ __forceinline__ bool fov_exact(const K2Fov &f, const double *__restrict__ xyz, int64_t nb,
+__device__ __forceinline__ bool fov_exact(const K2FovExact &f, const double *__restrict__ xyz, int64_t nb,
                                        int64_t bin) {
     const double x1 = __dadd_rn(xyz[bin], -f.com[0]);
     const double y1 = __dadd_rn(xyz[nb + bin], -f.com[1]);
@@ -76,9 +76,9 @@ __device__ __forceinline__ bool fov_exact(const K2Fov &f, const double *__restri
     const double r1 =
         __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x1, x1), __dmul_rn(y1, y1)), __dmul_rn(z1, z1)));
     const double v0 = __ddiv_rn(x1, r1), v1 = __ddiv_rn(y1, r1), v2 = __ddiv_rn(z1, r1);
-    const double d = __dadd_rn(__dadd_rn(__dmul_rn(v0, f.p0d[0]), __dmul_rn(v1, f.p0d[1])),
-                               __dmul_rn(v2, f.p0d[2]));
-    return !(d < f.cos_fovd);
+    const double d = __dadd_rn(__dadd_rn(__dmul_rn(v0, f.p0[0]), __dmul_rn(v1, f.p0[1])),
+                               __dmul_rn(v2, f.p0[2]));
+    return !(d < f.cos_fov);
 }
 
 // ---------------------------------------------------------------- set-up
@@ -172,8 +172,8 @@ __device__ __forceinline__ void store_pair_half(K2Pair *pairs, int64_t r, const 
 }
 
 // A record's field-of-view data: prop0, fov and the facet centre.
-__device__ __forceinline__ K2Fov make_fov(const double *prop0, double fov, const double *com) {
-    K2Fov fv;
+__device__ __forceinline__ void make_fov(const double *prop0, double fov, const double *com, K2Fov &fv,
+                                         K2FovExact &fx) {
     fv.p0[0] = (float)prop0[0];
     fv.p0[1] = (float)prop0[1];
     fv.p0[2] = (float)prop0[2];
@@ -190,20 +190,20 @@ __device__ __forceinline__ K2Fov make_fov(const double *prop0, double fov, const
     const double e2 = (cn / kFarR) * (cn / kFarR);
     fv.tol = (float)(3.0 * e2 + 8e-7);
     for (int c = 0; c < 3; c++) {
-        fv.com[c] = com[c];
-        fv.p0d[c] = prop0[c];
+        fx.com[c] = com[c];
+        fx.p0[c] = prop0[c];
     }
-    fv.cos_fovd = cos(fov);
-    fv.pad = 0.0;
-    return fv;
+    fx.cos_fov = cos(fov);
+    fx.pad = 0.0;
 }
 
 __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restrict__ verts,
                                 int64_t nverts, const int64_t *__restrict__ face_off,
                                 int64_t nfaces, const int64_t *__restrict__ face_vi, double waveno, double lambda, int fast_diff,
                                 K2Rec *__restrict__ recs, K2Pair *__restrict__ pairs,
-                                K2Fov *__restrict__ fovs, float2 *__restrict__ rlo,
-                                int *__restrict__ err, unsigned *__restrict__ epsmax) {
+                                K2Fov *__restrict__ fovs, K2FovExact *__restrict__ fovx,
+                                float2 *__restrict__ rlo, int *__restrict__ err,
+                                unsigned *__restrict__ epsmax) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nrefs) return;
     int64_t o;
@@ -226,7 +226,10 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
                     float2 &l = rlo[(r >> 1) * 3 + i];
                     (r & 1 ? l.y : l.x) = 0.0f;
                 }
-                if (fast_diff) fovs[r] = K2Fov{};
+                if (fast_diff) {
+                    fovs[r] = K2Fov{};
+                    fovx[r] = K2FovExact{};
+                }
             }
         }
         return;
@@ -325,7 +328,7 @@ __global__ void k2_setup_kernel(RefSrc S, int64_t nrefs, const double *__restric
             recs[r0 + t] = rec;
         }
         if (fast_diff) {
-            fovs[r0 + t] = make_fov(prop0, kind ? kPiRef / 2.0 : ob->fov, fr.com);
+            make_fov(prop0, kind ? kPiRef / 2.0 : ob->fov, fr.com, fovs[r0 + t], fovx[r0 + t]);
         }
     }
 }
@@ -336,7 +339,8 @@ __global__ void k2_setup_poly_kernel(RefSrc S, int64_t nrefs, const double *__re
                                      int64_t nverts, const int64_t *__restrict__ face_off,
                                      int64_t nfaces, const int64_t *__restrict__ face_vi, double waveno,
                                      double lambda, int fast_diff, int nvmax, char *__restrict__ polys,
-                                     int64_t stride, K2Fov *__restrict__ fovs, float2 *__restrict__ rlo,
+                                     int64_t stride, K2Fov *__restrict__ fovs,
+                                     K2FovExact *__restrict__ fovx, float2 *__restrict__ rlo,
                                      int *__restrict__ err, unsigned *__restrict__ epsmax) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nrefs) return;
@@ -432,7 +436,7 @@ __global__ void k2_setup_poly_kernel(RefSrc S, int64_t nrefs, const double *__re
         xp = x;
         yp = y;
     }
-    if (fast_diff) fovs[g] = make_fov(ob->prop_out, kind ? kPiRef / 2.0 : ob->fov, com);
+    if (fast_diff) make_fov(ob->prop_out, kind ? kPiRef / 2.0 : ob->fov, com, fovs[g], fovx[g]);
 }
 
 // Per orientation chunk [o0, o0+no): segment records and work-item prefix (block 0, a
@@ -548,13 +552,19 @@ __device__ __forceinline__ uint64_t gtimer() {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
         "l"(src), "r"(bytes), "r"(bar)
         : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    mbar_expect(bar, bytes);
+    bulk_copy(dst, src, bytes, bar);
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -638,6 +648,7 @@ __device__ __forceinline__ void ordered_add(double *__restrict__ out, int64_t nb
 struct K2MainArgs {
     const K2Rec *recs;
     const K2Fov *fovs;
+    const K2FovExact *fovx;
     const float2 *rlo;  // R_1 - (float)R_1, pair layout (3 per pair)
     const int64_t *seg_rec;
     const int64_t *item_pre;
@@ -669,7 +680,8 @@ __device__ __forceinline__ float clamp_v(float hi, float lo, double u, float sig
 }
 
 template <int BPT, bool FAST>
-__device__ __forceinline__ void k2_record(const K2Rec &r, const K2Fov *fv, const BinDev (&bd)[BPT],
+__device__ __forceinline__ void k2_record(const K2Rec &r, const K2Fov *fv, const K2FovExact *fx,
+                                          const BinDev (&bd)[BPT],
                                           const bool (&valid)[BPT], float (&acc)[BPT][8], float k,
                                           float hkR, float sgh, const double *__restrict__ xyz,
                                           int64_t nb, const float2 *__restrict__ rl, int half) {
@@ -709,7 +721,7 @@ __device__ __forceinline__ void k2_record(const K2Rec &r, const K2Fov *fv, const
             const float dz = fmaf(B.fz, opa, -r.eps[2]);
             const float dp = fmaf(dz, fv->p0[2], fmaf(dy, fv->p0[1], dx * fv->p0[0]));
             bool in = !(dp < fv->cos_fov);
-            if (use && fabsf(dp - fv->cos_fov) < fv->tol) in = fov_exact(*fv, xyz, nb, B.bin);
+            if (use && fabsf(dp - fv->cos_fov) < fv->tol) in = fov_exact(*fx, xyz, nb, B.bin);
             use = use && in;
         }
         // aperture integral
@@ -893,7 +905,8 @@ __global__ void __launch_bounds__(K2_THREADS, 2) k2_main_kernel(K2MainArgs P) {
             const K2Fov *fv = FAST ? P.fovs + rbeg + c * K2_CH : nullptr;
             for (int j = 0; j < n; j++) {
                 const int64_t ri = rbeg + c * K2_CH + j;
-                k2_record<BPT, FAST>(sbuf[st][j], FAST ? fv + j : nullptr, bd, valid, acc, P.k,
+                k2_record<BPT, FAST>(sbuf[st][j], FAST ? fv + j : nullptr,
+                                     FAST ? P.fovx + ri : nullptr, bd, valid, acc, P.k,
                                      P.hkR, P.sgh, P.xyz, P.nb, P.rlo + (ri >> 1) * 3, (int)(ri & 1));
             }
 #pragma unroll
@@ -1109,7 +1122,7 @@ __device__ __forceinline__ Reach k2_reach(float epsmax, float turns) {
 // at or below the clamp's the caller takes the Full step, with a branch for either.
 enum class Step { Main, Pole, Full };
 template <bool FAST, Step STEP, Reach REACH, class PairT>
-__device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const BinPk &B,
+__device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const K2FovExact *fx, const BinPk &B,
                                         float2 (&acc)[8], float2 hkRh, float &tmin,
                                         const float4 &hb, bool lo_ok, bool hi_ok,
                                         const double *__restrict__ xyz, int64_t nb,
@@ -1365,8 +1378,8 @@ __device__ __forceinline__ void k2_pair(const PairT &P, const K2Fov *fv, const B
         const float dpx = fmaf(c.x, fa.p0[2], fmaf(b.x, fa.p0[1], a.x * fa.p0[0]));
         const float dpy = fmaf(c.y, fb.p0[2], fmaf(b.y, fb.p0[1], a.y * fb.p0[0]));
         bool in_x = !(dpx < fa.cos_fov), in_y = !(dpy < fb.cos_fov);
-        if (ok_x && fabsf(dpx - fa.cos_fov) < fa.tol) in_x = fov_exact(fa, xyz, nb, B.bin);
-        if (ok_y && fabsf(dpy - fb.cos_fov) < fb.tol) in_y = fov_exact(fb, xyz, nb, B.bin);
+        if (ok_x && fabsf(dpx - fa.cos_fov) < fa.tol) in_x = fov_exact(fx[0], xyz, nb, B.bin);
+        if (ok_y && fabsf(dpy - fb.cos_fov) < fb.tol) in_y = fov_exact(fx[1], xyz, nb, B.bin);
         ok_x = ok_x && in_x;
         ok_y = ok_y && in_y;
     }
@@ -1399,7 +1412,8 @@ using WideC = std::integral_constant<Reach, Reach::Wide>;
 // four CTAs per SM); 32 with the field-of-view cull, whose per-stage keep masks are
 // two 32-bit ballot words of the stage's 64 records.
 constexpr int K2P_CH_FULL = 44, K2P_CH_FOV = 32;
-constexpr int kPolyStage = 44 * 288;  // bytes a stage of polygons: 29 pairs of up to 6 vertices
+// bytes a stage of polygons: 29 pairs of up to 6 vertices, 24 beside the field-of-view data
+constexpr int poly_stage(bool fast) { return (fast ? 37 : 44) * 288; }
 
 // The record's per-bin test passes no bin of the tile when the angle between
 // prop0 and the tile centre exceeds fovm + psi (fovm includes the parallax
@@ -1416,6 +1430,7 @@ struct K2PkArgs {
     const char *polys;  // polygons: K2Poly and vertices, stride bytes a pair
     int stride, chunk;  // and pairs per shared-memory stage
     const K2Fov *fovs;
+    const K2FovExact *fovx;
     const int *perm;        // is_fast_diff: tile-major bin order (-1: padding)
     const K2Cone *cones;    // is_fast_diff: cone of each warp's 32 bins
     const int64_t *seg_rec;
@@ -1442,21 +1457,26 @@ struct K2PkArgs {
 // chunks.
 // With the field-of-view test each warp culls the stage's records against the cone of
 // its own 4 x 8 bins (13.3 ms; 14.9 with one 8 x 16 cone for the CTA, on 16 lists of
-// 3,500 polygons x 64,979 bins).
+// 3,500 polygons x 64,979 bins).  The records' field-of-view data come through the
+// stages too and the warp's cones lie in shared memory: read from global memory they held
+// 2.0 of the 7.7 stalled cycles an issue (200,000 triangles x 259,560 bins, 13 % of the
+// pairs kept: 49.0 -> 45.6 ms).
 // POLY: facets of up to 16 vertices as one record each (K2Poly): the direction, the
 // polarisation block and the phase once a facet, a divided difference for each triangle
-// of its fan.  16 lists of 3,500 facets of 3-6 vertices with the field-of-view test: 9.85
-// ms against 12.75 as fans.
+// of its fan.  16 lists of 3,500 facets of 3-6 vertices with the field-of-view test: 9.64
+// ms, 12.75 as fans (measured at 9.85).
 template <int BPT, bool FAST, bool POLY>
 __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kernel(K2PkArgs P) {
     using PairT = std::conditional_t<POLY, K2Poly, K2Pair>;
     constexpr int CHT = FAST ? K2P_CH_FOV : K2P_CH_FULL;
     const int CH = POLY ? P.chunk : CHT;
     constexpr int NW = K2_THREADS / 32;
-    __shared__ __align__(128) char sbuf[K2_NST][POLY ? kPolyStage : CHT * sizeof(K2Pair)];
+    __shared__ __align__(128) char sbuf[K2_NST][POLY ? poly_stage(FAST) : CHT * sizeof(K2Pair)];
+    __shared__ __align__(128) K2Fov sfov[FAST ? K2_NST : 1][FAST ? 2 * CHT : 1];
     const int stride = POLY ? P.stride : (int)sizeof(K2Pair);
     auto pair_at = [&](int s, int j) -> PairT & { return *reinterpret_cast<PairT *>(sbuf[s] + j * stride); };
     __shared__ __align__(8) uint64_t full[K2_NST], empty[K2_NST];
+    __shared__ K2Cone s_cone[FAST ? BPT : 1][NW];  // cones of each warp's bins, written by the warp itself
     __shared__ float4 s_hb[BPT][K2_THREADS];  // forward-bodge bin directions of this CTA's bins
     // the item's FP64 sums, a column per thread: in registers (two bins a thread) they
     // made the compiler spill inside the pair loop
@@ -1497,8 +1517,10 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
             const int n = min(CH, I.npair - c * CH);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const char *src = POLY ? P.polys : reinterpret_cast<const char *>(P.pairs);
-            bulk_load(smem_u32(sbuf[s]), src + (I.p0 + c * CH) * stride, (uint32_t)(n * stride),
-                      smem_u32(&full[s]));
+            const uint32_t bytes = (uint32_t)(n * stride), fbytes = FAST ? (uint32_t)(2 * n * sizeof(K2Fov)) : 0;
+            mbar_expect(smem_u32(&full[s]), bytes + fbytes);
+            bulk_copy(smem_u32(sbuf[s]), src + (I.p0 + c * CH) * stride, bytes, smem_u32(&full[s]));
+            if (FAST) bulk_copy(smem_u32(sfov[s]), P.fovs + 2 * (I.p0 + c * CH), fbytes, smem_u32(&full[s]));
         };
         if (tid == 0) {
             const int64_t item = (int64_t)atomicAdd(P.counter, 1ull);
@@ -1568,6 +1590,14 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
         for (int q = 0; q < BPT; q++)
 #pragma unroll
             for (int c = 0; c < 8; c++) sum(q, c) = 0.0;
+        if (FAST) {
+#pragma unroll
+            for (int q = 0; q < BPT; q++)
+                if (lane < 8)
+                    reinterpret_cast<float *>(&s_cone[q][tid >> 5])[lane] = reinterpret_cast<const float *>(
+                        &P.cones[((int64_t)I.tile * BPT + q) * NW + (tid >> 5)])[lane];
+            __syncwarp();
+        }
         bool pole = false;
 #pragma unroll
         for (int q = 0; q < BPT; q++) pole = pole || bd[q].pole;
@@ -1620,10 +1650,10 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     const int r = h * 32 + lane;
                     bool k = false;
                     if (r < 2 * n) {
-                        const K2Fov &f = P.fovs[2 * (I.p0 + c * CH) + r];
+                        const K2Fov &f = sfov[st][r];
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k = k || !cone_culled(f, P.cones[((int64_t)I.tile * BPT + q) * NW + (tid >> 5)]);
+                            k = k || !cone_culled(f, s_cone[q][tid >> 5]);
                     }
                     keep[h] = __ballot_sync(0xffffffffu, k);
                 }
@@ -1655,10 +1685,10 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     for (unsigned pm = pm0; pm; pm &= pm - 1u) {
                         const int j = __ffs(pm) - 1;
                         const unsigned m = (j & 16 ? keep[1] : keep[0]) >> (2 * (j & 15));
-                        const K2Fov *fv = P.fovs + 2 * (I.p0 + c * CH + j);
+                        const K2FovExact *fx = P.fovx + 2 * (I.p0 + c * CH + j);
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<true, ST, RE>(pair_at(st, j), fv, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
+                            k2_pair<true, ST, RE>(pair_at(st, j), &sfov[st][2 * j], fx, bd[q], acc[q], hkRh, tmin, s_hb[q][tid],
                                                  (m & 1u) && bd[q].bin >= 0, (m & 2u) && bd[q].bin >= 0,
                                                  P.xyz, P.nb, P.rlo + (I.p0 + c * CH + j) * 3);
                     }
@@ -1666,7 +1696,7 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                     for (int j = 0; j < n; j++)
 #pragma unroll
                         for (int q = 0; q < BPT; q++)
-                            k2_pair<false, ST, RE>(pair_at(st, j), nullptr, bd[q], acc[q], hkRh, tmin,
+                            k2_pair<false, ST, RE>(pair_at(st, j), nullptr, nullptr, bd[q], acc[q], hkRh, tmin,
                                                   s_hb[q][tid], true, true, P.xyz, P.nb,
                                                   P.rlo + (I.p0 + c * CH + j) * 3);
                 }
@@ -2052,6 +2082,7 @@ struct K2Setup {
     char *polys = nullptr;  // facet pairs of polygons, poly_stride bytes each
     int64_t poly_stride = 0;
     K2Fov *fovs = nullptr;
+    K2FovExact *fovx = nullptr;
     float2 *rlo = nullptr;  // R_1 - (float)R_1 per record (the y row), pair layout (3 per pair)
     RefSrc src{};
 };
@@ -2124,12 +2155,14 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     const size_t rec_bytes = poly      ? (size_t)(nrec2 / 2) * S.poly_stride
                              : variant ? (size_t)(nrec2 / 2) * sizeof(K2Pair)
                                        : (size_t)max_recs * sizeof(K2Rec);
-    const size_t fov_bytes = fast_diff ? align_up(nrec2 * sizeof(K2Fov)) : 0;
+    const size_t fov_head = fast_diff ? align_up(nrec2 * sizeof(K2Fov)) : 0;
+    const size_t fov_bytes = fast_diff ? fov_head + align_up(nrec2 * sizeof(K2FovExact)) : 0;
     PBT_TRY(ctx->d_rec.ensure(align_up(rec_bytes) + fov_bytes + (size_t)(nrec2 / 2) * 3 * sizeof(float2)));
     S.recs = variant ? nullptr : ctx->d_rec.as<K2Rec>();
     S.pairs = variant && !poly ? ctx->d_rec.as<K2Pair>() : nullptr;
     S.polys = poly ? ctx->d_rec.as<char>() : nullptr;
     S.fovs = fast_diff ? (K2Fov *)(ctx->d_rec.as<char>() + align_up(rec_bytes)) : nullptr;
+    S.fovx = fast_diff ? (K2FovExact *)(ctx->d_rec.as<char>() + align_up(rec_bytes) + fov_head) : nullptr;
     S.rlo = (float2 *)(ctx->d_rec.as<char>() + align_up(rec_bytes) + fov_bytes);
     // host-side offsets -> device (pinned staging; the previous call's copy
     // out of the staging buffer must have run before it is overwritten)
@@ -2165,11 +2198,11 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     if (nrefs > 0 && poly)
         k2_setup_poly_kernel<<<(unsigned)((nrefs + th - 1) / th), th, 0, st>>>(
             src, nrefs, d_verts, nverts, d_face_off, nfaces, d_face_vi, waveno, lambda, fast_diff, (int)nvp,
-            S.polys, S.poly_stride, S.fovs, S.rlo, &flags->err, &flags->epsmax);
+            S.polys, S.poly_stride, S.fovs, S.fovx, S.rlo, &flags->err, &flags->epsmax);
     else if (nrefs > 0)
         k2_setup_kernel<<<(unsigned)((nrefs + th - 1) / th), th, 0, st>>>(
             src, nrefs, d_verts, nverts, d_face_off, nfaces, d_face_vi, waveno, lambda, fast_diff,
-            S.recs, S.pairs, S.fovs, S.rlo, &flags->err, &flags->epsmax);
+            S.recs, S.pairs, S.fovs, S.fovx, S.rlo, &flags->err, &flags->epsmax);
     ctx->launches++;
     PBT_CUDA_TRY(cudaGetLastError());
     return PBT_OK;
@@ -2339,6 +2372,7 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags
     K2MainArgs A;
     A.recs = S.recs;
     A.fovs = S.fovs;
+    A.fovx = S.fovx;
     A.rlo = S.rlo;
     A.seg_rec = seg_rec;
     A.item_pre = item_pre;
@@ -2361,9 +2395,10 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags
         B.pairs = S.pairs;
         B.polys = S.polys;
         B.stride = (int)S.poly_stride;
-        B.chunk = S.polys ? std::min(fast_diff ? K2P_CH_FOV : K2P_CH_FULL, (int)(kPolyStage / S.poly_stride)) : 0;
+        B.chunk = S.polys ? std::min(fast_diff ? K2P_CH_FOV : K2P_CH_FULL, (int)(poly_stage(fast_diff) / S.poly_stride)) : 0;
         B.rlo = S.rlo;
         B.fovs = S.fovs;
+        B.fovx = S.fovx;
         B.perm = cull ? g.fast_perm.as<int>() : nullptr;
         B.cones = cull ? g.fast_cone.as<K2Cone>() : nullptr;
         B.seg_rec = seg_rec;
