@@ -2332,19 +2332,26 @@ int k2_fast_tiles(pbt_ctx *ctx, cudaStream_t st, int64_t tile) {
     return PBT_OK;
 }
 
-// Records per work item of the default plan: about eight items per resident CTA
-// (four per SM) for the call's records and bin tiles, in multiples of 64, between
-// 256 and 2,048.  Fewer, larger items cost less per item on large lists (24 lists of
-// 3,500 on 361 x 180 bins: 22.2 ms at 1,024, 23.6 at 128); on small grids larger items
-// leave the SMs short of work at the end of the launch (a 31,000-outbeam orientation on
-// 16,290 bins: 2.95 ms at 1,024 records per item, 3.56 ms at 4,096).  A call that does
-// not give every resident CTA an item of 256 takes smaller ones, down to 64 (528
-// outbeams on 6,552 bins, a pass: 147 us at 64, 164 at 128, 205 at 256, 157 at 32).
-int64_t k2_auto_rpi(int64_t nrec, int64_t ntiles, int nsm) {
-    const int64_t slots = (int64_t)4 * std::max(nsm, 1);
-    const int64_t r = (nrec * ntiles / (8 * slots) / 64) * 64;
-    const int64_t one = (nrec * ntiles / slots / 32) * 32;  // one item per resident CTA
-    return std::min<int64_t>({2048, std::max<int64_t>(256, r), std::max<int64_t>(64, one)});
+// Records per work item of the default plan, in multiples of 32.  Fewer, larger items
+// cost less per item; too few leave SMs short of work at the end of the launch.  About
+// eight items per resident CTA (four per SM) up to 2,048 records, and from there twelve
+// up to 8,192:
+// * 24 lists of 3,300 on 64,980 bins, which 5,600 leaves whole: 20.84 ms against 21.09 at
+//   2,048; 60,000 records on 259,560 bins with the field-of-view test 13.72 against 14.04
+//   (without: 63.9 and 63.8); 7,000 records 7.58 at 2,048, 7.88 at 8,192.
+// * Not below 160 records for one list, where the items' number decides how even the
+//   launch ends (eleven lists of 600 to 5,000 on 8,000 to 65,000 bins: 1.5 % above each
+//   one's best on average at 160, 5.1 % at 256, 4 % at 96), and 256 for several, whose
+//   shorter lists split less (60 lists of 200: 0.42 ms, 0.46 at 160).
+// * A call that does not give every resident CTA an item of that takes smaller ones, down
+//   to 64 (528 outbeams on 6,552 bins, a pass: 147 us at 64, 164 at 128, 205 at 256, 157
+//   at 32).
+int64_t k2_auto_rpi(int64_t nrec, int64_t ntiles, int64_t norient, int nsm) {
+    const int64_t per_slot = nrec * ntiles / ((int64_t)4 * std::max(nsm, 1));
+    const int64_t least = norient > 1 ? 256 : 160;
+    const int64_t r = std::max<int64_t>(std::min<int64_t>(2048, std::max(least, per_slot / 8)),
+                                        std::min<int64_t>(8192, per_slot / 12));
+    return std::min(r, std::max<int64_t>(64, per_slot)) / 32 * 32;
 }
 
 int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags, int64_t o0, int64_t no,
@@ -2359,7 +2366,7 @@ int k2_run_chunk(pbt_ctx *ctx, cudaStream_t st, const K2Setup &S, K2Flags *flags
         PBT_TRY(k2_fast_tiles(ctx, st, tile));
         ntiles = g.fast_ntiles;
     }
-    if (plan.auto_rpi) plan.rpi = k2_auto_rpi(nrefs, ntiles, ctx->sm_count);
+    if (plan.auto_rpi) plan.rpi = k2_auto_rpi(nrefs, ntiles, S.src.norient, ctx->sm_count);
     // split tickets of every (segment, tile)
     const int64_t ntk = 2 * no * ntiles;
     PBT_TRY(ctx->d_tk.ensure((size_t)ntk * sizeof(unsigned)));
