@@ -34,6 +34,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <algorithm>
 #include <type_traits>
@@ -94,6 +95,8 @@ struct RefSrc {
     // face has per + 2 vertices (start NULL): nothing to count then
     const int64_t *start;
     int64_t per;
+    // outbeam at position g of the call's list, NULL: g itself (k2_order_kernel)
+    const int *order;
     __device__ __forceinline__ int64_t first(int64_t g) const { return start ? start[g] : g * per; }
 };
 
@@ -111,6 +114,7 @@ __device__ __forceinline__ int64_t find_orient(const int64_t *base, int64_t n, i
 
 __device__ __forceinline__ const pbt_outbeam *ref_lookup(const RefSrc &S, int64_t g, int64_t &o,
                                                          int &kind) {
+    if (S.order) g = S.order[g];
     o = find_orient(S.refbase, S.norient, g);
     const int64_t local = g - S.refbase[o];
     const int64_t nb = S.beam_off[o + 1] - S.beam_off[o];
@@ -120,6 +124,48 @@ __device__ __forceinline__ const pbt_outbeam *ref_lookup(const RefSrc &S, int64_
     }
     kind = 1;
     return S.ext + S.ext_off[o] + (local - nb);
+}
+
+// Sort keys of the field-of-view sum's order: the list (orientation, kind), then the
+// outbeam's direction in the 32 x 32 cells of an octahedral map, in Z order.  A record
+// pair is visited where either record's field of view meets a warp's bins, so partners,
+// and a stage's records, should look the same way.  `alike` counts the pairs that do.
+constexpr int kOrderBits = 5;
+__global__ void k2_order_kernel(RefSrc S, int64_t nrefs, unsigned *__restrict__ keys, int *__restrict__ pos,
+                                int *__restrict__ alike) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lanes = __ballot_sync(0xffffffffu, g < nrefs);
+    if (g >= nrefs) return;
+    int64_t o;
+    int kind;
+    const pbt_outbeam *ob = ref_lookup(S, g, o, kind);
+    const float x = (float)ob->prop_out[0], y = (float)ob->prop_out[1], z = (float)ob->prop_out[2];
+    const float s = 1.0f / (fabsf(x) + fabsf(y) + fabsf(z));
+    float u = x * s, v = y * s;
+    if (z < 0.0f) {
+        const float t = (1.0f - fabsf(v)) * (u < 0.0f ? -1.0f : 1.0f);
+        v = (1.0f - fabsf(u)) * (v < 0.0f ? -1.0f : 1.0f);
+        u = t;
+    }
+    constexpr int n = 1 << kOrderBits;
+    auto cell = [](float w) { return min(max((int)((0.5f * w + 0.5f) * n), 0), n - 1); };
+    const int cu = cell(u), cv = cell(v);
+    unsigned code = 0;
+    for (int b = 0; b < kOrderBits; b++)
+        code |= ((unsigned)(cu >> b) & 1u) << (2 * b) | ((unsigned)(cv >> b) & 1u) << (2 * b + 1);
+    const unsigned key = (unsigned)(2 * o + kind) << (2 * kOrderBits) | code;
+    keys[g] = key;
+    pos[g] = (int)g;
+    const unsigned next = __shfl_down_sync(lanes, key, 1);
+    const unsigned same = __ballot_sync(lanes, !(g & 1) && g + 1 < nrefs && next == key);
+    if ((threadIdx.x & 31) == 0 && same) atomicAdd(alike, __popc(same));
+}
+
+// Lists in which three of four pairs look the same way already (a beam's outbeams one
+// after the other) keep their order: sorting whole beams gains nothing.
+__global__ void k2_keep_order_kernel(int64_t nrefs, unsigned *__restrict__ keys, const int *__restrict__ alike) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < nrefs && 4 * (int64_t)*alike >= 3 * (nrefs / 2)) keys[g] &= ~0u << (2 * kOrderBits);
 }
 
 __global__ void k2_count_kernel(RefSrc S, int64_t nrefs, const int64_t *__restrict__ face_off,
@@ -1463,8 +1509,8 @@ struct K2PkArgs {
 // pairs kept: 49.0 -> 45.6 ms).
 // POLY: facets of up to 16 vertices as one record each (K2Poly): the direction, the
 // polarisation block and the phase once a facet, a divided difference for each triangle
-// of its fan.  16 lists of 3,500 facets of 3-6 vertices with the field-of-view test: 9.64
-// ms, 12.75 as fans (measured at 9.85).
+// of its fan.  16 lists of 3,500 facets of 3-6 vertices with the field-of-view test: 9.85
+// ms against 12.75 as fans (8.37 now).
 template <int BPT, bool FAST, bool POLY>
 __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kernel(K2PkArgs P) {
     using PairT = std::conditional_t<POLY, K2Poly, K2Pair>;
@@ -2133,10 +2179,26 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     if (!uniform)
         cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp, (int64_t *)nullptr, (int64_t *)nullptr,
                                       (int)(nrefs + 1), st);
-    // d_scan: refbase, beam_off, ext_off | cnt | start | scan tmp
+    // With the field-of-view test the outbeams of each list are put in order of direction,
+    // where the sum is large enough to pay for the sort (40 us): 16 lists of 3,500 polygons
+    // of random directions x 64,979 bins, kernel 9.44 -> 8.37 ms; one list of 4,800
+    // triangles x 259,560 bins, a pass 2.18 -> 1.96 ms; 2,000 beams of 100 outbeams x
+    // 259,560 bins, which keep their order, 44.55 ms (45.3 sorted).  The sort is stable, so
+    // the order depends on the lists alone.
+    int sort_bits = 2 * kOrderBits;
+    while (sort_bits < 40 && ((int64_t)1 << (sort_bits - 2 * kOrderBits)) < 2 * norient) sort_bits++;
+    const bool sorted = fast_diff && variant == 1 && sort_bits <= 32 && nrefs < INT32_MAX &&
+                        (double)nrefs * (double)ctx->grid.nb >= 1e9;
+    size_t sort_tmp = 0;
+    if (sorted)
+        cub::DeviceRadixSort::SortPairs(nullptr, sort_tmp, (const unsigned *)nullptr, (unsigned *)nullptr,
+                                        (const int *)nullptr, (int *)nullptr, (int)nrefs, 0, sort_bits, st);
+    // d_scan: refbase, beam_off, ext_off | cnt | start | scan tmp | sort keys, positions, tmp
     const size_t nc = uniform ? 0 : (size_t)(nrefs + 1) * 8;
     const size_t o_rb = 0, o_cnt = align_up(o_rb + 3 * (norient + 1) * 8), o_start = align_up(o_cnt + nc),
-                 o_tmp = align_up(o_start + nc), o_end = align_up(o_tmp + scan_tmp);
+                 o_tmp = align_up(o_start + nc), o_key = align_up(o_tmp + scan_tmp);
+    const size_t n4 = sorted ? align_up((size_t)nrefs * 4) : 0;
+    const size_t o_alike = o_key + 4 * n4, o_stmp = o_alike + (sorted ? 256 : 0), o_end = align_up(o_stmp + sort_tmp);
     PBT_TRY(ctx->d_scan.ensure(o_end));
     char *base = ctx->d_scan.as<char>();
     int64_t *rb = (int64_t *)(base + o_rb), *cnt = (int64_t *)(base + o_cnt);
@@ -2149,6 +2211,7 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     src.norient = norient;
     src.start = uniform ? nullptr : (int64_t *)(base + o_start);
     src.per = poly ? 1 : nv.lo - 2;
+    src.order = nullptr;
     S.poly_stride = poly ? (int64_t)(sizeof(K2Poly) + nvp * sizeof(K2PolyVertex)) : 0;
     // records (or record pairs; an even count so the last pair is whole)
     const int64_t nrec2 = (max_recs + 1) & ~(int64_t)1;
@@ -2182,6 +2245,20 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     if (!ctx->capturing) {
         PBT_CUDA_TRY(cudaEventRecord(ctx->stage_ev, st));
         ctx->stage_pending = true;
+    }
+    if (sorted) {
+        unsigned *keys = (unsigned *)(base + o_key);
+        int *pos = (int *)(base + o_key + 2 * n4), *order = (int *)(base + o_key + 3 * n4);
+        int *alike = (int *)(base + o_alike);
+        const unsigned blocks = (unsigned)((nrefs + 127) / 128);
+        PBT_CUDA_TRY(cudaMemsetAsync(alike, 0, sizeof(int), st));
+        k2_order_kernel<<<blocks, 128, 0, st>>>(src, nrefs, keys, pos, alike);
+        k2_keep_order_kernel<<<blocks, 128, 0, st>>>(nrefs, keys, alike);
+        PBT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(base + o_stmp, sort_tmp, (const unsigned *)keys,
+                                                     (unsigned *)(base + o_key + n4), (const int *)pos, order,
+                                                     (int)nrefs, 0, sort_bits, st));
+        ctx->launches += 3;
+        src.order = order;
     }
     if (!uniform) {
         const int th = 256;

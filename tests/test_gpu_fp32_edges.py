@@ -232,3 +232,26 @@ def test_reach_and_poles(ctx, offset, rows, corners, fast):
         assert rel_err(g, r) <= 2e-5
         if fast:
             assert np.array_equal(g == 0, r == 0)
+
+
+@pytest.mark.parametrize("nv", [[3] * 60, [3] * 55 + [7] * 5, [3, 4, 5] * 20])
+@pytest.mark.parametrize("alike", [False, True])
+def test_direction_order(ctx, nv, alike):
+    """Field-of-view lists long enough (1e9 outbeam-bins) to be put in order of direction,
+    records per face 1 or of a fan, and lists that look alike already and keep their order:
+    the FP64 drop-in's masks, 2e-5 of its largest amplitude, the same bits again."""
+    rng = np.random.default_rng(sum(nv) + alike)
+    geo = _polygon_mesh(rng, nv)
+    beam, ext = outbeams(12001, rng, 60), outbeams(8000, rng, 60, prop=(np.sin(0.3), 0, -np.cos(0.3)))
+    if alike:
+        beam["prop_out"] = beam["prop_out"][np.arange(len(beam)) // 100 * 100]
+        beam["vk7"] = beam["vk7"][np.arange(len(beam)) // 100 * 100]
+    th = np.linspace(4.0, 180.0, 259) * abt_b200.PI_REF / 180.0
+    ph = (0.3 + np.arange(200) * 360.0 / 200) * abt_b200.PI_REF / 180.0
+    got = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=True, precision="fp32")
+    ref = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=True, precision="fp64")
+    again = ctx.diff_main(beam, ext, geo, th, ph, LAM, is_fast_diff=True, precision="fp32")
+    for g, r, a in zip(got, ref, again):
+        assert rel_err(g, r) <= 2e-5
+        assert np.array_equal(g == 0, r == 0)
+        assert np.array_equal(g, a)
