@@ -1,9 +1,11 @@
 // k2_fp32.cu -- batched far-field sum in FP32 with the phase formed in FP64.
 //
 // Pipeline for a batch of orientations (all on the GPU, no host round trip):
-//   1. k2_count / CUB scan / k2_setup: one thread per outgoing facet forms the
-//      facet's aperture frame in FP64 (frame.h, the reference's set-up of
-//      src/diff_mod.f90:515-574) and writes nv-2 K2Rec triangle records.
+//   1. k2_setup: one thread per outgoing facet forms the facet's aperture frame in
+//      FP64 (frame.h, the reference's set-up of src/diff_mod.f90:515-574) and writes
+//      nv-2 triangle records, or one polygon record.  Fans of mixed faces count their
+//      records first (k2_count, CUB scan); large calls with the field-of-view test
+//      take each list in order of direction (k2_order, CUB sort).
 //   2. k2_plan: per (orientation, beam|external) segment, the number of
 //      work items = facet splits x bin tiles.
 //   3. k2_main: a persistent kernel; each CTA claims work items with an
@@ -16,9 +18,9 @@
 //      T(phi) rotation, Mueller matrix (ampl_to_mueller, src/outputs_mod.f90:
 //      473-549), running orientation sum, and per-orientation weighted sums
 //      that equal the reference's simpne phi/theta integrals of M11.
-//   5. k2_final / k2_average: per-orientation parameters (finalise,
+//   5. k2_final: per-orientation parameters (finalise,
 //      src/outputs_mod.f90:133-245) and the orientation average
-//      (summation + divide_by_num_orientations).
+//      (summation + divide_by_num_orientations); k2_avg: its Mueller matrix.
 //
 // Per facet x bin arithmetic.  The reference evaluates, per edge, a contour
 // term with a 1/(kxx kyy) coordinate singularity (src/diff_mod.f90:408-420).
@@ -29,7 +31,8 @@
 // sinc((d_b - d_a)/2) (stable for every pair gap), with a Taylor series when
 // all three phases lie within 0.25 rad.  The far-field phase
 // k(|X - c| - |X|) = -k u.c + k(|c|^2 - (u.c)^2)(1 + u.c/R)/(2R) is formed
-// with k u.c in FP64 and reduced mod 2 pi before the FP32 work; the common
+// with k u.c in FP64 and reduced (as a fixed-point fraction of a turn) before the
+// FP32 work; the common
 // e^{ik|X|} is applied per bin only when amplitudes are returned.
 #include <stdio.h>
 #include <stdlib.h>
@@ -2184,10 +2187,11 @@ int k2_prepare(pbt_ctx *ctx, cudaStream_t st, int64_t norient, const pbt_outbeam
     // of random directions x 64,979 bins, kernel 9.44 -> 8.37 ms; one list of 4,800
     // triangles x 259,560 bins, a pass 2.18 -> 1.96 ms; 2,000 beams of 100 outbeams x
     // 259,560 bins, which keep their order, 44.55 ms (45.3 sorted).  The sort is stable, so
-    // the order depends on the lists alone.
+    // the order depends on the lists alone.  An explicit plan fixes the order of summation
+    // whatever the call's size and sorts nothing.
     int sort_bits = 2 * kOrderBits;
     while (sort_bits < 40 && ((int64_t)1 << (sort_bits - 2 * kOrderBits)) < 2 * norient) sort_bits++;
-    const bool sorted = fast_diff && variant == 1 && sort_bits <= 32 && nrefs < INT32_MAX &&
+    const bool sorted = fast_diff && variant == 1 && plan.auto_rpi && sort_bits <= 32 && nrefs < INT32_MAX &&
                         (double)nrefs * (double)ctx->grid.nb >= 1e9;
     size_t sort_tmp = 0;
     if (sorted)

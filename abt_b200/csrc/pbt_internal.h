@@ -92,8 +92,8 @@ constexpr size_t kIoPar = (size_t)1536 << 10; // copies from here on use several
 constexpr int kIoRent = 24;                   // large copies of a context before it pins them
 
 // ------------------------------------------- reference-exact FP64 records
-// One outgoing facet, prepared for the FP64 kernel (all values formed in the
-// reference's operation order).  384 bytes, in the order the kernel reads it
+// One outgoing facet, prepared for the FP64 kernel (frame, centre and edges formed in
+// the reference's operation order).  384 bytes, in the order the kernel reads it
 // from shared memory, 16 bytes at a time.
 struct alignas(16) K1Facet {
     double com[3];

@@ -89,7 +89,8 @@ int pbt_version(void);
  * Sums every beam outbeam into ampl_far_beam and every external-diffraction
  * outbeam (with fov forced to pi/2, src/diff_mod.f90:797) into
  * ampl_far_ext_diff.  precision = PBT_PREC_FP64 reproduces the reference's
- * arithmetic (facet order 1..n, no FMA); PBT_PREC_FP32 is the fast form.
+ * result (within 1e-10 of its largest amplitude, facets summed in order within
+ * runs of the list); PBT_PREC_FP32 is the fast form.
  * Both output grids are overwritten. */
 int pbt_diff_main_c(pbt_ctx *ctx, const pbt_outbeam *beam, int64_t nbeam,
                     const pbt_outbeam *ext, int64_t next, const double *verts, int64_t nverts,
@@ -286,8 +287,8 @@ int pbt_set_kernel_timing(pbt_ctx *ctx, int32_t enable);
  * two-facet kernel, 0 = one facet per step; bins_per_thread 1 or 2;
  * records_per_item = facet records per work item (32 .. 2^22).  variant < 0
  * restores the default: the packed kernel, one bin per thread, and work items
- * sized per call (about eight per resident CTA for the call's records and bin
- * tiles, 256 to 2,048 records).  Chosen by the tuner (abt_b200/tune.py). */
+ * sized per call (eight to twelve per resident CTA for the call's records and
+ * bin tiles, 64 to 8,192 records).  Chosen by the tuner (abt_b200/tune.py). */
 int pbt_set_plan(pbt_ctx *ctx, int32_t variant, int32_t bins_per_thread, int64_t records_per_item);
 
 /* Sum of the device durations (ms) of the far-field kernel launches timed
