@@ -1658,37 +1658,36 @@ __global__ void __launch_bounds__(K2_THREADS, BPT == 1 ? 4 : 0) k2_main_pk_kerne
                 break;
             }
             const int n = min(CH, I.npair - c * CH);
-            if (!FAST) {
-                // The item's first pair (odd rbeg) and last pair (odd rend) hold a
-                // record of another item or the array's padding: that half takes a
-                // copy of the pair's other record with zero amplitude, so the pair
-                // loop needs no per-pair range test.  Every warp writes the same
-                // values for itself: 3 FP64 phases, then the float2 fields from eps on
-                // (8 of them the amplitudes; a polygon's length m belongs to both halves,
-                // its vertices follow).
-                auto patch = [&](int j, int src, int dst) {
-                    PairT &Q = pair_at(st, j);
-                    float2 *f = &Q.eps[0];
-                    const int amp0 = (int)(&Q.amp[0] - f);
-                    const int nf = (stride - (int)((char *)f - (char *)&Q)) / 8;
-                    for (int t = lane; t < 3 + nf; t += 32) {
-                        if (t < 3) {
-                            Q.kc[t][dst] = Q.kc[t][src];
-                        } else if (!POLY || t - 3 != amp0 - 1) {
-                            const int i = t - 3;
-                            const float v = i >= amp0 && i < amp0 + 8 ? 0.0f : (src ? f[i].y : f[i].x);
-                            if (dst)
-                                f[i].y = v;
-                            else
-                                f[i].x = v;
-                        }
+            // The item's first pair (odd rbeg) and last pair (odd rend) hold a record of another
+            // item or, at the end of an odd list, one that was never written: that half takes a
+            // copy of the pair's other record with zero amplitude.  A stranger's infinite or
+            // NaN amplitude cannot reach the sums then (0 times it is NaN), nor its kx^2 + kz^2
+            // the choice of the step, and without the field-of-view test the pair loop
+            // needs no per-pair range test.  Every warp writes the same values for itself:
+            // 3 FP64 phases, then the float2 fields from eps on (8 of them the amplitudes; a
+            // polygon's length m belongs to both halves, its vertices follow).
+            auto patch = [&](int j, int src, int dst) {
+                PairT &Q = pair_at(st, j);
+                float2 *f = &Q.eps[0];
+                const int amp0 = (int)(&Q.amp[0] - f);
+                const int nf = (stride - (int)((char *)f - (char *)&Q)) / 8;
+                for (int t = lane; t < 3 + nf; t += 32) {
+                    if (t < 3) {
+                        Q.kc[t][dst] = Q.kc[t][src];
+                    } else if (!POLY || t - 3 != amp0 - 1) {
+                        const int i = t - 3;
+                        const float v = i >= amp0 && i < amp0 + 8 ? 0.0f : (src ? f[i].y : f[i].x);
+                        if (dst)
+                            f[i].y = v;
+                        else
+                            f[i].x = v;
                     }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                };
-                if (c == 0 && (I.edge & 1)) patch(0, 1, 0);
-                if (c == I.nchunk - 1 && (I.edge & 2)) patch(n - 1, 0, 1);
-            }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            };
+            if (c == 0 && (I.edge & 1)) patch(0, 1, 0);
+            if (c == I.nchunk - 1 && (I.edge & 2)) patch(n - 1, 0, 1);
             float2 acc[BPT][8];
             [[maybe_unused]] unsigned pm0 = 0, keep[2] = {0, 0};
             if (FAST) {
