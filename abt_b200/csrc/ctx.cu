@@ -24,17 +24,20 @@ void set_error(const char *fmt, ...) {
 void clear_error() { g_last_error.clear(); }
 const char *last_error() { return g_last_error.c_str(); }
 
-// pending injected allocation failures (pbt_test_fail_next_alloc)
-static std::atomic<int32_t> g_fail_allocs{0};
+// pending injected allocation failures (pbt_test_fail_next_alloc, ..._host_alloc)
+static std::atomic<int32_t> g_fail_allocs{0}, g_fail_host_allocs{0};
+static bool take_failure(std::atomic<int32_t> &pending) {
+    int32_t n = pending.load();
+    while (n > 0 && !pending.compare_exchange_weak(n, n - 1)) {
+    }
+    return n > 0;
+}
 
 int DevBuf::ensure(size_t bytes) {
     if (bytes <= cap && p) return PBT_OK;
     release();
     size_t want = bytes < 256 ? 256 : bytes;
-    int32_t pending = g_fail_allocs.load();
-    while (pending > 0 && !g_fail_allocs.compare_exchange_weak(pending, pending - 1)) {
-    }
-    if (pending > 0) {
+    if (take_failure(g_fail_allocs)) {
         set_error("cudaMalloc(%zu) failed: out of memory (injected by pbt_test_fail_next_alloc)", want);
         return PBT_ENOMEM;
     }
@@ -59,6 +62,10 @@ int HostBuf::ensure(size_t bytes) {
     if (bytes <= cap && p) return PBT_OK;
     release();
     size_t want = bytes < 4096 ? 4096 : bytes;
+    if (take_failure(g_fail_host_allocs)) {
+        set_error("cudaMallocHost(%zu) failed: out of memory (injected by pbt_test_fail_next_host_alloc)", want);
+        return PBT_ENOMEM;
+    }
     cudaError_t e = cudaMallocHost(&p, want);
     if (e != cudaSuccess) {
         p = nullptr;
@@ -92,12 +99,21 @@ bool pageable(const void *p) {
 // only after kIoRent large copies by the driver.
 bool io_rented(pbt_ctx *ctx) { return ctx->io_copies < kIoRent && ++ctx->io_copies; }
 
-int io_prepare(pbt_ctx *ctx) {
-    PBT_TRY(ctx->h_io.ensure(kIoSlots * kIoChunk));
-    for (int i = 0; i < kIoSlots; i++)
-        if (!ctx->io_ev[i])
-            PBT_CUDA_TRY(cudaEventCreateWithFlags(&ctx->io_ev[i], cudaEventDisableTiming));
-    return PBT_OK;
+// The slots and their events.  Where they cannot be had (the limit of locked memory, say)
+// the context's copies stay with the driver, and nothing is tried again.
+bool io_prepare(pbt_ctx *ctx) {
+    if (ctx->io_state == 0) {
+        bool ok = ctx->h_io.ensure(kIoSlots * kIoChunk) == PBT_OK;
+        for (int i = 0; ok && i < kIoSlots; i++)
+            ok = cudaEventCreateWithFlags(&ctx->io_ev[i], cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) {
+            (void)cudaGetLastError();
+            clear_error();
+            ctx->h_io.release();
+        }
+        ctx->io_state = ok ? 1 : -1;
+    }
+    return ctx->io_state > 0;
 }
 
 // memcpy of a chunk, by up to eight threads in 64 KB pieces when the whole copy is
@@ -118,12 +134,11 @@ void copy_threads(char *dst, const char *src, size_t n, bool par) {
 // 2.1 MB to the host took 138 us, 8.3 MB 438 us, against 49 and 159 us of transfer.
 // Here the transfer of one chunk runs while the host threads move the chunks before it.
 int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st) {
-    if (bytes < kIoMin || !pageable(dst) || io_rented(ctx)) {
+    if (bytes < kIoMin || !pageable(dst) || io_rented(ctx) || !io_prepare(ctx)) {
         PBT_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         PBT_CUDA_TRY(cudaStreamSynchronize(st));
         return PBT_OK;
     }
-    PBT_TRY(io_prepare(ctx));
     char *pin = ctx->h_io.as<char>();
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     auto size_of = [&](size_t c) { return std::min(kIoChunk, bytes - c * kIoChunk); };
@@ -147,11 +162,10 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
 }
 
 int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st) {
-    if (bytes < kIoMinUp || !pageable(src) || io_rented(ctx)) {
+    if (bytes < kIoMinUp || !pageable(src) || io_rented(ctx) || !io_prepare(ctx)) {
         PBT_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return PBT_OK;
     }
-    PBT_TRY(io_prepare(ctx));
     char *pin = ctx->h_io.as<char>();
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     for (size_t c = 0; c < nch; c++) {
@@ -361,4 +375,8 @@ extern "C" int64_t pbt_last_launch_count(pbt_ctx *ctx) { return ctx ? ctx->launc
 
 extern "C" int pbt_test_fail_next_alloc(int32_t count) {
     return pbt::g_fail_allocs.exchange(count > 0 ? count : 0);
+}
+
+extern "C" int pbt_test_fail_next_host_alloc(int32_t count) {
+    return pbt::g_fail_host_allocs.exchange(count > 0 ? count : 0);
 }

@@ -170,6 +170,7 @@ struct pbt_ctx {
     pbt::HostBuf h_io;               // pinned slots of copy_to_host / copy_to_device
     cudaEvent_t io_ev[pbt::kIoSlots] = {};
     int io_copies = 0;               // large copies left to the driver so far
+    int io_state = 0;                // 0: slots not tried yet, 1: there, -1: not to be had
     cudaEvent_t stage_ev = nullptr;  // last copy out of h_stage (wait before reuse)
     bool stage_pending = false;
     pbt::DevTotals tot;    // user-visible totals (pbt_summation_c / pbt_finalise_c accumulate)

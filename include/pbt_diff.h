@@ -407,6 +407,10 @@ int pbt_selftest_bounded_wait_c(pbt_ctx *ctx, int32_t limit_ms);
  * 0 clears the injection.  Returns the count that was pending before. */
 int pbt_test_fail_next_alloc(int32_t count);
 
+/* The same for the next `count` allocations of pinned host memory.  The slots for
+ * large copies are not needed for a result: without them the driver copies. */
+int pbt_test_fail_next_host_alloc(int32_t count);
+
 #ifdef __cplusplus
 }
 #endif
