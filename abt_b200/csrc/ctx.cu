@@ -6,7 +6,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <new>
 
+#include "copy_pool.h"
 #include "pbt_internal.h"
 
 namespace pbt {
@@ -116,17 +118,28 @@ bool io_prepare(pbt_ctx *ctx) {
     return ctx->io_state > 0;
 }
 
-// memcpy of a chunk, by up to eight threads in 64 KB pieces when the whole copy is
-// kIoPar or more (2.1 MB out: 113 us a call against 186 on one thread).  Smaller ones
-// stay on the calling thread: the threads wait actively for a while afterwards, and a
-// caller with threaded work of its own (the torch operations of a gradient step on
-// 6,000 bins) lost 4 % to them.
-void copy_threads(char *dst, const char *src, size_t n, bool par) {
-    const int64_t piece = 64 << 10, np = (int64_t)((n + piece - 1) / piece);
-#pragma omp parallel for schedule(static) num_threads(8) if (par && np > 1)
-    for (int64_t i = 0; i < np; i++)
-        memcpy(dst + i * piece, src + i * piece, std::min<size_t>(piece, n - i * piece));
+// The helpers of a copy of kIoPar or more (2.1 MB out: 120 us a call with them, 190
+// without); NULL for a smaller one, which the calling thread moves alone.
+CopyPool *io_helpers(pbt_ctx *ctx, size_t bytes) {
+    if (bytes < kIoPar) return nullptr;
+    if (!ctx->io_pool) ctx->io_pool.reset(new (std::nothrow) CopyPool);
+    return ctx->io_pool.get();
 }
+struct Helped {
+    CopyPool *pool;
+    explicit Helped(CopyPool *p) : pool(p) {
+        if (pool) pool->begin();
+    }
+    ~Helped() {
+        if (pool) pool->end();
+    }
+    void copy(char *dst, const char *src, size_t n) {
+        if (pool)
+            pool->run(dst, src, n);
+        else
+            memcpy(dst, src, n);
+    }
+};
 
 }  // namespace
 
@@ -140,6 +153,7 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
         return PBT_OK;
     }
     char *pin = ctx->h_io.as<char>();
+    Helped helped{io_helpers(ctx, bytes)};
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     auto size_of = [&](size_t c) { return std::min(kIoChunk, bytes - c * kIoChunk); };
     for (size_t c = 0; c < nch + kIoSlots - 1; c++) {
@@ -154,8 +168,7 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
             const size_t d = c + 1 - kIoSlots, s = d % kIoSlots;
             if (d >= nch) continue;
             PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
-            copy_threads((char *)dst + d * kIoChunk, pin + s * kIoChunk, size_of(d),
-                         bytes >= kIoPar);
+            helped.copy((char *)dst + d * kIoChunk, pin + s * kIoChunk, size_of(d));
         }
     }
     return PBT_OK;
@@ -167,12 +180,13 @@ int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaS
         return PBT_OK;
     }
     char *pin = ctx->h_io.as<char>();
+    Helped helped{io_helpers(ctx, bytes)};
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     for (size_t c = 0; c < nch; c++) {
         const size_t s = c % kIoSlots, n = std::min(kIoChunk, bytes - c * kIoChunk);
         // the slot's last transfer, of this copy or of an earlier one
         PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
-        copy_threads(pin + s * kIoChunk, (const char *)src + c * kIoChunk, n, bytes >= kIoPar);
+        helped.copy(pin + s * kIoChunk, (const char *)src + c * kIoChunk, n);
         PBT_CUDA_TRY(cudaMemcpyAsync((char *)dst + c * kIoChunk, pin + s * kIoChunk, n,
                                      cudaMemcpyHostToDevice, st));
         PBT_CUDA_TRY(cudaEventRecord(ctx->io_ev[s], st));
@@ -353,6 +367,7 @@ extern "C" int pbt_ctx_destroy(pbt_ctx *ctx) {
         ctx->btot.release();
         ctx->h_stage.release();
         ctx->h_io.release();
+        ctx->io_pool.reset();
         for (cudaEvent_t e : ctx->io_ev)
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
