@@ -460,24 +460,29 @@ int k1_launch(pbt_ctx *ctx, cudaStream_t st, const K1Facet *d_fac, int64_t n0, i
     // the result is deterministic; it differs from the one-run order by rounding.
     // Measured on 1,700 + 882 triangles x 32,580 bins: 10 waves 1.48 ms, 14 1.45, 18 1.43,
     // 24 1.42, 32 1.41 with the sum of the partial grids, which takes 37 us of it.
+    // The partial grids take 64 B a bin and run, 195 MB for a grid of up to a million bins; a
+    // device without room for them gets fewer runs, at last one a list, which needs none.
     const int64_t resident = (int64_t)ctx->sm_count * K1_MINB;
     const int64_t all = std::max<int64_t>(n0 + n1, 1);
-    const int64_t runs = (K1_WAVES * resident + blocks - 1) / blocks;
-    for (int k = 0; k < 2; k++) {
-        int64_t s = std::min<int64_t>(std::min<int64_t>(runs * n[k] / all, n[k] / 16), 64);
-        s = std::max<int64_t>(s, 1);
-        A.n[k] = n[k];
-        A.first[k] = first[k];
-        A.run[k] = std::max<int64_t>((n[k] + s - 1) / s, 1);
-        A.split[k] = n[k] > 0 ? (int)((n[k] + A.run[k] - 1) / A.run[k]) : 1;
+    int ysum = 0;
+    bool parts = false;
+    for (int64_t waves = K1_WAVES;; waves /= 2) {
+        const int64_t runs = (waves * resident + blocks - 1) / blocks;
+        for (int k = 0; k < 2; k++) {
+            int64_t s = std::min<int64_t>(std::min<int64_t>(runs * n[k] / all, n[k] / 16), 64);
+            s = std::max<int64_t>(s, 1);
+            A.n[k] = n[k];
+            A.first[k] = first[k];
+            A.run[k] = std::max<int64_t>((n[k] + s - 1) / s, 1);
+            A.split[k] = n[k] > 0 ? (int)((n[k] + A.run[k] - 1) / A.run[k]) : 1;
+        }
+        if (!d_grid1) A.split[1] = 0;
+        ysum = A.split[0] + A.split[1];
+        parts = A.split[0] > 1 || A.split[1] > 1;
+        if (!parts || ctx->d_k1part.ensure((size_t)ysum * 8 * g.nb * sizeof(double)) == PBT_OK) break;
+        clear_error();
     }
-    if (!d_grid1) A.split[1] = 0;
-    const int ysum = A.split[0] + A.split[1];
-    const bool parts = A.split[0] > 1 || A.split[1] > 1;
-    if (parts) {
-        PBT_TRY(ctx->d_k1part.ensure((size_t)ysum * 8 * g.nb * sizeof(double)));
-        A.part = ctx->d_k1part.as<double>();
-    }
+    if (parts) A.part = ctx->d_k1part.as<double>();
     timing_begin(ctx, st);
     const dim3 grid((unsigned)blocks, (unsigned)ysum);
     if (fast_diff)
