@@ -52,6 +52,7 @@
 #include <mutex>
 
 #include "frame.h"
+#include "k1_math.cuh"
 #include "pbt_internal.h"
 
 namespace pbt {
@@ -80,45 +81,6 @@ __device__ __forceinline__ double dot_3(const double a[3], const double b[3]) {
     s = s + a[1] * b[1];
     s = s + a[2] * b[2];
     return s;
-}
-
-// 1/x and 1/sqrt(x): the hardware's FP64 seeds (about 20 bits) and one Newton step
-// of third order, e^3 below 2^-58; x normal and positive (rcp_n: any sign).
-__device__ __forceinline__ double rcp_n(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double rsqrt_n(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-// e^{ix} from a table of the 128th roots of unity and short polynomials: x = n h + r, h =
-// 2 pi / 128 in two parts (each product fused, so r is good to 1e-16 absolute for
-// |x| < 2^30), and e^{ir} on |r| <= h/2 from minimax fits (Remez exchange in 50 digits:
-// 3e-17 for sin, 3e-20 for cos - 1).  15 FP64 operations; the quadrant form with
-// polynomials to r^13 and r^14 takes 20 and as many selects and sign changes again, the
-// library's checks for huge arguments too and reads its coefficients from memory.
-constexpr int kRoots = 128;
-__device__ __forceinline__ double reduce_n(double x, int *n32) {
-    const double t = fma(x, 20.371832715762604, 6755399441055744.0);
-    *n32 = __double2loint(t);  // n modulo 2^32
-    const double n = t - 6755399441055744.0;
-    return fma(-n, 1.9135106236677394e-18, fma(-n, 0.04908738521234052, x));
-}
-// e^{i (x + nk h)}, roots[k] = (cos, sin)(k h)
-__device__ __forceinline__ void sincos_n(double x, int nk, const double2 *roots, double *sn, double *cs) {
-    int n;
-    const double r = reduce_n(x, &n);
-    const double2 w = roots[(n + nk) & (kRoots - 1)];
-    const double z = r * r;
-    const double s = fma(r * z, fma(z, 0.008333155366073453, -0.16666666662958388), r);
-    const double c = z * fma(z, fma(z, -0.0013888601850806472, 0.041666666656641586), -0.499999999999999);
-    *cs = fma(-w.y, s, fma(w.x, c, w.x));
-    *sn = fma(w.x, s, fma(w.y, c, w.y));
 }
 
 // contour_integral for one bin (src/diff_mod.f90:357-428), operation by operation
