@@ -6,9 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
-#include <new>
 
-#include "copy_pool.h"
 #include "pbt_internal.h"
 
 namespace pbt {
@@ -118,24 +116,19 @@ bool io_prepare(pbt_ctx *ctx) {
     return ctx->io_state > 0;
 }
 
-// The helpers of a copy of kIoPar or more (2.1 MB out: 120 us a call with them, 190
-// without); NULL for a smaller one, which the calling thread moves alone.
-CopyPool *io_helpers(pbt_ctx *ctx, size_t bytes) {
-    if (bytes < kIoPar) return nullptr;
-    if (!ctx->io_pool) ctx->io_pool.reset(new (std::nothrow) CopyPool);
-    return ctx->io_pool.get();
-}
-struct Helped {
-    CopyPool *pool;
-    explicit Helped(CopyPool *p) : pool(p) {
-        if (pool) pool->begin();
+// The host side of one copy: by the context's team from kIoPar on, by the calling thread
+// below.
+struct Mover {
+    CopyTeam *team;
+    Mover(pbt_ctx *ctx, size_t bytes) : team(bytes >= kIoPar ? &ctx->io_team : nullptr) {
+        if (team) team->begin();
     }
-    ~Helped() {
-        if (pool) pool->end();
+    ~Mover() {
+        if (team) team->end();
     }
     void copy(char *dst, const char *src, size_t n) {
-        if (pool)
-            pool->run(dst, src, n);
+        if (team)
+            team->run(dst, src, n);
         else
             memcpy(dst, src, n);
     }
@@ -153,7 +146,7 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
         return PBT_OK;
     }
     char *pin = ctx->h_io.as<char>();
-    Helped helped{io_helpers(ctx, bytes)};
+    Mover mover(ctx, bytes);
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     auto size_of = [&](size_t c) { return std::min(kIoChunk, bytes - c * kIoChunk); };
     for (size_t c = 0; c < nch + kIoSlots - 1; c++) {
@@ -168,7 +161,7 @@ int copy_to_host(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStr
             const size_t d = c + 1 - kIoSlots, s = d % kIoSlots;
             if (d >= nch) continue;
             PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
-            helped.copy((char *)dst + d * kIoChunk, pin + s * kIoChunk, size_of(d));
+            mover.copy((char *)dst + d * kIoChunk, pin + s * kIoChunk, size_of(d));
         }
     }
     return PBT_OK;
@@ -180,13 +173,13 @@ int copy_to_device(pbt_ctx *ctx, void *dst, const void *src, size_t bytes, cudaS
         return PBT_OK;
     }
     char *pin = ctx->h_io.as<char>();
-    Helped helped{io_helpers(ctx, bytes)};
+    Mover mover(ctx, bytes);
     const size_t nch = (bytes + kIoChunk - 1) / kIoChunk;
     for (size_t c = 0; c < nch; c++) {
         const size_t s = c % kIoSlots, n = std::min(kIoChunk, bytes - c * kIoChunk);
         // the slot's last transfer, of this copy or of an earlier one
         PBT_CUDA_TRY(cudaEventSynchronize(ctx->io_ev[s]));
-        helped.copy(pin + s * kIoChunk, (const char *)src + c * kIoChunk, n);
+        mover.copy(pin + s * kIoChunk, (const char *)src + c * kIoChunk, n);
         PBT_CUDA_TRY(cudaMemcpyAsync((char *)dst + c * kIoChunk, pin + s * kIoChunk, n,
                                      cudaMemcpyHostToDevice, st));
         PBT_CUDA_TRY(cudaEventRecord(ctx->io_ev[s], st));
@@ -367,7 +360,6 @@ extern "C" int pbt_ctx_destroy(pbt_ctx *ctx) {
         ctx->btot.release();
         ctx->h_stage.release();
         ctx->h_io.release();
-        ctx->io_pool.reset();
         for (cudaEvent_t e : ctx->io_ev)
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
