@@ -4,16 +4,14 @@
 #include <nvtx3/nvToolsExt.h>
 #include <stdint.h>
 
-#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/pbt_diff.h"
+#include "copy_team.h"
 
 namespace pbt {
-
-class CopyPool;  // copy_pool.h
 
 // A named NVTX range over a host-side stage (set-up, far-field sum, epilogue,
 // finalise, adjoint), the counterpart of the reference's timing spans
@@ -91,7 +89,7 @@ constexpr int kIoSlots = 4;
 constexpr size_t kIoChunk = (size_t)512 << 10;
 constexpr size_t kIoMin = (size_t)256 << 10;  // smaller results go to the driver as they are
 constexpr size_t kIoMinUp = (size_t)64 << 10; // smaller uploads too (from here on they wait for the stream there)
-constexpr size_t kIoPar = (size_t)1536 << 10; // copies from here on use helper threads (copy_pool.h)
+constexpr size_t kIoPar = (size_t)1536 << 10; // copies from here on use several host threads (copy_team.h)
 constexpr int kIoRent = 24;                   // large copies of a context before it pins them
 
 // ------------------------------------------- reference-exact FP64 records
@@ -172,7 +170,7 @@ struct pbt_ctx {
     pbt::HostBuf h_stage;
     pbt::HostBuf h_io;               // pinned slots of copy_to_host / copy_to_device
     cudaEvent_t io_ev[pbt::kIoSlots] = {};
-    std::unique_ptr<pbt::CopyPool> io_pool;  // helpers of copies of kIoPar or more
+    pbt::CopyTeam io_team;           // of copies of kIoPar or more
     int io_copies = 0;               // large copies left to the driver so far
     int io_state = 0;                // 0: slots not tried yet, 1: there, -1: not to be had
     cudaEvent_t stage_ev = nullptr;  // last copy out of h_stage (wait before reuse)
