@@ -269,10 +269,11 @@ void k1_facet(const FacetFrame &fr, const pbt_outbeam &ob, double fov, int nv, c
     }
     F.pad[0] = F.pad[1] = 0.0;
     // The contour's rounding noise relative to the facet's area: nv edges of
-    // ulp(d) L / (min(|kxx|, |kyy|) |omega| A), |d| <= 2 k rmax; `cond` is where it
+    // 2.2e-16 max(|d|, 1) L / (min(|kxx|, |kyy|) |omega| A), |d| <= 2 k rmax the phases
+    // (the cosines it subtracts are known to 1.1e-16 however small d is); `cond` is where it
     // reaches 5e-11.  A clamped slope has no closed form: the contour everywhere (and
     // with phases beyond the kernel's argument reduction).
-    const double noise = nv * 2.0 * waveno * rmax * 2.2e-16 * lmax;
+    const double noise = nv * std::max(2.0 * waveno * rmax, 1.0) * 2.2e-16 * lmax;
     F.cond = clamped || !(fabs(area) > 0) || 2.0 * waveno * (rmax + kFarR) > 1e9
                  ? HUGE_VAL
                  : noise / (fabs(area) * 5e-11);
