@@ -1,8 +1,10 @@
 // k1_fp64.cu -- FP64 far-field sum in the reference's arithmetic (the plain drop-in).
 //
-// One thread per far-field bin; each thread walks the facet list in order and
-// adds every facet's 2x2 complex amplitude to its bin, so the sum has the
-// reference's association ((0 + c_1) + c_2) + ... (src/diff_mod.f90:744-766).
+// One thread per far-field bin; each thread walks a run of the facet list in order and
+// adds every facet's 2x2 complex amplitude to its bin.  Within a run the order is the
+// reference's, ((0 + c_1) + c_2) + ... (src/diff_mod.f90:744-766), in fused
+// multiply-adds and the circular basis; a list is one run on large grids and up to 64 on
+// small ones (k1_launch), whose sums are added in run order.
 //
 // The rounding of a few quantities decides the result far above 1e-16 and they
 // are formed operation by operation as the reference forms them: the rotated
@@ -19,9 +21,10 @@
 // * The reference's noise in an edge's term is about ulp(d) L / (min(|kxx|,
 //   |kyy|) |omega|), omega the phase step along the edge, L the edge's extent.
 //   A lane with omega_min * min(|kxx|, |kyy|) below the facet's `cond`
-//   (K1Facet) has a noise above 1e-11 of the facet's area and takes the
-//   contour itself, so both agree to 1e-11 everywhere.  Facets with a clamped
-//   edge slope (:379-382) always take it.
+//   (K1Facet; ulp(max(|d|, 1)), since cosines near 1 are known to 1.1e-16 only) has a
+//   noise above 5e-11 of the facet's area and takes the contour itself, so both agree to
+//   5e-11 of the area everywhere.  Facets with a clamped edge slope (:379-382) always
+//   take it.
 // * The polarisation block (karczewski :124-198 and the scattering-plane
 //   rotation :628-658) reduces, away from the clamp of ky, to A = sc (P d + Q e),
 //   B = sc (P e - Q d) with d = -(Kz t + kz), e = -kx ky, t = kx^2 + kz^2, h = (b, -a, 0) the incidence direction times the unit
@@ -32,8 +35,9 @@
 //   in which the sums are kept; the basis change and the rotation T(phi), which
 //   depends on the bin alone, are applied once at the end.
 //
-// Bound: FP64 pipe (65 % of cycles; 360 instructions a triangle and bin, 196 of them
-// FP64, against 1,813 with every operation of the reference).  A triangle list of
+// Bound: FP64 pipe (66 % of cycles; 351 instructions a triangle and bin, 191 of them FP64,
+// and 331 and 185 on 2,000 triangles x 259,560 bins, where fewer lanes take the contour;
+// 1,813 with every operation of the reference).  A triangle list of
 // 2,582 x 32,580 bins takes 1.42 ms (5.9e10 facet-bin/s), the operation-by-operation
 // kernel took 6.92 ms (1.59 ms with quadrant polynomials in place of the table of
 // roots, 1.51 ms with the forward bodge in the aperture frame).  The facet records go
@@ -422,8 +426,9 @@ int k1_launch(pbt_ctx *ctx, cudaStream_t st, const K1Facet *d_fac, int64_t n0, i
     // the result is deterministic; it differs from the one-run order by rounding.
     // Measured on 1,700 + 882 triangles x 32,580 bins: 10 waves 1.48 ms, 14 1.45, 18 1.43,
     // 24 1.42, 32 1.41 with the sum of the partial grids, which takes 37 us of it.
-    // The partial grids take 64 B a bin and run, 195 MB for a grid of up to a million bins; a
-    // device without room for them gets fewer runs, at last one a list, which needs none.
+    // The partial grids take 64 B a bin and run, 195 MB on grids of up to 200,000 bins and
+    // 600 MB at most (near 3 million); a device without room for them gets fewer runs, at
+    // last one a list, which needs none.
     const int64_t resident = (int64_t)ctx->sm_count * K1_MINB;
     const int64_t all = std::max<int64_t>(n0 + n1, 1);
     int ysum = 0;

@@ -429,7 +429,11 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
                                         int64_t nphi, int64_t theta_i, float *acc) {
     // forward: k u.c modulo 2 pi as a fixed-point fraction of a turn (2^-32 units), the low
     // word of the FP64 sum added to 1.5 * 2^20; beyond 2^18 turns (WIDE) the nearest
-    // integer is taken off first
+    // integer is taken off first.  The fraction's FP32 form and the rounded constant make
+    // 8.0e-8 rad rms and 3.0e-7 at most, 4.6e-8 and 1.2e-7 with one rounding of an FP64
+    // remainder; the gradients' error against 64 bits did not grow with it (250 random
+    // cases at each of five sizes: vertices within 3 % of that form's either way,
+    // amplitudes 4 % below).
     float fr;
     if (!WIDE) {
         fr = (float)__double2loint(fma(B.uz, r.kc[2], fma(B.uy, r.kc[1], fma(B.ux, r.kc[0], kFracMagic4))));
@@ -628,8 +632,9 @@ __device__ __forceinline__ void k4_eval(const K4Rec &r, const Bin4 &B, float k, 
 // reduction and the FP64 atomic into out[record][30] happen once per
 // (record, range).  The warps of a CTA walk the same bins, which the L1 serves.
 //
-// Bound: issue (78 % of the slots; 366 instructions a facet and bin, 272 of them on the
-// FMA pipe).  In the aperture frame, with the sums of the incidence direction and of the
+// Bound: issue.  78 % of the slots and 372 instructions a facet and bin, 275 of them on the
+// FMA pipe, on the plate below, whose 16,290 bins end in part-filled steps; 76 %, 354 and 260
+// on 2,000 triangles x 259,560 bins.  In the aperture frame, with the sums of the incidence direction and of the
 // centre's frame components kept apart (36 sums, 168 registers, three CTAs per SM), a
 // plate of 30,968 triangles x 16,290 bins took 7.32 ms; in the lab frame 6.92 (30 sums,
 // 128 registers, four CTAs), with scalar instead of packed FP32x2 operations, whose

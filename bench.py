@@ -759,11 +759,12 @@ def diffraction_call(ncalls):
         L.pbt_ctx_destroy(h)
 
 
-def fast_diff_kept_fraction(beam, geo, th, ph, sample=20000, tile_theta=8, tile_phi=16):
-    """Fraction of (record, bin tile) pairs that the -fast_diff tile cull keeps,
-    estimated on the host on the first `sample` records with the kernel's test:
-    a record is skipped for a tile when the angle between its prop_out and the
-    tile's centre exceeds fov + 2|com|/R + 1e-5 plus the tile's angular radius."""
+def fast_diff_kept_fraction(beam, geo, th, ph, sample=20000, tile_theta=4, tile_phi=8):
+    """Fraction of (record, warp) pairs that the -fast_diff cull keeps, estimated on the
+    host on the first `sample` records with the kernel's test: a record is skipped for a
+    warp's 4 x 8 bins when the angle between its prop_out and their centre exceeds
+    fov + 2|com|/R + 1e-5 plus their angular radius.  (The kernel evaluates a pair of
+    records where either is kept.)"""
     ob = beam[:sample]
     TH, PH = np.meshgrid(th, ph, indexing="ij")  # (ntheta, nphi)
     u = np.stack([np.sin(TH) * np.cos(PH), np.sin(TH) * np.sin(PH), -np.cos(TH)], -1)
@@ -779,10 +780,12 @@ def fast_diff_kept_fraction(beam, geo, th, ph, sample=20000, tile_theta=8, tile_
     fo, fv, V = geo["face_off"], geo["face_vi"], geo["verts"]
     com = np.array([V[fv[fo[f - 1]:fo[f]] - 1].mean(0) for f in ob["fi"]])
     fovm = ob["fov"] + 2 * np.linalg.norm(com, axis=1) / 1e6 + 1e-5
-    ang = np.arccos(np.clip(ob["prop_out"] @ cen.T, -1, 1))
-    lim = fovm[:, None] + psi[None, :]
-    kept = (lim >= np.pi) | (ang <= lim)
-    return float(kept.mean())
+    kept = 0
+    for r in range(0, len(ob), 1000):
+        ang = np.arccos(np.clip(ob["prop_out"][r:r + 1000] @ cen.T, -1, 1))
+        lim = fovm[r:r + 1000, None] + psi[None, :]
+        kept += int(((lim >= np.pi) | (ang <= lim)).sum())
+    return kept / (len(ob) * len(cen))
 
 
 def run_reference(args, world, rank):
@@ -1035,14 +1038,14 @@ def main():
                                              "the kernel time, culled pairs included",
                               "kept_pair_fraction": kept,
                               "evaluated_value": kept * work / (kf_ms / 1e3),
-                              "evaluated_basis": "facet-bins of the (record, tile) pairs the "
+                              "evaluated_basis": "facet-bins of the (record, warp) pairs the "
                                                  "cull keeps (fraction estimated on the host on "
                                                  "20,000 records) over the kernel time",
                               "speedup_vs_full_kernel": (kern_ms / max(kern_n, 1)) / kf_ms,
                               "max_rel_mueller_err_vs_fp64_fast_20000_facets":
                                   mueller_rel_err(m32, m64, 1e-6),
-                              "cull": "records whose field of view misses a 8x16 (theta x phi) "
-                                      "bin tile are skipped for that tile"}
+                              "cull": "records whose field of view misses a warp's 4x8 (theta x phi) "
+                                      "bins are skipped for that warp"}
 
     if args.diffraction_calls > 0 and solo:
         extra["diffraction_call"] = diffraction_call(args.diffraction_calls)

@@ -89,8 +89,10 @@ int pbt_version(void);
  * Sums every beam outbeam into ampl_far_beam and every external-diffraction
  * outbeam (with fov forced to pi/2, src/diff_mod.f90:797) into
  * ampl_far_ext_diff.  precision = PBT_PREC_FP64 reproduces the reference's
- * result (within 1e-10 of its largest amplitude, facets summed in order within
- * runs of the list); PBT_PREC_FP32 is the fast form.
+ * result (each facet's amplitude within 5e-11 of its area over the wavelength and
+ * so, on a grid that holds the facets' main lobes, within 1e-10 of the largest
+ * amplitude; facets summed in order within runs of the list); PBT_PREC_FP32 is
+ * the fast form.
  * Both output grids are overwritten. */
 int pbt_diff_main_c(pbt_ctx *ctx, const pbt_outbeam *beam, int64_t nbeam,
                     const pbt_outbeam *ext, int64_t next, const double *verts, int64_t nverts,
@@ -275,7 +277,8 @@ int pbt_graph_destroy_c(pbt_graph *graph);
 /* ---------------------------------------------------------- introspection */
 
 /* Number of kernel launches made by the last completed compute call on this
- * context (for launch accounting in benchmarks). */
+ * context (for launch accounting in benchmarks; a scan or a sort of CUB counts as
+ * one, whatever kernels it is made of). */
 int64_t pbt_last_launch_count(pbt_ctx *ctx);
 
 /* Enable (1) or disable (0) CUDA-event timing of the far-field kernels (the
